@@ -151,111 +151,222 @@ struct Op32ScStats {
   }
 };
 
+// ---- statistics of a kick that the element map before it could not certify --
 // The longitudinal-loss test (UpdateLongitudinalLossCoordinateKernel with the
 // lloss and good counts and <phi>_good, beam.cpp:780-781, 1008-1009) and the
-// SCHEFF moments in one sweep, when the element map before the kick could
-// not certify its own statistics (sc_redo == 2).  The relative phases are
-// taken about the <phi>_good that sweep recorded; when the test flags no
+// SCHEFF moments in one sweep (sc_redo == 2).  The relative phases are taken
+// about the <phi>_good that the map's sweep recorded; when the test flags no
 // particle of the good set, that is the <phi>_good the separate sweeps would
-// have used, and the totals are the same ones in the same order.  Otherwise
-// the sweep records the new <phi>_good and asks for the moments sweep again
-// (sc_redo = 1).
-struct Op32LlossScStats {
-  static constexpr int K = 12;
-  static constexpr bool kFast = true;
-  using Comb = SumComb;
-  struct Ctx { float lim, pag; };
+// have used.  Otherwise the moments are swept again about the new <phi>_good.
+//
+// One launch of clusters of kStatCluster CTAs: the whole grid takes the first
+// sweep, and the last cluster to finish takes the totals and, when the good
+// set changed, sweeps the moments again with all its threads (partial sums
+// through distributed shared memory in rank order).  Beams whose bunch
+// stretches over the whole period (a quad channel behind one buncher) lose
+// particles longitudinally at almost every kick, so the second sweep is their
+// common path: one block of 256 threads took 31 us a kick at 20,011 particles
+// (sweep phase of the quad channel, 1.26 ms over 40 kicks) and over a
+// millisecond at 524,288; a second grid-wide launch would cost its launch at
+// every kick of every beam, where this one returns at once when it is not
+// needed.
+constexpr int kStatCluster = 8;
+constexpr int kStatThreads = 1024;
+constexpr int kStatWarps = kStatThreads / 32;
+constexpr int kStatBatch = 4;  // particles a thread has in flight
+
+struct StatArgs {
   DevBeam b;
   ScState *sc;
   ScTables t;
   double freq, frac;
   Sc32Host h;
-  __device__ bool enabled() const { return b.st->sc_redo == 2u; }
-  __device__ Ctx setup() const {
-    const double pag = b.st->st[PHI_AVG_GOOD] - b.phi_ref;
-    return {(float)(pag + TWOPI + PI), (float)pag};
+  PassScratch scr;
+};
+
+struct StatIn {
+  uint32_t lo, ll;
+  float ph, x, y, w;
+};
+__device__ __forceinline__ StatIn stat_load(const DevBeam &b, uint32_t i) {
+  return {b.loss[i], b.lloss[i], b.fphi[i], b.fx[i], b.fy[i], b.fw[i]};
+}
+
+// block sums of a[0..K) into out[0..K) (shared memory): a fixed shuffle tree,
+// then the warps in order
+template <int K>
+__device__ __forceinline__ void stat_block_sum(const float (&a)[12], float (*red)[12], float *out) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    float v = a[k];
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+    if (lane == 0) red[warp][k] = v;
   }
-  struct P { uint32_t lo, ll; float ph, x, y, w; };
-  __device__ P load(uint32_t i) const { return {b.loss[i], b.lloss[i], b.fphi[i], b.fx[i], b.fy[i], b.fw[i]}; }
-  __device__ void use(uint32_t i, const P &p, float (&a)[K], const Ctx &c) const {
-    uint32_t ll = p.ll;
-    float newly = 0.0f;
-    if (p.ph > c.lim && ll != 1u) {
-      if (p.lo == 0u && ll == 0u) newly = 1.0f;
-      ll = 1u;
-      b.lloss[i] = 1u;
-    }
-    const float pr = rel_phase_f(p.ph - c.pag);
-    b.fphi_r[i] = pr;
-    sc_moments_add(a, pr, p.lo, ll, p.x, p.y, p.w);
-    const bool g = (uint32_t)(p.lo + ll) == 0u;
-    a[8] += ll != 0u ? 1.0f : 0.0f;
-    a[9] += g ? 1.0f : 0.0f;
-    a[10] += g ? p.ph : 0.0f;
-    a[11] += newly;
+  __syncthreads();
+  if (threadIdx.x < K) {
+    float v = 0.0f;
+    for (int w = 0; w < kStatWarps; ++w) v += red[w][threadIdx.x];
+    out[threadIdx.x] = v;
   }
-  __device__ void finalize(const double *s, int tid, int nth) const {
-    __shared__ int redo;
-    __shared__ float red[kBlock / 32][8];
-    __shared__ double mom[8];
-    if (tid == 0) {
-      sc->n_stat_sweeps += 1;
-      BeamStats &st = *b.st;
-      const uint32_t ng = (uint32_t)s[9];
-      st.num_lloss = (uint32_t)s[8];
-      st.num_good = ng;
-      redo = s[11] != 0.0;
-      if (redo) {
-        st.st[PHI_AVG_GOOD] = ng > 0 ? (double)((float)s[10] / (float)ng) + b.phi_ref : -99999;
-      } else {
-        sc_moments_finish(b, s, sc, t, freq, frac, h);
-        st.sc_redo = 0u;
+  __syncthreads();
+}
+
+// blocks [0, nblk) of the launch, whole clusters
+__device__ __forceinline__ void stat_body(const StatArgs &a, uint32_t bid, uint32_t nblk) {
+  const DevBeam &b = a.b;
+  if (b.st->sc_redo != 2u) return;  // uniform over the launch: it is reset behind the last cluster's sum
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  __shared__ float red[kStatWarps][12];
+  __shared__ float sums[12];
+  __shared__ double tot[12];
+  __shared__ int last, again;
+  __shared__ float pag_new;
+  const int tid = threadIdx.x;
+  const uint32_t rank = cl.block_rank();
+  {
+    const double pag_abs = b.st->st[PHI_AVG_GOOD];
+    const float lim = (float)(pag_abs - b.phi_ref + TWOPI + PI), pag = (float)(pag_abs - b.phi_ref);
+    float s[12];
+#pragma unroll
+    for (int k = 0; k < 12; ++k) s[k] = 0.0f;
+    const uint32_t stride = nblk * kStatThreads;
+    for (uint32_t base = bid * kStatThreads + tid; base < b.n; base += kStatBatch * stride) {
+      StatIn p[kStatBatch];
+#pragma unroll
+      for (int u = 0; u < kStatBatch; ++u)
+        if (base + u * stride < b.n) p[u] = stat_load(b, base + u * stride);
+#pragma unroll
+      for (int u = 0; u < kStatBatch; ++u) {
+        const uint32_t i = base + u * stride;
+        if (i >= b.n) continue;
+        uint32_t ll = p[u].ll;
+        float newly = 0.0f;
+        if (p[u].ph > lim && ll != 1u) {
+          if (p[u].lo == 0u && ll == 0u) newly = 1.0f;
+          ll = 1u;
+          b.lloss[i] = 1u;
+        }
+        const float pr = rel_phase_f(p[u].ph - pag);
+        b.fphi_r[i] = pr;
+        sc_moments_add(s, pr, p[u].lo, ll, p[u].x, p[u].y, p[u].w);
+        const bool g = (uint32_t)(p[u].lo + ll) == 0u;
+        s[8] += ll != 0u ? 1.0f : 0.0f;
+        s[9] += g ? 1.0f : 0.0f;
+        s[10] += g ? p[u].ph : 0.0f;
+        s[11] += newly;
       }
+    }
+    stat_block_sum<12>(s, red, sums);
+  }
+  // the block's partials, then one count per cluster
+  float *partf = (float *)a.scr.part;
+  if (tid < 12) partf[(size_t)bid * 12 + tid] = sums[tid];
+  __threadfence();
+  cl.sync();
+  if (rank == 0 && tid == 0) {
+    last = (atomicAdd(a.scr.counter, 1u) == nblk / kStatCluster - 1);
+    __threadfence();
+  }
+  cl.sync();
+  if (!*cl.map_shared_rank(&last, 0)) {
+    cl.sync();  // rank 0's flag stays readable until every CTA has read it
+    return;
+  }
+  __threadfence();
+  // the last cluster: totals in block order, on its first CTA
+  if (rank == 0) {
+    const int lane = tid & 31, warp = tid >> 5;
+    if (warp < 12) {
+      float v = 0.0f;
+      for (uint32_t k = lane; k < nblk; k += 32) v += __ldcg(partf + (size_t)k * 12 + warp);
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+      if (lane == 0) tot[warp] = (double)v;
     }
     __syncthreads();
-    if (redo) {
-      // the loss test changed the good set: the moments again about the new
-      // <phi>_good (Op32ScStats), swept by this last block alone -- a rare
-      // path, kept out of a launch of its own; thread order, then a fixed
-      // shuffle tree and the warps in order
-      const float pag = (float)(b.st->st[PHI_AVG_GOOD] - b.phi_ref);
-      float a[8];
-#pragma unroll
-      for (int k = 0; k < 8; ++k) a[k] = 0.0f;
-      for (uint32_t i = tid; i < b.n; i += nth) {
-        const float pr = rel_phase_f(b.fphi[i] - pag);
-        b.fphi_r[i] = pr;
-        float a12[12];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) a12[k] = a[k];
-        sc_moments_add(a12, pr, b.loss[i], b.lloss[i], b.fx[i], b.fy[i], b.fw[i]);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) a[k] = a12[k];
+    if (tid == 0) {
+      *a.scr.counter = 0u;
+      a.sc->n_stat_sweeps += 1;
+      BeamStats &st = *b.st;
+      const uint32_t ng = (uint32_t)tot[9];
+      st.num_lloss = (uint32_t)tot[8];
+      st.num_good = ng;
+      again = tot[11] != 0.0;
+      if (again) {
+        const double pag_abs = ng > 0 ? (double)((float)tot[10] / (float)ng) + b.phi_ref : -99999;
+        st.st[PHI_AVG_GOOD] = pag_abs;
+        pag_new = (float)(pag_abs - b.phi_ref);
       }
-      const int lane = tid & 31, warp = tid >> 5;
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        float v = a[k];
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-        if (lane == 0) red[warp][k] = v;
-      }
-      __syncthreads();
-      if (tid < 8) {
-        double v = 0.0;
-        for (int w = 0; w < nth / 32; ++w) v += (double)red[w][tid];
-        mom[tid] = v;
-      }
-      __syncthreads();
-      if (tid == 0) {
-        sc_moments_finish(b, mom, sc, t, freq, frac, h);
-        b.st->sc_redo = 0u;
-      }
-      __syncthreads();
     }
-    zero_mesh_tables(sc, t, tid, nth);
   }
-};
+  cl.sync();
+  if (*cl.map_shared_rank(&again, 0)) {
+    const float pag = *cl.map_shared_rank(&pag_new, 0);
+    float s[12];
+#pragma unroll
+    for (int k = 0; k < 12; ++k) s[k] = 0.0f;
+    constexpr uint32_t stride = kStatCluster * kStatThreads;
+    for (uint32_t base = rank * kStatThreads + tid; base < b.n; base += kStatBatch * stride) {
+      StatIn p[kStatBatch];
+#pragma unroll
+      for (int u = 0; u < kStatBatch; ++u)
+        if (base + u * stride < b.n) {
+          p[u] = stat_load(b, base + u * stride);
+          // the flags as the first sweep left them (other CTAs wrote some)
+          p[u].ll = __ldcg(b.lloss + base + u * stride);
+        }
+#pragma unroll
+      for (int u = 0; u < kStatBatch; ++u) {
+        const uint32_t i = base + u * stride;
+        if (i >= b.n) continue;
+        const float pr = rel_phase_f(p[u].ph - pag);
+        b.fphi_r[i] = pr;
+        sc_moments_add(s, pr, p[u].lo, p[u].ll, p[u].x, p[u].y, p[u].w);
+      }
+    }
+    stat_block_sum<8>(s, red, sums);
+    cl.sync();
+    if (rank == 0 && tid < 8) {
+      double v = 0.0;
+      for (int c = 0; c < kStatCluster; ++c) v += (double)*cl.map_shared_rank(sums + tid, c);
+      tot[tid] = v;
+    }
+  }
+  cl.sync();  // no CTA leaves while its sums or rank 0's flags are read
+  if (rank != 0) return;
+  if (tid == 0) {
+    sc_moments_finish(b, tot, a.sc, a.t, a.freq, a.frac, a.h);
+    b.st->sc_redo = 0u;
+  }
+  __syncthreads();
+  zero_mesh_tables(a.sc, a.t, tid, kStatThreads);
+}
+
+__global__ void __cluster_dims__(kStatCluster, 1, 1) __launch_bounds__(kStatThreads) k32_stat_sweeps(StatArgs a) {
+  stat_body(a, blockIdx.x, gridDim.x);
+}
+// lockstep form: every beam's clusters in one flat launch
+template <int B>
+__global__ void __cluster_dims__(kStatCluster, 1, 1) __launch_bounds__(kStatThreads)
+    k32_stat_sweeps_seg(const __grid_constant__ SegArgs<StatArgs, B> a) {
+  uint32_t bid, nblk;
+  const StatArgs &p = a.p[seg_find(a, blockIdx.x, bid, nblk)];
+  stat_body(p, bid, nblk);
+}
+void stat_merge(const std::vector<const Rec *> &recs, SegFork &, cudaStream_t st, cudaStream_t) {
+  seg_chunks<StatArgs>(recs, [&](const auto &a, uint32_t blocks) {
+    k32_stat_sweeps_seg<std::decay_t<decltype(a)>::kB><<<blocks, kStatThreads, 0, st>>>(a);
+  });
+}
+// whole clusters, a batch of particles per thread, at most one CTA per SM
+uint32_t stat_blocks(uint32_t n) {
+  constexpr uint32_t per = kStatCluster * kStatThreads * kStatBatch;
+  const uint32_t clusters = std::min<uint32_t>(std::max<uint32_t>((n + per - 1) / per, 1u), 152u / kStatCluster);
+  return clusters * kStatCluster;
+}
 
 struct Op32AdjMesh {
   static constexpr int K = 2;
@@ -666,16 +777,18 @@ void sc32_stats(const DevBeam &b, ScState *sc, const ScTables &t, const ScKickAr
   }
 }
 
-// one launch of one block per SM: it returns at once when the element map
-// before the kick certified its statistics (every kick of the bench
-// workloads), so its cost there is the launch alone
+// one launch that returns at once when the element map before the kick
+// certified its statistics
 void sc32_stats_after_push(const DevBeam &b, ScState *sc, const ScTables &t, const ScKickArgs &a,
                            PassScratch s, cudaStream_t st) {
-  ScTables u = tables32(t);
-  const Sc32Host h = sc32_host(b, a);
-  launch_pass_f_grid(Op32LlossScStats{b, sc, u, a.freq, a.frac, h}, b.n, s, st, (uint32_t)pass_blocks_f(b.n, 1),
-                     "stats_fallback");
-  if (!recorder()) note_launch();
+  const StatArgs k{b, sc, tables32(t), a.freq, a.frac, sc32_host(b, a), s};
+  const uint32_t blocks = stat_blocks(b.n);
+  if (recorder()) {
+    record("stats_fallback", &stat_merge, blocks, k);
+    return;
+  }
+  k32_stat_sweeps<<<blocks, kStatThreads, 0, st>>>(k);
+  note_launch();
 }
 
 void sc32_mesh(const DevBeam &b, ScState *sc, const ScTables &t, const ScKickArgs &a, PassScratch s,
