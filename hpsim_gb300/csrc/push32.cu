@@ -116,8 +116,8 @@ __global__ void __launch_bounds__(kBlock) k32_push(DevBeam b, Map m, Shift sh) {
 // loss test flags none) and no relative phase lies within |<phi>_good - s|
 // of a wrap boundary (it wraps about <phi>_good as about s).  Without the
 // certificate the finaliser records the counts and <phi>_good and sets
-// sc_redo = 2 for the loss-test and moments sweeps (one grid-wide launch
-// after this one, sc32_stats_after_push); so it does when s lies more than 4
+// sc_redo = 2 for the loss-test and moments sweeps (one launch after this
+// one, sc32_stats_after_push); so it does when s lies more than 4
 // sigma_phi from <phi>_good, where sigma_phi^2 as a difference of FP32
 // moments about s would lose precision.
 template <class Map>
@@ -130,7 +130,9 @@ struct OpPushScStats {
   static constexpr int kMaxFrom = 12;
   static constexpr int kBatch = 4;
   static constexpr bool kFast = true;
+  static constexpr bool kThreadSetup = true;
   using Comb = SumComb;
+  using Stage = Sc32Stage;
   struct Ctx { float s; };
   struct P { Part p; uint32_t ll; };
   DevBeam b;  // carries the synchronous particle after the element
@@ -168,11 +170,15 @@ struct OpPushScStats {
     if (alive) a[12] = fmaxf(a[12], fabsf(f));
     if (q.ll != 1u) a[13] = fmaxf(a[13], p.ph);
   }
-  __device__ void finalize(const double *t, int tid, int nth) const {
+  __device__ void stage_load(Stage &g, int tid, int nth) const {
+    sc32_stage_load(g, b, sc, tid, nth);
+    if (tid == nth - 1) g.c.pag = setup().s;  // until the kick's constants take its place
+  }
+  __device__ void finalize(const double *t, int tid, int nth, Stage &stage) const {
     __shared__ int ok;
     if (tid == 0) {
-      BeamStats &st = *b.st;
-      const float s = setup().s;
+      BeamStats &st = stage.st;
+      const float s = stage.c.pag;
       const uint32_t ng = (uint32_t)t[0];
       const double pag_abs = ng > 0 ? (double)(s + (float)t[1] / (float)ng) + b.phi_ref : -99999.0;
       st.num_good = ng;
@@ -192,13 +198,15 @@ struct OpPushScStats {
         sm[0] = (float)t[9] - (float)t[10] * dm;
         for (int k = 1; k < 8; ++k) sm[k] = t[k + 1];
         st.sc_redo = 0u;
-        sc_moments_finish(b, sm, sc, tb, freq, frac, h);
+        sc_moments_finish(b, sm, stage, freq, frac, h);
       } else {
         st.sc_redo = 2u;
       }
     }
     __syncthreads();
-    if (ok) zero_mesh_tables(sc, tb, tid, nth);
+    if (ok) zero_mesh_tables(&stage.sc, tb, tid, nth);
+    __syncthreads();  // zero_mesh_tables resets the staged on-mesh count
+    sc32_stage_store(stage, b, sc, tb.c32, ok, tid, nth);
   }
 };
 

@@ -152,6 +152,25 @@ struct op_max_from : std::integral_constant<int, Op::K> {};
 template <class Op>
 struct op_max_from<Op, std::void_t<decltype(Op::kMaxFrom)>> : std::integral_constant<int, Op::kMaxFrom> {};
 
+// An Op with `static constexpr bool kThreadSetup = true` has setup() run by
+// every thread instead of once per block: for set-ups of a load or two in
+// FP32, whose latency then overlaps the first particles' loads instead of
+// standing before them behind a barrier.
+template <class Op, class = void>
+struct op_thread_setup : std::false_type {};
+template <class Op>
+struct op_thread_setup<Op, std::void_t<decltype(Op::kThreadSetup)>>
+    : std::integral_constant<bool, Op::kThreadSetup> {};
+
+// An Op with a nested `Stage` has one of them in the last block's shared
+// memory: stage_load(stage, tid, nthreads) runs before that block combines
+// the partials, and finalize takes the stage as a fourth argument.
+struct NoStage {};
+template <class Op, class = void>
+struct op_stage { using type = NoStage; static constexpr bool value = false; };
+template <class Op>
+struct op_stage<Op, std::void_t<typename Op::Stage>> { using type = typename Op::Stage; static constexpr bool value = true; };
+
 template <class C, int MF>
 __device__ inline float comb_k(int k, float a, float b) {
   return k >= MF ? fmaxf(a, b) : C::comb(a, b);
@@ -164,15 +183,21 @@ __device__ __forceinline__ void pass_body_f(const Op &op, uint32_t n, PassScratc
   constexpr int B = op_batch<Op>::value;
   using C = typename Op::Comb;
   if (!op.enabled()) return;
-  __shared__ double sm[kBlock / 32][K];
   __shared__ double tot[K];
   __shared__ int is_last;
-  __shared__ typename Op::Ctx sctx;
-  if (threadIdx.x == 0) sctx = op.setup();
-  __syncthreads();
-  const typename Op::Ctx ctx = sctx;
+  typename Op::Ctx ctx;
+  if constexpr (op_thread_setup<Op>::value) {
+    ctx = op.setup();
+  } else {
+    __shared__ typename Op::Ctx sctx;
+    if (threadIdx.x == 0) sctx = op.setup();
+    __syncthreads();
+    ctx = sctx;
+  }
   constexpr int MF = op_max_from<Op>::value;
   static_assert(MF == K || op_fast<Op>::value, "max slots need the FP32 combine");
+  static_assert(!op_stage<Op>::value || op_fast<Op>::value, "a stage needs the FP32 combine");
+  __shared__ typename op_stage<Op>::type stage;
   float acc[K];
 #pragma unroll
   for (int k = 0; k < K; ++k) acc[k] = k >= MF ? -INFINITY : 0.0f;
@@ -193,42 +218,72 @@ __device__ __forceinline__ void pass_body_f(const Op &op, uint32_t n, PassScratc
 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if constexpr (op_fast<Op>::value) {
-    // FP32 partials: warps summed in order per block, blocks by the warps of
-    // the last block (slot k by warp k mod 8; lane l takes blocks l, l + 32,
-    // ...; then a fixed shuffle tree).  No FP64 arithmetic on the
-    // reduction's critical path.
+    // FP32 partials, no FP64 arithmetic on the reduction's critical path:
+    // warps summed in order per block; then the last block's thread t takes
+    // the K slots of blocks t, t + 256, ... (every load of a row in flight at
+    // once: the 304 rows of a large beam's 14 slots cost one or two memory
+    // round trips, where a warp per slot took several per slot), the lanes by
+    // a fixed shuffle tree and the warps in order.  A pass of one block has
+    // its totals at once.
     __shared__ float smf[kBlock / 32][K];
     float *partf = (float *)scr.part;
+    auto warps = [&](const float (&a)[K]) {
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-      float v = acc[k];
+      for (int k = 0; k < K; ++k) {
+        float v = a[k];
 #pragma unroll
-      for (int off = 16; off > 0; off >>= 1) v = comb_k<C, MF>(k, v, __shfl_down_sync(0xffffffffu, v, off));
-      if (lane == 0) smf[warp][k] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x < K) {
-      const int k = threadIdx.x;
+        for (int off = 16; off > 0; off >>= 1) v = comb_k<C, MF>(k, v, __shfl_down_sync(0xffffffffu, v, off));
+        if (lane == 0) smf[warp][k] = v;
+      }
+    };
+    auto block_sum = [&](int k, int nw) {
       float v = k >= MF ? -INFINITY : 0.0f;
-      for (int w = 0; w < kBlock / 32; ++w) v = comb_k<C, MF>(k, v, smf[w][k]);
-      partf[bid * K + k] = v;
-    }
-    __threadfence();
+      for (int w = 0; w < nw; ++w) v = comb_k<C, MF>(k, v, smf[w][k]);
+      return v;
+    };
+    warps(acc);
     __syncthreads();
-    if (threadIdx.x == 0) is_last = (atomicAdd(scr.counter, 1u) == nblk - 1);
-    __syncthreads();
-    if (!is_last) return;
-    __threadfence();
-    // warp w combines slots w, w + 8, ...: the slots' chains run side by side
-    for (int k = warp; k < K; k += kBlock / 32) {
-      float v = k >= MF ? -INFINITY : 0.0f;
-      for (uint32_t b = lane; b < nblk; b += 32) v = comb_k<C, MF>(k, v, __ldcg(partf + (size_t)b * K + k));
+    if (nblk == 1) {
+      if constexpr (op_stage<Op>::value) op.stage_load(stage, threadIdx.x, blockDim.x);
+      if (threadIdx.x < K) tot[threadIdx.x] = (double)block_sum(threadIdx.x, kBlock / 32);
+      __syncthreads();
+    } else {
+      if (threadIdx.x < K) partf[bid * K + threadIdx.x] = block_sum(threadIdx.x, kBlock / 32);
+      __threadfence();
+      __syncthreads();
+      if (threadIdx.x == 0) is_last = (atomicAdd(scr.counter, 1u) == nblk - 1);
+      __syncthreads();
+      if (!is_last) return;
+      __threadfence();
+      if constexpr (op_stage<Op>::value) op.stage_load(stage, threadIdx.x, blockDim.x);
+      const int nw = min(kBlock / 32, (int)((nblk + 31) / 32));  // warps with rows to take
+      if (warp < nw) {
 #pragma unroll
-      for (int off = 16; off > 0; off >>= 1) v = comb_k<C, MF>(k, v, __shfl_down_sync(0xffffffffu, v, off));
-      if (lane == 0) tot[k] = (double)v;
+        for (int k = 0; k < K; ++k) acc[k] = k >= MF ? -INFINITY : 0.0f;
+        for (uint32_t b = threadIdx.x; b < nblk; b += kBlock) {
+          float row[K];
+          if constexpr (K % 2 == 0) {
+#pragma unroll
+            for (int k = 0; k < K / 2; ++k) {
+              const float2 v = __ldcg((const float2 *)(partf + (size_t)b * K) + k);
+              row[2 * k] = v.x;
+              row[2 * k + 1] = v.y;
+            }
+          } else {
+#pragma unroll
+            for (int k = 0; k < K; ++k) row[k] = __ldcg(partf + (size_t)b * K + k);
+          }
+#pragma unroll
+          for (int k = 0; k < K; ++k) acc[k] = comb_k<C, MF>(k, acc[k], row[k]);
+        }
+        warps(acc);
+      }
+      __syncthreads();
+      if (threadIdx.x < K) tot[threadIdx.x] = (double)block_sum(threadIdx.x, nw);
+      __syncthreads();
     }
-    __syncthreads();
   } else {
+    __shared__ double sm[kBlock / 32][K];
 #pragma unroll
     for (int k = 0; k < K; ++k) {
       float v = acc[k];
@@ -250,7 +305,8 @@ __device__ __forceinline__ void pass_body_f(const Op &op, uint32_t n, PassScratc
     __threadfence();
     combine_partials<C, K>(scr.part, nblk, sm, tot);
   }
-  op.finalize(tot, threadIdx.x, blockDim.x);
+  if constexpr (op_stage<Op>::value) op.finalize(tot, threadIdx.x, blockDim.x, stage);
+  else op.finalize(tot, threadIdx.x, blockDim.x);
   __syncthreads();
   if (threadIdx.x == 0) *scr.counter = 0u;
 }

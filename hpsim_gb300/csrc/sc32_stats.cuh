@@ -124,9 +124,39 @@ __device__ void sc32_consts(const BeamStats &st, const DevBeam &b, const ScState
   c->green_c1 = h.c1;
 }
 
-// The decision and the kick constants on local copies of the solver state:
-// one burst of loads, one burst of stores, and no load waiting behind a
-// store that might alias it.
+// What the thread that finalises a kick's statistics reads and writes besides
+// the totals: the beam's scalars, the solver's state and the kick's
+// constants.  A block stages it in shared memory (sc32_stage_load) while the
+// partial sums arrive, the finalising thread works on it there, and the block
+// writes it back (sc32_stage_store): no chain of global loads and stores
+// behind the totals.
+struct Sc32Stage {
+  BeamStats st;
+  ScState sc;
+  Sc32Consts c;
+};
+static_assert(sizeof(BeamStats) % 4 == 0 && sizeof(ScState) % 4 == 0 && sizeof(Sc32Consts) % 4 == 0, "word copies");
+
+__device__ inline void sc32_stage_load(Sc32Stage &g, const DevBeam &b, const ScState *sc, int tid, int nth) {
+  constexpr int ns = sizeof(BeamStats) / 4, nc = sizeof(ScState) / 4;
+  for (int k = tid; k < ns + nc; k += nth) {
+    if (k < ns) ((uint32_t *)&g.st)[k] = ((const uint32_t *)b.st)[k];
+    else ((uint32_t *)&g.sc)[k - ns] = ((const uint32_t *)sc)[k - ns];
+  }
+}
+// with_kick: the solver's state and the kick's constants too
+__device__ inline void sc32_stage_store(const Sc32Stage &g, const DevBeam &b, ScState *sc, Sc32Consts *c, bool with_kick,
+                                        int tid, int nth) {
+  constexpr int ns = sizeof(BeamStats) / 4, nc = sizeof(ScState) / 4, nk = sizeof(Sc32Consts) / 4;
+  const int n = with_kick ? ns + nc + nk : ns;
+  for (int k = tid; k < n; k += nth) {
+    if (k < ns) ((uint32_t *)b.st)[k] = ((const uint32_t *)&g.st)[k];
+    else if (k < ns + nc) ((uint32_t *)sc)[k - ns] = ((const uint32_t *)&g.sc)[k - ns];
+    else ((uint32_t *)c)[k - ns - nc] = ((const uint32_t *)&g.c)[k - ns - nc];
+  }
+}
+
+// The decision and the kick constants on local copies of the solver state.
 __device__ void sc32_decide_consts(const BeamStats &st, const DevBeam &b, ScState *sc, Sc32Consts *c32,
                                    const Sc32Host &h, double freq, double frac) {
   ScState s = *sc;
@@ -137,13 +167,9 @@ __device__ void sc32_decide_consts(const BeamStats &st, const DevBeam &b, ScStat
   *c32 = c;
 }
 
-
 // The SCHEFF moments from their totals s[0..7] (FP32 arithmetic, see
-// Sc32Host), then, with a solver, the decision and the kick's constants
-// (thread 0); the caller zeroes the tables afterwards.
-__device__ void sc_moments_finish(const DevBeam &b, const double *s, ScState *sc, const ScTables &t, double freq,
-                                  double frac, const Sc32Host &h) {
-  BeamStats st = *b.st;  // local copy, written back once
+// Sc32Host) into the beam's scalars (num_loss and num_good set), one thread
+__device__ inline void sc_moments(const DevBeam &b, BeamStats &st, const double *s) {
   const float isv = 1.0f / (float)(uint32_t)(b.n - st.num_loss), ing = 1.0f / (float)st.num_good;
   st.st[PHI_AVG_R] = (float)s[0] * isv;
   const float pa = (float)s[1] * ing, pa2 = (float)s[2] * ing;
@@ -154,8 +180,24 @@ __device__ void sc_moments_finish(const DevBeam &b, const double *s, ScState *sc
   st.st[Y_AVG_GOOD] = ya;
   st.st[Y_SIG_GOOD] = sqrtf(y2 - ya * ya);
   st.st[W_AVG_GOOD] = st.num_good > 0 ? (double)((float)s[7] * ing) + b.w_ref : -99999;
+}
+
+// The moments from their totals, then, with a solver, the decision and the
+// kick's constants (thread 0); the caller zeroes the tables afterwards.
+__device__ void sc_moments_finish(const DevBeam &b, const double *s, ScState *sc, const ScTables &t, double freq,
+                                  double frac, const Sc32Host &h) {
+  BeamStats st = *b.st;  // local copy, written back once
+  sc_moments(b, st, s);
   *b.st = st;
   if (sc) sc32_decide_consts(st, b, sc, t.c32, h, freq, frac);
+}
+// the same on a staged copy
+__device__ void sc_moments_finish(const DevBeam &b, const double *s, Sc32Stage &g, double freq, double frac,
+                                  const Sc32Host &h) {
+  BeamStats st = g.st;
+  sc_moments(b, st, s);
+  g.st = st;
+  sc32_decide_consts(st, b, &g.sc, &g.c, h, freq, frac);
 }
 
 // the SCHEFF moments' per-particle terms: 0 mean relative phase of the live

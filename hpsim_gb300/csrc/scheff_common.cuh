@@ -83,14 +83,25 @@ __device__ inline void scheff_decide(const DevBeam &b, ScState *s, double freq, 
   }
 }
 
+// The tables a kick starts from: charge bins at zero for a solve (16 bytes a
+// store: the bins of a 32 x 128 mesh are 8 stores a thread of the one block
+// that does this), and the field table at zero only after a resize without a
+// solve -- the contraction (or a surrogate's field) overwrites every entry of
+// the table otherwise.
 __device__ inline void zero_mesh_tables(ScState *s, const ScTables &t, int tid, int nth) {
   if (!(s->remesh || s->resized)) return;
-  uint32_t nb = s->nx * s->nz, nf = (s->nx + 1) * (s->nz + 1) * 2;
-  for (uint32_t k = tid; k < nb; k += nth) t.bin_fx[k] = 0ull;
-  if (t.fld2)
-    for (uint32_t k = tid; k < nf; k += nth) t.fld2[k] = 0.0;
-  if (t.ffld2)
-    for (uint32_t k = tid; k < nf; k += nth) t.ffld2[k] = 0.0f;
+  const uint32_t nb = s->nx * s->nz;
+  if (nb % 2 == 0)
+    for (uint32_t k = tid; k < nb / 2; k += nth) ((ulonglong2 *)t.bin_fx)[k] = make_ulonglong2(0ull, 0ull);
+  else
+    for (uint32_t k = tid; k < nb; k += nth) t.bin_fx[k] = 0ull;
+  if (!s->remesh) {
+    const uint32_t nf = (s->nx + 1) * (s->nz + 1) * 2;
+    if (t.fld2)
+      for (uint32_t k = tid; k < nf; k += nth) t.fld2[k] = 0.0;
+    if (t.ffld2)
+      for (uint32_t k = tid; k < nf; k += nth) t.ffld2[k] = 0.0f;
+  }
   if (tid == 0 && s->remesh) s->num_on_mesh = 0u;
 }
 }  // namespace hps
