@@ -110,26 +110,17 @@ struct Op32Emittance {
     a[10] += pr; a[11] += pr * pr; a[12] += w; a[13] += w * w; a[14] += pr * w;
   }
   __device__ void finalize(const double *t, int tid, int) const {
+    __shared__ double pl[3][5];
+    plane_moments(t, surv(b), b.w_ref + (double)b.fw[0], b.mass, pl);
     if (tid) return;
-    double sv = surv(b);
-    double g1 = (b.w_ref + (double)b.fw[0]) / b.mass, bg = sqrt(g1 * (g1 + 2.0));
-    for (int pl = 0; pl < 2; ++pl) {
-      const double *q = t + 5 * pl;
-      double x = q[0] / sv, x2 = q[1] / sv, xp = q[2] / sv, xp2 = q[3] / sv, xxp = q[4] / sv;
-      double *s = b.st->st;
-      s[pl ? Y_AVG : X_AVG] = x;
-      s[pl ? Y_SIG : X_SIG] = sqrt(x2 - x * x);
-      s[pl ? YP_AVG : XP_AVG] = xp;
-      s[pl ? YP_SIG : XP_SIG] = sqrt(xp2 - xp * xp);
-      s[pl ? Y_EMIT : X_EMIT] = sqrt((x2 - x * x) * (xp2 - xp * xp) - (xxp - x * xp) * (xxp - x * xp)) * bg;
-    }
-    double phi = t[10] / sv, phi2 = t[11] / sv, w = t[12] / sv, w2 = t[13] / sv, pw = t[14] / sv;
-    double pv = phi2 - phi * phi, wv = w2 - w * w, cv = pw - phi * w;
-    b.st->st[PHI_AVG_R] = phi;
-    b.st->st[W_AVG] = w + b.w_ref;
-    b.st->st[PHI_SIG_R] = sqrt(pv);
-    b.st->st[W_SIG] = sqrt(wv);
-    b.st->st[Z_EMIT] = sqrt(pv * wv - cv * cv);
+    double *s = b.st->st;
+    s[X_AVG] = pl[0][0]; s[X_SIG] = pl[0][1]; s[XP_AVG] = pl[0][2]; s[XP_SIG] = pl[0][3]; s[X_EMIT] = pl[0][4];
+    s[Y_AVG] = pl[1][0]; s[Y_SIG] = pl[1][1]; s[YP_AVG] = pl[1][2]; s[YP_SIG] = pl[1][3]; s[Y_EMIT] = pl[1][4];
+    s[PHI_AVG_R] = pl[2][0];
+    s[PHI_SIG_R] = pl[2][1];
+    s[W_AVG] = pl[2][2] + b.w_ref;
+    s[W_SIG] = pl[2][3];
+    s[Z_EMIT] = pl[2][4];
   }
 };
 
@@ -228,44 +219,26 @@ struct Op32Monitor {
     a[11] += pr; a[12] += pr * pr; a[13] += w; a[14] += w * w; a[15] += pr * w;
   }
   __device__ void finalize(const double *s, int tid, int) const {
-    if (tid) return;
-    double *o = out;
-    for (int k = 0; k < HPS_NMON; ++k) o[k] = 0.0;
-    double m = s[0];
-    o[HPS_MON_NALIVE] = m;
-    o[HPS_MON_NGOOD] = s[16];
-    double w0 = b.w_ref + (double)b.fw[0];
-    double g1 = w0 / b.mass, bg = sqrt(g1 * (g1 + 2.0));
-    if (m > 0) {
-      for (int pl = 0; pl < 2; ++pl) {
-        const double *q = s + 1 + 5 * pl;
-        double a = q[0] / m, a2 = q[1] / m, ap = q[2] / m, ap2 = q[3] / m, aap = q[4] / m;
-        int base = pl ? HPS_MON_Y_AVG : HPS_MON_X_AVG;
-        o[base] = a;
-        o[base + 1] = sqrt(a2 - a * a);
-        o[base + 2] = ap;
-        o[base + 3] = sqrt(ap2 - ap * ap);
-        o[base + 4] = sqrt((a2 - a * a) * (ap2 - ap * ap) - (aap - a * ap) * (aap - a * ap)) * bg;
-      }
-      double p = s[11] / m, p2 = s[12] / m, w = s[13] / m, w2 = s[14] / m, pw = s[15] / m;
-      double pv = p2 - p * p, wv = w2 - w * w, cv = pw - p * w;
-      o[HPS_MON_PHIR_AVG] = p;
-      o[HPS_MON_PHIR_SIG] = sqrt(pv);
-      o[HPS_MON_W_AVG] = w + b.w_ref;
-      o[HPS_MON_W_SIG] = sqrt(wv);
-      o[HPS_MON_Z_EMIT] = sqrt(pv * wv - cv * cv);
-    }
-    o[HPS_MON_W0] = w0;
-    o[HPS_MON_PHI0] = b.phi_ref + (double)b.fphi[0];
-    if (sc) {
-      o[HPS_MON_SC_DR] = sc->dr;
-      o[HPS_MON_SC_DZ] = sc->dz;
-      o[HPS_MON_SC_REMESH] = (double)sc->n_solves;
-      o[HPS_MON_SC_ONMESH] = (double)sc->num_on_mesh;
-    }
-    o[HPS_MON_ELEM] = (double)elem;
+    __shared__ double pl[3][5];
+    const double m = s[0], w0 = b.w_ref + (double)b.fw[0];
+    if (m > 0) plane_moments(s + 1, m, w0, b.mass, pl);
+    if (tid >= HPS_NMON) return;
+    double v = 0.0;  // record entry tid
+    if (tid == HPS_MON_NALIVE) v = m;
+    else if (tid == HPS_MON_NGOOD) v = s[16];
+    else if (tid <= HPS_MON_Z_EMIT) v = m > 0 ? (&pl[0][0])[tid - HPS_MON_X_AVG] + (tid == HPS_MON_W_AVG ? b.w_ref : 0.0) : 0.0;
+    else if (tid == HPS_MON_W0) v = w0;
+    else if (tid == HPS_MON_PHI0) v = b.phi_ref + (double)b.fphi[0];
+    else if (tid == HPS_MON_SC_DR) v = sc ? sc->dr : 0.0;
+    else if (tid == HPS_MON_SC_DZ) v = sc ? sc->dz : 0.0;
+    else if (tid == HPS_MON_SC_REMESH) v = sc ? (double)sc->n_solves : 0.0;  // cumulative; the host takes differences
+    else if (tid == HPS_MON_SC_ONMESH) v = sc ? (double)sc->num_on_mesh : 0.0;
+    else if (tid == HPS_MON_ELEM) v = (double)elem;
+    out[tid] = v;
   }
 };
+static_assert(HPS_MON_X_AVG == 2 && HPS_MON_Y_AVG == HPS_MON_X_AVG + 5 && HPS_MON_PHIR_AVG == HPS_MON_X_AVG + 10 &&
+              HPS_MON_Z_EMIT == HPS_MON_X_AVG + 14, "a monitor record holds the planes' moments in a row");
 
 #define PARTICLES(b) for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < (b).n; i += gridDim.x * blockDim.x)
 

@@ -193,8 +193,12 @@ __host__ __device__ inline void ref_launch(uint32_t n, uint32_t *grid, uint32_t 
   else { *grid = 1; *blck = nt; }
 }
 
+// Blocks of an FP64 pass: one particle a thread until every SM has two blocks
+// (the per-particle FP64 arithmetic is the time, and four particles a thread
+// left a 65,536-particle beam on 64 of 152 SMs), then up to four a thread.
 inline int pass_blocks(uint32_t n) {
-  uint32_t b = (n + 4 * kBlock - 1) / (4 * kBlock);
+  const uint32_t one = (uint32_t)(((uint64_t)n + kBlock - 1) / kBlock), four = (uint32_t)(((uint64_t)n + 4 * kBlock - 1) / (4 * kBlock));
+  uint32_t b = one < 304u ? one : four > 304u ? four : 304u;
   if (b < 1) b = 1;
   if (b > (uint32_t)kMaxPassBlocks) b = kMaxPassBlocks;
   return (int)b;

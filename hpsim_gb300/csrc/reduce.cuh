@@ -5,9 +5,9 @@
 // (src/beam/src/beam.cu:411-436, 651-678); about 30 launches and 5 blocking
 // scalar reads per space-charge kick.  Here one launch does all of it: every
 // block reduces its grid-stride share of the particles (each thread in index
-// order, warps by a fixed shuffle tree, warps in index order), writes one
+// order, warps by a fixed shuffle order, warps in index order), writes one
 // partial per block, and the last block to finish (threadfence + counter)
-// sums the partials in block order and runs the finaliser.  The result is
+// sums the partials in a fixed order and runs the finaliser.  The result is
 // bitwise reproducible for a given particle count, and the per-particle
 // callback may also write per-particle outputs (relative phase, loss flags)
 // in the same sweep.
@@ -36,33 +36,101 @@ struct MaxComb {  // MaxR2PhiReduceKernel starts from 0 (beam_kernel.cu:809-810)
   __device__ static float comb(float a, float b) { return a < b ? b : a; }
 };
 
-// Total of the per-block partials, taken by the last block: thread t combines
-// blocks t, t + blockDim, ... in order (independent loads, so the sweep runs
-// at memory parallelism rather than one L2 round trip per block), then the
-// lanes by a fixed shuffle tree and the warps in order.
+// Totals over a warp of K accumulators a lane, K <= 32, by folding: a step
+// halves the lanes' distance and the accumulators a lane still carries (it
+// sends one half to its partner and keeps the other), so K sums cost about
+// K + log2(32 / K) combinations a lane where a shuffle tree for each costs
+// 5 K.  The lanes whose low bits are zero hold the totals: true with the slot
+// number, in an order fixed by the lane numbers.
+template <class C, int K, class T>
+__device__ __forceinline__ bool warp_fold(const T (&a)[K], int lane, int &slot, T &total) {
+  constexpr int P = K > 16 ? 32 : K > 8 ? 16 : K > 4 ? 8 : K > 2 ? 4 : K > 1 ? 2 : 1;
+  T v[P];
+#pragma unroll
+  for (int k = 0; k < P; ++k) v[k] = k < K ? a[k] : (T)C::ident();
+  int base = 0, off = 16;
+#pragma unroll
+  for (int cnt = P / 2; cnt >= 1; cnt /= 2, off /= 2) {
+    const bool hi = lane & off;
+#pragma unroll
+    for (int k = 0; k < cnt; ++k) {
+      const T keep = hi ? v[k + cnt] : v[k], send = hi ? v[k] : v[k + cnt];
+      v[k] = C::comb(keep, __shfl_xor_sync(0xffffffffu, send, off));
+    }
+    if (hi) base += cnt;
+  }
+  T x = v[0];
+#pragma unroll
+  for (int o = 16 / P; o > 0; o /= 2) x = C::comb(x, __shfl_xor_sync(0xffffffffu, x, o));
+  slot = base;
+  total = x;
+  return (lane & (32 / P - 1)) == 0 && base < K;
+}
+
+// Rows per slot that the FP64 combine's first step leaves: as many as the
+// block has threads for, within a short second step.
+template <int K>
+constexpr int combine_rows() {
+  return K <= 4 ? 64 : kBlock / K < 16 ? (kBlock / K > 8 ? kBlock / K : 8) : 16;
+}
+
+// Total of the per-block partials, taken by the last block: thread t sums
+// slot t mod K over rows t / K, t / K + G, ... (eight loads in flight, so the
+// sweep costs a memory round trip or two), then K threads the G rows left.
+// FP64 additions run at two a cycle on an SM, and a warp's instruction takes
+// its 64 cycles whatever lanes it has: a shuffle tree per slot (5 K additions
+// by every warp) was 5 us of a beam statistics record's 17 slots, this order
+// does one addition per partial.
 template <class C, int K>
 __device__ inline void combine_partials(const double *part, uint32_t nb, double (*sm)[K], double *tot) {
-  double v[K];
-#pragma unroll
-  for (int k = 0; k < K; ++k) v[k] = C::ident();
-  for (uint32_t b = threadIdx.x; b < nb; b += blockDim.x) {
-#pragma unroll
-    for (int k = 0; k < K; ++k) v[k] = C::comb(v[k], __ldcg(part + (size_t)b * K + k));
-  }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  __syncthreads();
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    double x = v[k];
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) x = C::comb(x, __shfl_down_sync(0xffffffffu, x, off));
-    if (lane == 0) sm[warp][k] = x;
-  }
-  __syncthreads();
-  if (threadIdx.x < K) {
+  constexpr int G = combine_rows<K>();
+  static_assert(G * K <= kBlock, "a thread per row and slot");
+  const int t = threadIdx.x;
+  if (t < G * K) {
     double x = C::ident();
-    for (int w = 0; w < kBlock / 32; ++w) x = C::comb(x, sm[w][threadIdx.x]);
-    tot[threadIdx.x] = x;
+    for (uint32_t r = t / K; r < nb; r += 8 * G) {
+      double v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = r + u * G < nb ? __ldcg(part + (size_t)(r + u * G) * K + t % K) : C::ident();
+      x = C::comb(x, C::comb(C::comb(C::comb(v[0], v[1]), C::comb(v[2], v[3])),
+                             C::comb(C::comb(v[4], v[5]), C::comb(v[6], v[7]))));
+    }
+    sm[t / K][t % K] = x;
+  }
+  __syncthreads();
+  if (t < K) {
+    double v[4] = {C::ident(), C::ident(), C::ident(), C::ident()};
+#pragma unroll
+    for (int g = 0; g < G; ++g) v[g & 3] = C::comb(v[g & 3], sm[g][t]);
+    tot[t] = C::comb(C::comb(v[0], v[1]), C::comb(v[2], v[3]));
+  }
+  __syncthreads();
+}
+
+// From the totals q of three coordinate pairs (a, a^2, b, b^2, a b of the
+// horizontal, vertical and longitudinal plane) over m particles: o[plane][0..4]
+// = <a>, sigma_a, <b>, sigma_b, emittance, the transverse emittances times
+// beta gamma of kinetic energy w0.  Every thread of the block calls it.  A
+// dependent FP64 quotient or root costs about a third of a microsecond on one
+// thread, so the 15 quotients are taken by 15 threads and the 9 roots by 9.
+__device__ inline void plane_moments(const double *q, double m, double w0, double mass, double (*o)[5]) {
+  __shared__ double mean[15], bg;
+  const int t = threadIdx.x;
+  if (t < 15) mean[t] = q[t] / m;
+  if (t == 32) {
+    const double g1 = w0 / mass;
+    bg = sqrt(g1 * (g1 + 2.0));
+  }
+  __syncthreads();
+  if (t < 9) {
+    const int pl = t / 3, kind = t % 3;
+    const double *c = mean + 5 * pl;
+    const double a = c[0], a2 = c[1], b = c[2], b2 = c[3], ab = c[4];
+    const double va = a2 - a * a, vb = b2 - b * b, cv = ab - a * b;
+    const double r = sqrt(kind == 0 ? va : kind == 1 ? vb : va * vb - cv * cv);
+    if (kind == 0) { o[pl][0] = a; o[pl][1] = r; }
+    else if (kind == 1) { o[pl][2] = b; o[pl][3] = r; }
+    else o[pl][4] = pl < 2 ? r * bg : r;
   }
   __syncthreads();
 }
@@ -84,20 +152,18 @@ __global__ void __launch_bounds__(kBlock) pass_kernel(Op op, uint32_t n, PassScr
   const uint32_t stride = gridDim.x * blockDim.x;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) op.particle(i, acc);
 
-  __shared__ double sm[kBlock / 32][K];
+  __shared__ double sm[combine_rows<K>()][K];
   __shared__ double tot[K];
   __shared__ int is_last;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    double v = acc[k];
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) v = C::comb(v, __shfl_down_sync(0xffffffffu, v, off));
-    if (lane == 0) sm[warp][k] = v;
+  {
+    int slot;
+    double v;
+    if (warp_fold<C>(acc, threadIdx.x & 31, slot, v)) sm[threadIdx.x >> 5][slot] = v;
   }
   __syncthreads();
   if (threadIdx.x < K) {
     double v = C::ident();
+#pragma unroll
     for (int w = 0; w < kBlock / 32; ++w) v = C::comb(v, sm[w][threadIdx.x]);
     scr.part[blockIdx.x * K + threadIdx.x] = v;
   }
@@ -283,7 +349,7 @@ __device__ __forceinline__ void pass_body_f(const Op &op, uint32_t n, PassScratc
       __syncthreads();
     }
   } else {
-    __shared__ double sm[kBlock / 32][K];
+    __shared__ double sm[combine_rows<K>()][K];
 #pragma unroll
     for (int k = 0; k < K; ++k) {
       float v = acc[k];
@@ -294,6 +360,7 @@ __device__ __forceinline__ void pass_body_f(const Op &op, uint32_t n, PassScratc
     __syncthreads();
     if (threadIdx.x < K) {
       double v = C::ident();
+#pragma unroll
       for (int w = 0; w < kBlock / 32; ++w) v = C::comb(v, sm[w][threadIdx.x]);
       scr.part[bid * K + threadIdx.x] = v;
     }
@@ -391,6 +458,7 @@ __device__ inline double rel_phase(double phi, double ref) {
   double tmp = phi - ref + PI;
   double sign = 1.0;
   if (tmp < 0) { sign = -1.0; tmp = -tmp; }
+  if (tmp < TWOPI) return sign * (tmp - PI);  // fmod returns it as it is
   return sign * (fmod(tmp, TWOPI) - PI);
 }
 

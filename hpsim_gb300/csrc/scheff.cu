@@ -102,20 +102,37 @@ struct OpScStats {
     a[7] += b.w[i];
   }
   __device__ void finalize(const double *s, int tid, int nth) const {
+    // independent quotients and roots on a thread each (a dependent FP64
+    // quotient costs about a third of a microsecond)
+    __shared__ double q[8], sig[3];
+    __shared__ ScheffKin kin;
+    if (tid < 8) {
+      const double sv = surv(b), ng = b.st->num_good;
+      q[tid] = s[tid] / (tid == 1 || tid == 2 || tid == 7 ? ng : sv);
+    }
+    __syncthreads();
+    if (tid < 3) {  // sigma of phi, x, y
+      const double a = q[1 + 2 * tid];
+      sig[tid] = sqrt(q[2 + 2 * tid] - a * a);
+    } else if (tid == 32) {
+      q[7] = b.st->num_good > 0 ? q[7] : -99999;
+      const ScheffKin k = scheff_kin(q[7], b.mass);
+      kin.gamma = k.gamma;
+      kin.beta = k.beta;
+    } else if (tid == 64) {
+      kin.lmbd = 299.792458 / freq;
+    }
+    __syncthreads();
     if (tid == 0) {
       BeamStats &st = *b.st;
-      double sv = surv(b);
-      double ng = st.num_good;
-      st.st[PHI_AVG_R] = s[0] / sv;
-      double pa = s[1] / ng, pa2 = s[2] / ng;
-      st.st[PHI_SIG_GOOD] = sqrt(pa2 - pa * pa);
-      double xa = s[3] / sv, x2 = s[4] / sv, ya = s[5] / sv, y2 = s[6] / sv;
-      st.st[X_AVG_GOOD] = xa;
-      st.st[X_SIG_GOOD] = sqrt(x2 - xa * xa);
-      st.st[Y_AVG_GOOD] = ya;
-      st.st[Y_SIG_GOOD] = sqrt(y2 - ya * ya);
-      st.st[W_AVG_GOOD] = st.num_good > 0 ? s[7] / st.num_good : -99999;
-      if (sc) scheff_decide(b, sc, freq, frac);
+      st.st[PHI_AVG_R] = q[0];
+      st.st[PHI_SIG_GOOD] = sig[0];
+      st.st[X_AVG_GOOD] = q[3];
+      st.st[X_SIG_GOOD] = sig[1];
+      st.st[Y_AVG_GOOD] = q[5];
+      st.st[Y_SIG_GOOD] = sig[2];
+      st.st[W_AVG_GOOD] = q[7];
+      if (sc) scheff_decide(b, sc, freq, frac, kin);
     }
     if (!sc) return;
     __syncthreads();
@@ -151,7 +168,11 @@ struct OpAdjMesh {
 // Scheff::Start with num_particle <= 2: statistics are not refreshed, the
 // decision still runs on whatever they hold.
 __global__ void k_decide_only(DevBeam b, ScState *sc, ScTables t, double freq, double frac) {
-  if (threadIdx.x == 0) scheff_decide(b, sc, freq, frac);
+  if (threadIdx.x == 0) {
+    ScheffKin kin = scheff_kin(b.st->st[W_AVG_GOOD], b.mass);
+    kin.lmbd = 299.792458 / freq;
+    scheff_decide(b, sc, freq, frac, kin);
+  }
   __syncthreads();
   zero_mesh_tables(sc, t, threadIdx.x, blockDim.x);
 }

@@ -30,18 +30,25 @@ __device__ inline void mesh_size(ScState *s, double partial_r, double partial_z,
   }
 }
 
+// Lorentz factors of the mean energy and the beam's wavelength
+struct ScheffKin {
+  double gamma, beta, lmbd;
+};
+__device__ inline ScheffKin scheff_kin(double ke, double mass) {
+  const double gamma = ke / mass + 1.0;
+  return {gamma, sqrt(1.0 - 1.0 / (gamma * gamma)), 0.0};
+}
+
 // The host-side body of Scheff::Start after the statistics
 // (space_charge.cpp:86-138) plus UpdateMeshKernelCall (space_charge.cu:122-138).
-__device__ inline void scheff_decide(const DevBeam &b, ScState *s, double freq, double frac) {
+__device__ inline void scheff_decide(const DevBeam &b, ScState *s, double freq, double frac, const ScheffKin &kin) {
   const BeamStats &st = *b.st;
   uint32_t good_cnt = st.num_good;
   double sigphi = b.n < 2 ? 0.0 : st.st[PHI_SIG_GOOD];
   double sigx = b.n < 2 ? 0.0 : st.st[X_SIG_GOOD];
   double sigy = b.n < 2 ? 0.0 : st.st[Y_SIG_GOOD];
   double ke = st.st[W_AVG_GOOD];
-  double gamma = (double)ke / b.mass + 1.0;
-  double beta = sqrt(1.0 - 1.0 / (gamma * gamma));
-  double lmbd = 299.792458 / freq;
+  const double gamma = kin.gamma, beta = kin.beta, lmbd = kin.lmbd;
   double sigz = sigphi * 0.5 / 3.14159265 * beta * lmbd;
   double sigr = sqrt(sigx * sigx + sigy * sigy);
   double cratior = sigr * sigz;
