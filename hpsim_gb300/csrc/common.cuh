@@ -136,33 +136,48 @@ __host__ __device__ inline RefK make_refk(double w, double mass) {
   return r;
 }
 
+// Square roots, reciprocal square roots and reciprocals by the hardware
+// approximations (within two ulp), and the quotient they give, for the
+// per-particle sweeps.  The .ftz forms take subnormal operands and results as
+// zero: quantities below 1e-38 of the coordinates' own units.  The other forms
+// scale their operands around every approximation, three to four more
+// instructions each in sweeps that are bound by their instructions.
+__device__ __forceinline__ float sqrt_fast(float x) {
+  float r;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float rsqrt_fast(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float rcp_fast(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float div_fast(float x, float y) { return x * rcp_fast(y); }
+
 // 1/beta_i - 1/beta_ref for a particle dw above the reference, computed from
 // beta_i^2 - beta_r^2 = (gamma_i^2 - gamma_r^2)/(gamma_i^2 gamma_r^2) so the
 // difference keeps FP32 relative precision:
 //   1/beta_i - 1/beta_r = -(dgamma (gamma_i + gamma_r)) /
 //                          (gamma_i gamma_r^2 (beta_i + beta_r) (beta gamma)_i beta_r)
 // (one division); also returns g_i = W_i/m, beta_i and (beta gamma)_i.
-// square root by the hardware approximation (sqrt.approx.f32: within about
-// an ulp; +0 -> +0, negative -> NaN), for the per-particle sweeps
-__device__ __forceinline__ float sqrt_fast(float x) {
-  float r;
-  asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
-
 __device__ inline float dinvb(float dw, const RefK &r, float &g, float &beta, float &bg) {
   g = fmaf(dw, r.minv, r.g);
   const float gam = g + 1.0f;
   bg = sqrt_fast(g * (g + 2.0f));
-  // both quotients by the two-ulp reciprocal-multiply: the denominators are
-  // products of gamma, beta and beta gamma of live particles, far from zero
-  // and from overflow
-  beta = __fdividef(bg, gam);
+  // the denominators are products of gamma, beta and beta gamma of live
+  // particles, far from zero and from overflow
+  const float rg = rcp_fast(gam);
+  beta = bg * rg;
   const float dg = dw * r.minv;
-  return -__fdividef(dg * (gam + r.gam), gam * r.gam * r.gam * (beta + r.beta) * bg * r.beta);
+  return -div_fast(dg * (gam + r.gam), gam * r.gam * r.gam * fmaf(bg, rg, r.beta) * bg * r.beta);
 }
-__device__ inline float dinvb(float dw, const RefK &r, float &g, float &beta) {
-  float bg;
+__device__ inline float dinvb(float dw, const RefK &r) {
+  float g, beta, bg;
   return dinvb(dw, r, g, beta, bg);
 }
 

@@ -6,6 +6,7 @@
 #include <stdint.h>
 
 #include <array>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -165,15 +166,29 @@ int sur_conv_state(const SurNet &n, int *tc_layers, unsigned int *err);
 // changed).  Both sweeps return at once when they are not needed.
 void sc32_stats_after_push(const DevBeam &b, ScState *sc, const ScTables &t, const ScKickArgs &a,
                            PassScratch s, cudaStream_t st);
-// An element map fused with the space-charge sweep next to it:
+// What an element map runs with:
+//  PUSH_PLAIN       nothing: maps with nothing between them become one sweep;
 //  PUSH_SCSTATS     the map, then every statistic of the kick after it from
 //                   the new state, the decision and the kick's constants,
 //                   when the sweep can certify them (else sc_redo = 2 and
 //                   sc32_stats_after_push completes them);
-//  PUSH_AFTER_KICK  the SCHEFF kick, then the map, in one sweep.
-enum { PUSH_SCSTATS = 1, PUSH_AFTER_KICK = 2 };
+//  PUSH_AFTER_KICK  the SCHEFF kick, then the map, in one sweep, joined by the
+//                   PUSH_SCSTATS map behind it when nothing comes between.
+enum { PUSH_PLAIN = 0, PUSH_SCSTATS = 1, PUSH_AFTER_KICK = 2 };
+// Maps wait in a queue of the range being run until the next one shows what
+// they can run with.  Whatever else reads or writes the particles on the
+// device, or ends the range, flushes the queue first.  defer = false: every
+// map is launched by itself (the phase timers time each).
+struct PushQueue;
+struct PushQueueDelete {
+  void operator()(PushQueue *q) const;
+};
+using PushQueueHandle = std::unique_ptr<PushQueue, PushQueueDelete>;
+PushQueueHandle push32_queue(bool defer);
+void push32_flush(PushQueue *q);  // q may be null
 struct PushFuse {
   int mode;
+  PushQueue *q;
   PassScratch scr;      // PUSH_SCSTATS: reduction scratch
   ScState *sc;          // solver state and tables
   ScTables t;
@@ -185,18 +200,18 @@ struct PushFuse {
 
 // Launchers that move the synchronous particle update b.phi_ref / b.w_ref.
 void push32_partial_drift(DevBeam &b, double wl, double hf, double aper, uint32_t eid, cudaStream_t st,
-                          const PushFuse *pf = nullptr);
+                          const PushFuse &pf);
 void push32_half_quad(DevBeam &b, double wl, double len, double aper, double grad, uint32_t eid, cudaStream_t st,
-                      const PushFuse *pf = nullptr);
-void push32_steerer(DevBeam &b, double blh, double blv, cudaStream_t st);
-void push32_gap_first(DevBeam &b, const GapArgs &g, cudaStream_t st, const PushFuse *pf = nullptr);
-void push32_gap_second(DevBeam &b, const GapArgs &g, cudaStream_t st, const PushFuse *pf = nullptr);
+                      const PushFuse &pf);
+void push32_steerer(DevBeam &b, double blh, double blv, cudaStream_t st, const PushFuse &pf);
+void push32_gap_first(DevBeam &b, const GapArgs &g, cudaStream_t st, const PushFuse &pf);
+void push32_gap_second(DevBeam &b, const GapArgs &g, cudaStream_t st, const PushFuse &pf);
 void push32_buncher(DevBeam &b, double wl, double w_ref_design, double freq, double voltage, double phase,
-                    double aper, double freq_ratio, uint32_t eid, cudaStream_t st);
-void push32_rotation(DevBeam &b, double angle, cudaStream_t st);
+                    double aper, double freq_ratio, uint32_t eid, cudaStream_t st, const PushFuse &pf);
+void push32_rotation(DevBeam &b, double angle, cudaStream_t st, const PushFuse &pf);
 void push32_aperture(DevBeam &b, int rect, const double *p, uint32_t eid, cudaStream_t st);
 void push32_dipole(DevBeam &b, const double *p, double wl, int second, cudaStream_t st,
-                   const PushFuse *pf = nullptr);
+                   const PushFuse &pf);
 
 void beam32_update_avg(const DevBeam &b, int coord, int good, PassScratch s, cudaStream_t st);
 void beam32_update_sig(const DevBeam &b, int coord, int good, PassScratch s, cudaStream_t st);

@@ -5,19 +5,23 @@
 // apply (simulation_kernel.cu), so absolute phases (hundreds of radians
 // after a DTL) and energies never pass through FP32.  Each launcher forms
 // its element's map (push32_maps.cuh) from the synchronous particle before
-// the element, moves the synchronous particle, and launches the map in one
-// of three forms: alone; followed by the statistics of the space-charge
-// kick that follows, taken from the new state in the same sweep; or preceded
-// by the space-charge kick (sc32_kick.cuh), so that a kick and the element
-// half after it are one sweep over the particles.
+// the element, moves the synchronous particle, and queues the map (PushQueue)
+// or launches it: maps with nothing between them run as one sweep over the
+// particles; a half behind a space-charge kick (sc32_kick.cuh) runs in the
+// kick's sweep, and so does the half of the next element with the statistics
+// of the kick after it, so that one sweep takes the particles from kick to
+// kick.
 //
 // Lost particles keep their absolute phase and energy (the reference's
 // kernels skip them): every sweep moves their offsets against the
 // synchronous particle's step through the element.
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <mutex>
+#include <type_traits>
 #include <unordered_map>
+#include <vector>
 
 #include "internal.h"
 #include "push32_maps.cuh"
@@ -61,8 +65,9 @@ __device__ inline uint32_t step(Part &p, const Map &m, const Shift &s) {
 // on the first, so each SM keeps enough loads in flight to cover latency.
 constexpr int kSweepBatch = 2;
 
-// cap: at most this many blocks per SM (0: as many as the SM holds)
-int sweep_grid(const void *kernel, uint32_t n, uint32_t cap) {
+// cap: at most this many blocks per SM (0: as many as the SM holds); batch:
+// particles a thread takes at a time
+int sweep_grid(const void *kernel, uint32_t n, uint32_t cap, int batch = kSweepBatch) {
   static std::mutex m;
   static std::unordered_map<const void *, int> resident;
   static int sms = 0;
@@ -75,7 +80,7 @@ int sweep_grid(const void *kernel, uint32_t n, uint32_t cap) {
     r = rr;
   }
   if (cap && (uint32_t)r > cap) r = (int)cap;
-  const uint64_t need = ((uint64_t)n + (uint64_t)kSweepBatch * kBlock - 1) / ((uint64_t)kSweepBatch * kBlock);
+  const uint64_t need = ((uint64_t)n + (uint64_t)batch * kBlock - 1) / ((uint64_t)batch * kBlock);
   return (int)std::max<uint64_t>(1, std::min<uint64_t>(need, (uint64_t)r * sms));
 }
 
@@ -98,9 +103,160 @@ __device__ __forceinline__ void push_body(const DevBeam &b, const Map &m, const 
   }
 }
 
-template <class Map>
-__global__ void __launch_bounds__(kBlock) k32_push(DevBeam b, Map m, Shift sh) {
-  push_body(b, m, sh, blockIdx.x, gridDim.x);
+// ---- runs of maps -------------------------------------------------------------
+enum MapKind : uint32_t { MAP_DRIFT, MAP_QUAD, MAP_GAP1, MAP_GAP2, MAP_STEER, MAP_BUNCH, MAP_ROT, MAP_DIP };
+template <class Map> constexpr MapKind map_kind();
+template <> constexpr MapKind map_kind<DriftMap>() { return MAP_DRIFT; }
+template <> constexpr MapKind map_kind<QuadMap>() { return MAP_QUAD; }
+template <> constexpr MapKind map_kind<Gap1Map>() { return MAP_GAP1; }
+template <> constexpr MapKind map_kind<Gap2Map>() { return MAP_GAP2; }
+template <> constexpr MapKind map_kind<SteerMap>() { return MAP_STEER; }
+template <> constexpr MapKind map_kind<BunchMap>() { return MAP_BUNCH; }
+template <> constexpr MapKind map_kind<RotMap>() { return MAP_ROT; }
+template <> constexpr MapKind map_kind<DipMap>() { return MAP_DIP; }
+
+// a map of a run; drift, quad and gap1 begin with the synchronous particle r
+struct RunRec {
+  MapKind kind;
+  uint16_t same;   // the energies and the synchronous particle are the previous map's
+  uint16_t loses;  // it may lose a particle
+  Shift sh;
+  union {
+    DriftMap drift;
+    QuadMap quad;
+    Gap1Map gap1;
+    SteerMap steer;
+    BunchMap bunch;
+    RotMap rot;
+    DipMap dip;
+  };
+};
+struct GapRunRec : RunRec {
+  Gap2Map gap2;
+};
+// what a map may change of a live particle
+uint32_t map_fields(MapKind k) {
+  switch (k) {
+    case MAP_DRIFT:
+    case MAP_GAP1: return WR_X | WR_Y | WR_PH;
+    case MAP_STEER: return WR_XP | WR_YP;
+    case MAP_BUNCH: return WR_XP | WR_YP | WR_W;
+    case MAP_ROT: return WR_X | WR_Y | WR_XP | WR_YP;
+    case MAP_GAP2: return WR_X | WR_Y | WR_XP | WR_YP | WR_PH | WR_W;
+    default: return WR_X | WR_Y | WR_XP | WR_YP | WR_PH;
+  }
+}
+// a run's maps travel as the kernel's own parameters (the constant bank): at
+// most 32,764 bytes
+template <class R, int B>
+struct RunArgs {
+  DevBeam b;
+  uint32_t n;
+  uint32_t fields;  // what the maps change of a live particle
+  R m[B];
+};
+constexpr int kRunMax = 256, kGapRunMax = 64;
+
+// Maps with nothing between them (no kick, no statistics, no display): each
+// particle is read once, goes through all of them in registers and is written
+// once.  81 launches of one map each moved the whole state 81 times (6,000,001
+// particles through 41 elements: 3.6 ms at 6.6 TB/s); here the time is the
+// maps' instructions.  Four particles a thread share a map's constants, whose
+// place depends on the loop, and hide the latency of its roots and quotients;
+// 1/beta - 1/beta_sync is kept while no map changes the energies; and maps
+// that cannot lose a particle skip every test while the thread's particles
+// are alive.
+constexpr int kRunBatch = 4;
+template <class R, int B>
+__global__ void __launch_bounds__(kBlock) k32_run(const __grid_constant__ RunArgs<R, B> a) {
+  const DevBeam &b = a.b;
+  const uint32_t stride = gridDim.x * blockDim.x;
+  for (uint32_t base = blockIdx.x * blockDim.x + threadIdx.x; base < b.n; base += kRunBatch * stride) {
+    Part p[kRunBatch];
+    float D[kRunBatch];
+    bool lost = false;  // any of the thread's particles
+    uint32_t was = 0;   // the ones lost before the run
+#pragma unroll
+    for (int u = 0; u < kRunBatch; ++u) {
+      D[u] = 0.0f;
+      if (base + u * stride < b.n) p[u] = load_part(b, base + u * stride);
+      else p[u] = {0u, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+      if (p[u].lo != 0u) was |= 1u << u;
+    }
+    lost = was != 0u;
+    for (uint32_t j = 0; j < a.n; ++j) {
+      const R &m = a.m[j];
+      if (!m.same && m.kind <= MAP_GAP1) {
+#pragma unroll
+        for (int u = 0; u < kRunBatch; ++u) D[u] = dinvb(p[u].w, m.drift.r);
+      }
+      if (!m.loses && !lost) {
+        auto each = [&](auto &&f) {
+#pragma unroll
+          for (int u = 0; u < kRunBatch; ++u) f(p[u], D[u]);
+        };
+        switch (m.kind) {
+          case MAP_DRIFT: each([&](Part &q, float d) { m.drift.open(q, d); }); break;
+          case MAP_QUAD:
+            if (m.quad.qg > 0.0f) each([&](Part &q, float d) { m.quad.template open<1>(q, d); });
+            else if (m.quad.qg < 0.0f) each([&](Part &q, float d) { m.quad.template open<-1>(q, d); });
+            else each([&](Part &q, float d) { m.quad.template open<0>(q, d); });
+            break;
+          case MAP_GAP1: each([&](Part &q, float d) { m.gap1.apply(q, [&] { return d; }); }); break;
+          case MAP_STEER: each([&](Part &q, float) { m.steer.apply(q); }); break;
+          case MAP_ROT: each([&](Part &q, float) { m.rot.apply(q); }); break;
+          default: each([&](Part &q, float) { m.dip.apply(q); }); break;
+        }
+        continue;
+      }
+      auto tested = [&](Part &q, auto &&f) {
+        if (q.lo == 0u) f(q);
+        if (q.lo != 0u) {
+          keep_lost(q, 0u, m.sh);
+          lost = true;
+        }
+      };
+      if (m.kind == MAP_BUNCH || m.kind == MAP_GAP2) {
+        // one particle after the other, rolled: four of these side by side
+        // would cost every map their registers
+#pragma unroll 1
+        for (int u = 0; u < kRunBatch; ++u) {
+          Part q = p[0];
+#pragma unroll
+          for (int v = 1; v < kRunBatch; ++v)
+            if (u == v) q = p[v];
+          tested(q, [&](Part &t) {
+            if constexpr (std::is_same_v<R, GapRunRec>) {
+              if (m.kind == MAP_GAP2) m.gap2.apply(t);
+              else m.bunch.apply(t);
+            } else {
+              m.bunch.apply(t);
+            }
+          });
+#pragma unroll
+          for (int v = 0; v < kRunBatch; ++v)
+            if (u == v) p[v] = q;
+        }
+        continue;
+      }
+      auto each = [&](auto &&f) {
+#pragma unroll
+        for (int u = 0; u < kRunBatch; ++u) tested(p[u], [&](Part &t) { f(t, [&] { return D[u]; }); });
+      };
+      switch (m.kind) {
+        case MAP_DRIFT: each([&](Part &q, auto &&d) { m.drift.apply(q, d); }); break;
+        case MAP_QUAD: each([&](Part &q, auto &&d) { m.quad.apply(q, d); }); break;
+        case MAP_GAP1: each([&](Part &q, auto &&d) { m.gap1.apply(q, d); }); break;
+        case MAP_STEER: each([&](Part &q, auto &&) { m.steer.apply(q); }); break;
+        case MAP_ROT: each([&](Part &q, auto &&) { m.rot.apply(q); }); break;
+        default: each([&](Part &q, auto &&) { m.dip.apply(q); }); break;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kRunBatch; ++u)
+      if (base + u * stride < b.n)
+        store_part(b, base + u * stride, p[u], (was >> u) & 1u ? (uint32_t)(WR_PH | WR_W) : a.fields | (p[u].lo != 0u ? (uint32_t)(WR_LOSS | WR_PH | WR_W) : 0u));
+  }
 }
 
 // The map, then every statistic the SCHEFF kick after it takes from the new
@@ -120,41 +276,37 @@ __global__ void __launch_bounds__(kBlock) k32_push(DevBeam b, Map m, Shift sh) {
 // one, sc32_stats_after_push); so it does when s lies more than 4
 // sigma_phi from <phi>_good, where sigma_phi^2 as a difference of FP32
 // moments about s would lose precision.
-template <class Map>
-struct OpPushScStats {
+struct ScStatsBase {
   // 0 good count, 1 sum d (raw, for <phi>_good), 2-3 sum f, f^2 (wrapped, for
   // sigma_phi), 4-8 x, x^2, y, y^2, W of the good set; 9 sum f, 10 count of the
   // live set; 11 lloss count; 12 max |f| over the live set; 13 max phi over
   // lloss != 1.  d = phi - s, f = wrap(d).
   static constexpr int K = 14;
   static constexpr int kMaxFrom = 12;
-  static constexpr int kBatch = 4;
+  // every form of the sweep has the same blocks, so that a kick's statistics
+  // are summed in the same order whatever the sweep runs with
+  static constexpr int kBatch = 1;
+  static constexpr int kMinBlocks = 4;
+  static constexpr int kGridPerSm = 4;
   static constexpr bool kFast = true;
-  static constexpr bool kThreadSetup = true;
   using Comb = SumComb;
   using Stage = Sc32Stage;
-  struct Ctx { float s; };
   struct P { Part p; uint32_t ll; };
   DevBeam b;  // carries the synchronous particle after the element
-  Map m;
-  Shift sh;
   int s_last;  // s from the last kick's <phi>_good offset (else 0)
   ScState *sc;
   ScTables tb;
   double freq, frac;
   Sc32Host h;
   __device__ bool enabled() const { return true; }
-  __device__ Ctx setup() const {
+  __device__ float origin() const {
     const float e = s_last ? tb.c32->pag : 0.0f;
-    return {fabsf(e) < 3.14159265f ? e : 0.0f};
+    return fabsf(e) < 3.14159265f ? e : 0.0f;
   }
   __device__ P load(uint32_t i) const { return {load_part(b, i), b.lloss[i]}; }
-  __device__ void use(uint32_t i, const P &q, float (&a)[K], const Ctx &c) const {
-    Part p = q.p;
-    const uint32_t w = step(p, m, sh);
-    if (w) store_part(b, i, p, w);
-    const bool alive = p.lo == 0u, g = alive && q.ll == 0u;
-    const float d = p.ph - c.s, f = rel_phase_f(d);
+  __device__ void add(const Part &p, uint32_t ll, float s, float (&a)[K]) const {
+    const bool alive = p.lo == 0u, g = alive && ll == 0u;
+    const float d = p.ph - s, f = rel_phase_f(d);
     a[0] += g ? 1.0f : 0.0f;
     a[1] += g ? d : 0.0f;
     a[2] += g ? f : 0.0f;
@@ -166,13 +318,13 @@ struct OpPushScStats {
     a[8] += g ? p.w : 0.0f;
     a[9] += alive ? f : 0.0f;
     a[10] += alive ? 1.0f : 0.0f;
-    a[11] += q.ll != 0u ? 1.0f : 0.0f;
+    a[11] += ll != 0u ? 1.0f : 0.0f;
     if (alive) a[12] = fmaxf(a[12], fabsf(f));
-    if (q.ll != 1u) a[13] = fmaxf(a[13], p.ph);
+    if (ll != 1u) a[13] = fmaxf(a[13], p.ph);
   }
   __device__ void stage_load(Stage &g, int tid, int nth) const {
     sc32_stage_load(g, b, sc, tid, nth);
-    if (tid == nth - 1) g.c.pag = setup().s;  // until the kick's constants take its place
+    if (tid == nth - 1) g.c.pag = origin();  // until the kick's constants take its place
   }
   __device__ void finalize(const double *t, int tid, int nth, Stage &stage) const {
     __shared__ int ok;
@@ -207,6 +359,65 @@ struct OpPushScStats {
     if (ok) zero_mesh_tables(&stage.sc, tb, tid, nth);
     __syncthreads();  // zero_mesh_tables resets the staged on-mesh count
     sc32_stage_store(stage, b, sc, tb.c32, ok, tid, nth);
+  }
+};
+
+template <class Map>
+struct OpPushScStats : ScStatsBase {
+  static constexpr bool kThreadSetup = true;
+  struct Ctx { float s; };
+  Map m;
+  Shift sh;
+  __device__ Ctx setup() const { return {origin()}; }
+  __device__ void use(uint32_t i, const P &q, float (&a)[K], const Ctx &c) const {
+    Part p = q.p;
+    const uint32_t w = step(p, m, sh);
+    if (w) store_part(b, i, p, w);
+    add(p, q.ll, c.s, a);
+  }
+};
+
+// the half of an element before its kick, by kind
+struct PreRec {
+  MapKind kind;
+  Shift sh;
+  union {
+    DriftMap drift;
+    QuadMap quad;
+    Gap1Map gap1;
+  };
+};
+
+// From kick to kick in one sweep: the SCHEFF kick on the particles it kicks,
+// the half behind it (A), the half of the next element (m) and the statistics
+// of the kick there.  The sweep is bound by its instructions on beams that L2
+// holds and by HBM on larger ones, so what it saves is a read and a write of
+// the state and a launch for each kick.  The kick reads the field table and
+// the constants of its kick, which only the finaliser replaces, after every
+// block has finished its particles.
+template <class A>
+struct OpKickPushScStats : ScStatsBase {
+  static constexpr bool kSharedCtx = true;
+  struct Ctx { float s; KickEnv e; };
+  RefK rk;
+  uint64_t skip_mask;
+  A a1;
+  Shift sh1;
+  PreRec m;
+  __device__ Ctx setup() const { return {origin(), kick_env(sc, tb, rk)}; }
+  __device__ void use(uint32_t i, const P &q, float (&a)[K], const Ctx &c) const {
+    Part p = q.p;
+    uint32_t w = 0;
+    if (p.lo == 0u && q.ll == 0u && ((uint64_t)i & skip_mask) != 0)
+      w = kick_particle(p, rel_phase_f(p.ph - c.e.pag), c.e);
+    w |= step(p, a1, sh1);
+    switch (m.kind) {
+      case MAP_DRIFT: w |= step(p, m.drift, m.sh); break;
+      case MAP_QUAD: w |= step(p, m.quad, m.sh); break;
+      default: w |= step(p, m.gap1, m.sh); break;
+    }
+    if (w) store_part(b, i, p, w);
+    add(p, q.ll, c.s, a);
   }
 };
 
@@ -291,37 +502,193 @@ void kick_push_merge(const std::vector<const Rec *> &recs, SegFork &, cudaStream
   });
 }
 
+// a half behind a kick that waits for the next element's half
+struct KickRec {
+  MapKind kind;
+  Shift sh;
+  RefK rk;
+  PushFuse pf;
+  DevBeam b;
+  cudaStream_t st;
+  union {
+    DriftMap drift;
+    QuadMap quad;
+    Gap2Map gap2;
+  };
+  template <class Map>
+  Map &as() {
+    if constexpr (std::is_same_v<Map, DriftMap>) return drift;
+    else if constexpr (std::is_same_v<Map, QuadMap>) return quad;
+    else return gap2;
+  }
+};
+template <class Map>
+constexpr bool waits_after_kick() {
+  return std::is_same_v<Map, DriftMap> || std::is_same_v<Map, QuadMap> || std::is_same_v<Map, Gap2Map>;
+}
+template <class Map>
+constexpr bool joins_kick() {
+  return std::is_same_v<Map, DriftMap> || std::is_same_v<Map, QuadMap> || std::is_same_v<Map, Gap1Map>;
+}
+template <class Map>
+constexpr bool has_halves() {
+  return waits_after_kick<Map>() || joins_kick<Map>() || std::is_same_v<Map, DipMap>;
+}
+
+}  // namespace
+
+// Work on the particles that has not been launched: a kick with the half
+// behind it, or a run of maps, never both.
+struct PushQueue {
+  bool defer = true;
+  bool kick = false;
+  KickRec k{};
+  std::vector<GapRunRec> run;
+  bool gap2 = false;    // the run has a gap's second half
+  DevBeam run_b{};
+  cudaStream_t run_st = nullptr;
+  RefK last_r{};        // of the run's last map, while no map since changed the energies
+  bool last_ok = false;
+};
+
+namespace {
+
+template <class Map>
+void launch_kick_push(const DevBeam &b, const PushFuse &pf, const RefK &rk, const Map &m, const Shift &sh,
+                      cudaStream_t st) {
+  const int grid = sweep_grid((const void *)k32_kick_push<Map>, b.n, b.sweep_cap);
+  if (recorder()) {
+    record("kick_push", &kick_push_merge<Map>, (uint32_t)grid,
+           KickPushSeg<Map>{b, (const ScState *)pf.sc, pf.t, rk, pf.skip_mask, m, sh});
+    return;
+  }
+  launch_k(k32_kick_push<Map>, dim3(grid), dim3(kBlock), 0, st, b, (const ScState *)pf.sc, pf.t, rk, pf.skip_mask, m,
+           sh);
+  note_launch();
+}
+
+template <class R, int B>
+void launch_run_chunk(const PushQueue &q, size_t k0, size_t n) {
+  static_assert(sizeof(RunArgs<R, B>) <= 32764, "a run's parameters exceed the kernel parameter limit");
+  std::vector<unsigned char> buf(sizeof(RunArgs<R, B>), 0);  // up to 32 KB: not on the stack
+  RunArgs<R, B> &a = *reinterpret_cast<RunArgs<R, B> *>(buf.data());
+  a.b = q.run_b;
+  a.n = (uint32_t)n;
+  for (size_t j = 0; j < n; ++j) {
+    a.m[j] = q.run[k0 + j];
+    a.fields |= map_fields(q.run[k0 + j].kind);
+  }
+  a.m[0].same = 0;  // the launch's first map takes the energies afresh
+  k32_run<R, B><<<sweep_grid((const void *)k32_run<R, B>, a.b.n, a.b.sweep_cap, kRunBatch), kBlock, 0, q.run_st>>>(a);
+  note_launch();
+}
+template <class R, int MAX>
+void launch_run(const PushQueue &q) {
+  for (size_t k0 = 0; k0 < q.run.size(); k0 += MAX) {
+    const size_t n = std::min(q.run.size() - k0, (size_t)MAX);
+    if (n <= 2) launch_run_chunk<R, 2>(q, k0, n);
+    else if (n <= 16) launch_run_chunk<R, 16>(q, k0, n);
+    else launch_run_chunk<R, MAX>(q, k0, n);
+  }
+}
+
+template <class Map>
+void queue_run(PushQueue &q, const DevBeam &b, const Map &m, const Shift &sh, cudaStream_t st) {
+  if (q.kick) push32_flush(&q);
+  GapRunRec r{};
+  constexpr MapKind kind = map_kind<Map>();
+  r.kind = kind;
+  r.sh = sh;
+  r.same = 0;
+  r.loses = kind == MAP_BUNCH || kind == MAP_GAP2;
+  if constexpr (kind == MAP_DRIFT || kind == MAP_QUAD) r.loses = m.aper2 != 0.0f;
+  if constexpr (kind == MAP_DRIFT) r.drift = m;
+  else if constexpr (kind == MAP_QUAD) r.quad = m;
+  else if constexpr (kind == MAP_GAP1) r.gap1 = m;
+  else if constexpr (kind == MAP_GAP2) { r.gap2 = m; q.gap2 = true; }
+  else if constexpr (kind == MAP_STEER) r.steer = m;
+  else if constexpr (kind == MAP_BUNCH) r.bunch = m;
+  else if constexpr (kind == MAP_ROT) r.rot = m;
+  else r.dip = m;
+  if constexpr (kind <= MAP_GAP1) {
+    r.same = q.last_ok && std::memcmp(&q.last_r, &m.r, sizeof(RefK)) == 0;
+    q.last_r = m.r;
+    q.last_ok = true;
+  } else if (kind == MAP_GAP2 || kind == MAP_BUNCH) {
+    q.last_ok = false;
+  }
+  q.run.push_back(r);
+  q.run_b = b;
+  q.run_st = st;
+  if (!q.defer) push32_flush(&q);
+}
+
+template <class A>
+bool launch_kick_to_kick(PushQueue &q, const ScStatsBase &base, const PreRec &m, const PushFuse &pf, cudaStream_t st) {
+  if (q.k.kind != map_kind<A>()) return false;
+  q.kick = false;
+  launch_pass_f(OpKickPushScStats<A>{base, q.k.rk, q.k.pf.skip_mask, q.k.as<A>(), q.k.sh, m}, base.b.n, pf.scr, st,
+                base.b.sweep_cap, "kick_push_scstats");
+  return true;
+}
+
 // b carries the synchronous particle after the element; rk is it before
 // (the kick of PUSH_AFTER_KICK happens there), phi0 / w0 its phase and energy
 template <class Map>
 void launch_map(const DevBeam &b, const Map &m, const RefK &rk, double phi0, double w0, cudaStream_t st,
-                const PushFuse *pf) {
+                const PushFuse &pf) {
+  PushQueue &q = *pf.q;
   const Shift sh{(float)(b.phi_ref - phi0), (float)(b.w_ref - w0)};
-  if (recorder()) {  // a lockstep range is being recorded
-    if (!pf) {
-      record("push", &push_merge<Map>, (uint32_t)sweep_grid((const void *)k32_push<Map>, b.n, b.sweep_cap),
-             PushSeg<Map>{b, m, sh});
-    } else if (pf->mode == PUSH_SCSTATS) {
-      launch_pass_f(OpPushScStats<Map>{b, m, sh, pf->s_last, pf->sc, pf->t, pf->freq, pf->frac, pf->h}, b.n, pf->scr,
-                    st, b.sweep_cap, "push_scstats");
-    } else {
-      record("kick_push", &kick_push_merge<Map>,
-             (uint32_t)sweep_grid((const void *)k32_kick_push<Map>, b.n, b.sweep_cap),
-             KickPushSeg<Map>{b, (const ScState *)pf->sc, pf->t, rk, pf->skip_mask, m, sh});
+  if (pf.mode == PUSH_PLAIN) {
+    if (!recorder()) {
+      queue_run(q, b, m, sh, st);
+      return;
     }
+    push32_flush(&q);
+    record("push", &push_merge<Map>, (uint32_t)sweep_grid((const void *)k32_push_seg<Map, 4>, b.n, b.sweep_cap),
+           PushSeg<Map>{b, m, sh});
     return;
   }
-  if (!pf) {
-    launch_k(k32_push<Map>, dim3(sweep_grid((const void *)k32_push<Map>, b.n, b.sweep_cap)), dim3(kBlock), 0, st, b,
-             m, sh);
-  } else if (pf->mode == PUSH_SCSTATS) {
-    launch_pass_f(OpPushScStats<Map>{b, m, sh, pf->s_last, pf->sc, pf->t, pf->freq, pf->frac, pf->h}, b.n, pf->scr,
-                  st, b.sweep_cap);
-  } else {
-    launch_k(k32_kick_push<Map>, dim3(sweep_grid((const void *)k32_kick_push<Map>, b.n, b.sweep_cap)), dim3(kBlock),
-             0, st, b, (const ScState *)pf->sc, pf->t, rk, pf->skip_mask, m, sh);
+  if constexpr (has_halves<Map>()) {
+    if (pf.mode == PUSH_SCSTATS) {
+      const ScStatsBase base{b, pf.s_last, pf.sc, pf.t, pf.freq, pf.frac, pf.h};
+      bool done = false;
+      if constexpr (joins_kick<Map>()) {
+        if (q.kick && q.k.b.n == b.n && q.k.pf.sc == pf.sc) {
+          PreRec r{};
+          r.kind = map_kind<Map>();
+          r.sh = sh;
+          if constexpr (map_kind<Map>() == MAP_DRIFT) r.drift = m;
+          else if constexpr (map_kind<Map>() == MAP_QUAD) r.quad = m;
+          else r.gap1 = m;
+          done = launch_kick_to_kick<DriftMap>(q, base, r, pf, st) || launch_kick_to_kick<QuadMap>(q, base, r, pf, st) ||
+                 launch_kick_to_kick<Gap2Map>(q, base, r, pf, st);
+        }
+      }
+      if (!done) {
+        push32_flush(&q);
+        if constexpr (joins_kick<Map>() || std::is_same_v<Map, DipMap>)
+          launch_pass_f(OpPushScStats<Map>{base, m, sh}, b.n, pf.scr, st, b.sweep_cap, "push_scstats");
+      }
+      if (!recorder()) note_launch();
+      return;
+    }
+    push32_flush(&q);
+    if constexpr (waits_after_kick<Map>()) {
+      if (q.defer) {
+        q.kick = true;
+        q.k.kind = map_kind<Map>();
+        q.k.sh = sh;
+        q.k.rk = rk;
+        q.k.pf = pf;
+        q.k.b = b;
+        q.k.st = st;
+        q.k.as<Map>() = m;
+        return;
+      }
+    }
+    if constexpr (waits_after_kick<Map>() || std::is_same_v<Map, DipMap>) launch_kick_push(b, pf, rk, m, sh, st);
   }
-  note_launch();
 }
 
 struct AptArgs {
@@ -374,11 +741,35 @@ void taylor(const double *a, int na, double b0, double *c) {
 
 }  // namespace
 
+PushQueueHandle push32_queue(bool defer) {
+  PushQueueHandle q(new PushQueue());
+  q->defer = defer;
+  return q;
+}
+void PushQueueDelete::operator()(PushQueue *q) const { delete q; }
+
+void push32_flush(PushQueue *q) {
+  if (!q) return;
+  if (q->kick) {
+    q->kick = false;
+    KickRec &k = q->k;
+    if (k.kind == MAP_DRIFT) launch_kick_push(k.b, k.pf, k.rk, k.drift, k.sh, k.st);
+    else if (k.kind == MAP_QUAD) launch_kick_push(k.b, k.pf, k.rk, k.quad, k.sh, k.st);
+    else launch_kick_push(k.b, k.pf, k.rk, k.gap2, k.sh, k.st);
+  }
+  if (!q->run.empty()) {
+    if (q->gap2) launch_run<GapRunRec, kGapRunMax>(*q);
+    else launch_run<RunRec, kRunMax>(*q);
+    q->run.clear();
+  }
+  q->gap2 = q->last_ok = false;
+}
+
 // ---------------------------------------------------------------------------
 // launchers: FP64 reference update on the host, FP32 map for the particles
 // ---------------------------------------------------------------------------
 void push32_partial_drift(DevBeam &b, double wl, double hf, double aper, uint32_t eid, cudaStream_t st,
-                          const PushFuse *pf) {
+                          const PushFuse &pf) {
   const double phi0 = b.phi_ref, w0 = b.w_ref;
   const RefK r = make_refk(b.w_ref, b.mass);
   const DriftMap m{r, (float)hf, (float)(aper * aper), (float)(TWOPI * hf / wl), eid};
@@ -387,7 +778,7 @@ void push32_partial_drift(DevBeam &b, double wl, double hf, double aper, uint32_
 }
 
 void push32_half_quad(DevBeam &b, double wl, double len, double aper, double grad, uint32_t eid, cudaStream_t st,
-                      const PushFuse *pf) {
+                      const PushFuse &pf) {
   const double phi0 = b.phi_ref, w0 = b.w_ref;
   const RefK r = make_refk(b.w_ref, b.mass);
   const double qg = grad * b.charge;
@@ -414,15 +805,15 @@ void push32_half_quad(DevBeam &b, double wl, double len, double aper, double gra
   launch_map(b, m, r, phi0, w0, st, pf);
 }
 
-void push32_steerer(DevBeam &b, double blh, double blv, cudaStream_t st) {
+void push32_steerer(DevBeam &b, double blh, double blv, cudaStream_t st, const PushFuse &pf) {
   const double phi0 = b.phi_ref, w0 = b.w_ref;
   const RefK r = make_refk(b.w_ref, b.mass);
   const float kh = blh > 1e-10 ? (float)(blh * b.charge * CLIGHT / b.mass) : 0.0f;
   const float kv = blv > 1e-10 ? (float)(blv * b.charge * CLIGHT / b.mass) : 0.0f;
-  launch_map(b, SteerMap{r, kh, kv}, r, phi0, w0, st, nullptr);
+  launch_map(b, SteerMap{r, kh, kv}, r, phi0, w0, st, pf);
 }
 
-void push32_gap_first(DevBeam &b, const GapArgs &g, cudaStream_t st, const PushFuse *pf) {
+void push32_gap_first(DevBeam &b, const GapArgs &g, cudaStream_t st, const PushFuse &pf) {
   const double phi0 = b.phi_ref, w0 = b.w_ref;
   const RefK r = make_refk(b.w_ref, b.mass);
   const double mass = b.mass;
@@ -459,7 +850,7 @@ void push32_gap_first(DevBeam &b, const GapArgs &g, cudaStream_t st, const PushF
   launch_map(b, Gap1Map{r, (float)dd1, (float)K}, r, phi0, w0, st, pf);
 }
 
-void push32_gap_second(DevBeam &b, const GapArgs &g, cudaStream_t st, const PushFuse *pf) {
+void push32_gap_second(DevBeam &b, const GapArgs &g, cudaStream_t st, const PushFuse &pf) {
   const double phi0 = b.phi_ref, w0 = b.w_ref;
   const double mass = b.mass;
   const RefK rkick = make_refk(b.w_ref, mass);
@@ -588,7 +979,7 @@ void push32_gap_second(DevBeam &b, const GapArgs &g, cudaStream_t st, const Push
 }
 
 void push32_buncher(DevBeam &b, double wl, double w_ref_design, double freq, double voltage, double phase,
-                    double aper, double freq_ratio, uint32_t eid, cudaStream_t st) {
+                    double aper, double freq_ratio, uint32_t eid, cudaStream_t st, const PushFuse &pf) {
   const double phi0 = b.phi_ref, w0 = b.w_ref;
   const double mass = b.mass;
   BunchMap B{};
@@ -612,12 +1003,12 @@ void push32_buncher(DevBeam &b, double wl, double w_ref_design, double freq, dou
   B.aper2 = (float)(aper * aper);
   B.eid = eid;
   b.w_ref += q * voltage * cos(h * b.phi_ref * freq_ratio + phase);
-  launch_map(b, B, B.r, phi0, w0, st, nullptr);
+  launch_map(b, B, B.r, phi0, w0, st, pf);
 }
 
-void push32_rotation(DevBeam &b, double angle, cudaStream_t st) {
+void push32_rotation(DevBeam &b, double angle, cudaStream_t st, const PushFuse &pf) {
   const double phi0 = b.phi_ref, w0 = b.w_ref;
-  launch_map(b, RotMap{(float)cos(angle), (float)sin(angle)}, RefK{}, phi0, w0, st, nullptr);
+  launch_map(b, RotMap{(float)cos(angle), (float)sin(angle)}, RefK{}, phi0, w0, st, pf);
 }
 
 void push32_aperture(DevBeam &b, int rect, const double *p, uint32_t eid, cudaStream_t st) {
@@ -631,7 +1022,7 @@ void push32_aperture(DevBeam &b, int rect, const double *p, uint32_t eid, cudaSt
   note_launch();
 }
 
-void push32_dipole(DevBeam &b, const double *p, double wl, int second, cudaStream_t st, const PushFuse *pf) {
+void push32_dipole(DevBeam &b, const double *p, double wl, int second, cudaStream_t st, const PushFuse &pf) {
   const double phi0 = b.phi_ref, w0 = b.w_ref;
   const double mass = b.mass;
   const RefK rkick = make_refk(b.w_ref, mass);

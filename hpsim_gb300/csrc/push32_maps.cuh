@@ -10,6 +10,10 @@
 // particle's increment: 1/beta_i - 1/beta_ref from dinvb, cos(p + e) - cos(p)
 // from half-angle products, transit-time factors re-expanded about the
 // reference's beta.
+//
+// A map gives a particle the same bits in every sweep it runs in (alone, in a
+// run, around a kick): where two products meet in a sum, fmaf says which of
+// them is rounded, so that the choice is not the compiler's in each kernel.
 #pragma once
 
 #include "common.cuh"
@@ -43,14 +47,22 @@ struct DriftMap {
   RefK r;
   float hf, aper2, c;  // c = 2 pi hf / lambda
   uint32_t eid;
-  __device__ uint32_t apply(Part &p) const {
+  __device__ uint32_t apply(Part &p) const { return apply(p, [&] { return dinvb(p.w, r); }); }
+  // D(): 1/beta of the particle minus the synchronous particle's
+  template <class F>
+  __device__ uint32_t apply(Part &p, const F &D) const {
     const float x = fmaf(p.xp, hf, p.x), y = fmaf(p.yp, hf, p.y);
     if (aper2 != 0.0f && x * x + y * y > aper2) { p.lo = eid; return WR_LOSS; }
     p.x = x;
     p.y = y;
-    float g, beta;
-    p.ph = fmaf(c, dinvb(p.w, r, g, beta), p.ph);
+    p.ph = fmaf(c, D(), p.ph);
     return WR_X | WR_Y | WR_PH;
+  }
+  // on a live particle, without an aperture
+  __device__ void open(Part &p, float D) const {
+    p.x = fmaf(p.xp, hf, p.x);
+    p.y = fmaf(p.yp, hf, p.y);
+    p.ph = fmaf(c, D, p.ph);
   }
 };
 
@@ -66,7 +78,9 @@ struct QuadMap {
   float sk0, isk0;                 // sqrt(|qG| c / m) and its inverse
   float kds_r, s_r, c_r, sh_r, ch_r;
   uint32_t eid;
-  __device__ uint32_t apply(Part &p) const {
+  __device__ uint32_t apply(Part &p) const { return apply(p, [&] { return dinvb(p.w, r); }); }
+  template <class F>
+  __device__ uint32_t apply(Part &p, const F &D) const {
     float x = p.x, y = p.y, xp = p.xp, yp = p.yp;
     uint32_t m;
     if (qg == 0.0f) {
@@ -77,42 +91,55 @@ struct QuadMap {
       p.y = y + yp * len * 0.5f;
       m = WR_X | WR_Y;
       if (aper2 != 0.0f && x * x + y * y > aper2) { p.lo = eid; return m | WR_LOSS; }
-      float g, beta;
-      p.ph = fmaf(c, dinvb(p.w, r, g, beta), p.ph);
+      p.ph = fmaf(c, D(), p.ph);
       return m | WR_PH;
     } else {
-      const float g = fmaf(p.w, r.minv, r.g);
-      const float bg = sqrt_fast(g * (g + 2.0f) * (1.0f + xp * xp + yp * yp));
-      const float rb = rsqrtf(bg);
-      const float k = sk0 * rb;              // sqrt(kcoef / bg)
-      const float inv_k = bg * rb * isk0;    // sqrt(bg / kcoef)
-      const float e = len * 0.25f * k - kds_r;
-      const float e2 = e * e;
-      const float t1 = e * (1.0f + e2 * (1.0f / 6.0f)), t0 = e2 * (0.5f + e2 * (1.0f / 24.0f));
-      // sin(a + e) = s_r (1 - e^2/2 + e^4/24) + c_r (e - e^3/6); sinh, cosh alike
-      const float s = fmaf(c_r, e - e * e2 * (1.0f / 6.0f), s_r * (1.0f - e2 * (0.5f - e2 * (1.0f / 24.0f))));
-      const float cc = fmaf(-s_r, e - e * e2 * (1.0f / 6.0f), c_r * (1.0f - e2 * (0.5f - e2 * (1.0f / 24.0f))));
-      const float sh = fmaf(ch_r, t1, sh_r * (1.0f + t0));
-      const float ch = fmaf(sh_r, t1, ch_r * (1.0f + t0));
-      const float sovk = s * inv_k, shovk = sh * inv_k, sk = s * k, shk = sh * k;
-      float xx, yy;
-#pragma unroll
-      for (int rep = 0; rep < 2; ++rep) {
-        if (qg > 0.0f) {
-          xx = cc * x + sovk * xp; xp = -sk * x + cc * xp; x = xx;
-          yy = ch * y + shovk * yp; yp = shk * y + ch * yp; y = yy;
-        } else {
-          xx = ch * x + shovk * xp; xp = shk * x + ch * xp; x = xx;
-          yy = cc * y + sovk * yp; yp = -sk * y + cc * yp; y = yy;
-        }
-      }
+      const float sl = fmaf(yp, yp, fmaf(xp, xp, 1.0f));
+      if (qg > 0.0f) focus(x, xp, y, yp, p.w, sl);
+      else focus(y, yp, x, xp, p.w, sl);
       m = WR_X | WR_Y | WR_XP | WR_YP;
     }
     p.x = x; p.y = y; p.xp = xp; p.yp = yp;
     if (aper2 != 0.0f && x * x + y * y > aper2) { p.lo = eid; return m | WR_LOSS; }
-    float g, beta;
-    p.ph = fmaf(c, dinvb(p.w, r, g, beta), p.ph);
+    p.ph = fmaf(c, D(), p.ph);
     return m | WR_PH;
+  }
+  // the half's two steps: u is the focusing plane, v the other; sl = 1 + x'^2 + y'^2
+  __device__ void focus(float &u, float &up, float &v, float &vp, float w, float sl) const {
+    const float g = fmaf(w, r.minv, r.g);
+    const float bg = sqrt_fast(g * (g + 2.0f) * sl);
+    const float rb = rsqrt_fast(bg);
+    const float k = sk0 * rb;              // sqrt(kcoef / bg)
+    const float inv_k = bg * rb * isk0;    // sqrt(bg / kcoef)
+    const float e = len * 0.25f * k - kds_r;
+    const float e2 = e * e;
+    const float t1 = e * (1.0f + e2 * (1.0f / 6.0f)), t0 = e2 * (0.5f + e2 * (1.0f / 24.0f));
+    // sin(a + e) = s_r (1 - e^2/2 + e^4/24) + c_r (e - e^3/6); sinh, cosh alike
+    const float s = fmaf(c_r, e - e * e2 * (1.0f / 6.0f), s_r * (1.0f - e2 * (0.5f - e2 * (1.0f / 24.0f))));
+    const float cc = fmaf(-s_r, e - e * e2 * (1.0f / 6.0f), c_r * (1.0f - e2 * (0.5f - e2 * (1.0f / 24.0f))));
+    const float sh = fmaf(ch_r, t1, sh_r * (1.0f + t0));
+    const float ch = fmaf(sh_r, t1, ch_r * (1.0f + t0));
+    const float sovk = s * inv_k, shovk = sh * inv_k, sk = s * k, shk = sh * k;
+#pragma unroll
+    for (int rep = 0; rep < 2; ++rep) {
+      const float un = fmaf(cc, u, sovk * up), vn = fmaf(ch, v, shovk * vp);
+      up = fmaf(cc, up, -sk * u);
+      vp = fmaf(shk, v, ch * vp);
+      u = un;
+      v = vn;
+    }
+  }
+  // on a live particle, without an aperture; SIGN of qg
+  template <int SIGN>
+  __device__ void open(Part &p, float D) const {
+    const float sl = fmaf(p.yp, p.yp, fmaf(p.xp, p.xp, 1.0f));
+    if constexpr (SIGN > 0) focus(p.x, p.xp, p.y, p.yp, p.w, sl);
+    else if constexpr (SIGN < 0) focus(p.y, p.yp, p.x, p.xp, p.w, sl);
+    else {
+      p.x = p.x + p.xp * len * 0.5f;
+      p.y = p.y + p.yp * len * 0.5f;
+    }
+    p.ph = fmaf(c, D, p.ph);
   }
 };
 
@@ -137,11 +164,12 @@ struct SteerMap {
 struct Gap1Map {
   RefK r;
   float dd1, K;
-  __device__ uint32_t apply(Part &p) const {
+  __device__ uint32_t apply(Part &p) const { return apply(p, [&] { return dinvb(p.w, r); }); }
+  template <class F>
+  __device__ uint32_t apply(Part &p, const F &D) const {
     p.x = fmaf(dd1, p.xp, p.x);
     p.y = fmaf(dd1, p.yp, p.y);
-    float g, beta;
-    p.ph = fmaf(K, dinvb(p.w, r, g, beta), p.ph);
+    p.ph = fmaf(K, D(), p.ph);
     return WR_X | WR_Y | WR_PH;
   }
 };
@@ -166,8 +194,8 @@ __device__ inline float fbessi0c(float x, float *m1) {
     *m1 = s;
     return 1.0f + s;
   }
-  const float cy = __fdividef(3.75f, ax);
-  const float ans = (expf(ax) * rsqrtf(ax)) * (0.39894228f + cy * (0.1328592e-1f + cy * (0.225319e-2f +
+  const float cy = div_fast(3.75f, ax);
+  const float ans = (expf(ax) * rsqrt_fast(ax)) * (0.39894228f + cy * (0.1328592e-1f + cy * (0.225319e-2f +
                     cy * (-0.157565e-2f + cy * (0.916281e-2f + cy * (-0.2057706e-1f + cy * (0.2635537e-1f +
                     cy * (-0.1647633e-1f + cy * 0.392377e-2f))))))));
   *m1 = ans - 1.0f;
@@ -182,11 +210,11 @@ __device__ inline float fbessi1c(float x) {
     ans = ax * (0.5f + cy * (0.87890594f + cy * (0.51498869f + cy * (0.15084934f + cy * (0.2658733e-1f +
           cy * (0.301532e-2f + cy * 0.32411e-3f))))));
   } else {
-    const float cy = __fdividef(3.75f, ax);
+    const float cy = div_fast(3.75f, ax);
     ans = 0.2282967e-1f + cy * (-0.2895312e-1f + cy * (0.1787654e-1f - cy * 0.420059e-2f));
     ans = 0.39894228f + cy * (-0.3988024e-1f + cy * (-0.362018e-2f + cy * (0.163801e-2f + cy *
           (-0.1031555e-1f + cy * ans))));
-    ans = ans * (expf(ax) * rsqrtf(ax));
+    ans = ans * (expf(ax) * rsqrt_fast(ax));
   }
   return x < 0.0f ? -ans : ans;
 }
@@ -237,7 +265,7 @@ struct Gap2Map {
     }
     float tw, dtw;
     if (G.ccl) {
-      tw = t - F_TWOPI * tp * (__fdividef(G.beta_in, beta) - 1.0f) * G.betag_ccl * G.inv_beta_in;
+      tw = t - F_TWOPI * tp * (div_fast(G.beta_in, beta) - 1.0f) * G.betag_ccl * G.inv_beta_in;
       dtw = tw - G.tw_r;
     } else {
       tw = t;
@@ -264,23 +292,23 @@ struct Gap2Map {
     float b0m1;
     const float b0c = fbessi0c(fkrris, &b0m1);
     const float b1c = fbessi1c(fkrris);
-    const float b1p = fkrris != 0.0f ? b0c - __fdividef(b1c, fkrris) : 0.5f;
-    const float bes1covr = ris != 0.0f ? __fdividef(b1c, ris) : G.fkr * 0.5f;
+    const float b1p = fkrris != 0.0f ? b0c - div_fast(b1c, fkrris) : 0.5f;
+    const float bes1covr = ris != 0.0f ? div_fast(b1c, ris) : G.fkr * 0.5f;
     const float rest = ((tw - F_TWOPI * tp) * G.inv_gmg * bes1covr + tw * G.inv_gmg * G.fkr * b1p -
                         tw * G.gmg * bes1covr) * rrp * sinp;
     const float ddelte = G.q * G.efl * (tw * b0c * dcos + (dtw * b0c + G.tw_r * b0m1) * G.cosP + rest);
     const float dwh = dw + ddelte;
     float gh, betah, bg;
     const float Dh = dinvb(dwh, G.rh, gh, betah, bg);
-    const float bgr = __fdividef(bg1, bg);
+    const float bgr = div_fast(bg1, bg);
     const float onema = 1.0f - (con5nex * bes1covr + con5nex1 * b1p + con5nex2 * bes1covr) * cosp;
     const float dovbl = G.con2nex * bes1covr * tw * sinp;
-    const float bgrovonema = __fdividef(bgr, onema);
+    const float bgrovonema = div_fast(bgr, onema);
     xp = -dovbl * x + bgrovonema * xp;
     x = x * onema + G.dd2 * xp;
     yp = -dovbl * y + bgrovonema * yp;
     y = y * onema + G.dd2 * yp;
-    const float rpris = rs_p > 0.0f ? __fdividef(rrp, ris) : 0.0f;
+    const float rpris = rs_p > 0.0f ? div_fast(rrp, ris) : 0.0f;
     const float prome = 2.0f * G.con1 * (-tp * b0c + ris * tw * b1c * G.inv_gmgcl) * (sinp - G.sinps) -
                         G.efl_m * tw * b1c * rpris * (cosp - G.cosps);
     const float dphih = dphi + G.K2 * Dh + (prome - G.prome_r);
@@ -303,20 +331,19 @@ struct BunchMap {
   uint32_t eid;
   __device__ uint32_t apply(Part &p) const {
     const float x = p.x, y = p.y, dw = p.w;
-    const float r2 = x * x + y * y;
+    const float r2 = fmaf(x, x, y * y);
     if (aper2 != 0.0f && r2 > aper2) { p.lo = eid; return WR_LOSS; }
     const float delta = hr * p.ph;
     float sd, cd;
     sincosf(delta, &sd, &cd);
-    const float cosph = cosB * cd - sinB * sd, sinph = sinB * cd + cosB * sd;
+    const float cosph = fmaf(cosB, cd, -(sinB * sd)), sinph = fmaf(sinB, cd, cosB * sd);
     const float sh = sinf(0.5f * delta);
-    const float dcos = -cosB * 2.0f * sh * sh - sinB * sd;
+    const float dcos = fmaf(-cosB * 2.0f * sh, sh, -(sinB * sd));
     const float arg = k2q * r2;
     const float poly = arg * (1.0f + arg * (0.25f + arg / 36.0f));
     const float dwi = qV * cosph * (1.0f + poly);
-    const float ddw = qV * (dcos + cosph * poly);
-    const float w = r.w + dw;
-    const float wb_par = w + 0.5f * dwi, wf = w + dwi;
+        const float w = r.w + dw;
+    const float wb_par = fmaf(0.5f, dwi, w), wf = __fadd_rn(w, dwi);
     if (wb_par <= 0.0f || wf <= 0.0f) { p.lo = eid; return WR_LOSS; }
     float gt = wb_par * r.minv;
     const float bav = sqrtf(gt * (gt + 2.0f)) / (gt + 1.0f);
@@ -325,9 +352,9 @@ struct BunchMap {
     gt = wf * r.minv;
     const float rbgf = rsqrtf(gt * (gt + 2.0f));
     const float del = -con1 * sinph * (1.0f - bav * beta_w) * (0.5f + arg * (0.25f + arg / 24.0f)) / bav;
-    p.xp = (p.xp * bg + del * x) * rbgf;
-    p.yp = (p.yp * bg + del * y) * rbgf;
-    p.w = dw + ddw;
+    p.xp = fmaf(p.xp, bg, del * x) * rbgf;
+    p.yp = fmaf(p.yp, bg, del * y) * rbgf;
+    p.w = fmaf(qV, fmaf(cosph, poly, dcos), dw);
     return WR_XP | WR_YP | WR_W;
   }
 };

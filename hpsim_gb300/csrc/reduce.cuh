@@ -36,6 +36,23 @@ struct MaxComb {  // MaxR2PhiReduceKernel starts from 0 (beam_kernel.cu:809-810)
   __device__ static float comb(float a, float b) { return a < b ? b : a; }
 };
 
+// a sum as a float and the float of its rounding errors (two-sum, Knuth)
+struct Pair2 {
+  float x, e;
+};
+__device__ __forceinline__ Pair2 shfl_xor_any(Pair2 v, int off) {
+  return {__shfl_xor_sync(0xffffffffu, v.x, off), __shfl_xor_sync(0xffffffffu, v.e, off)};
+}
+template <class T>
+__device__ __forceinline__ T shfl_xor_any(T v, int off) { return __shfl_xor_sync(0xffffffffu, v, off); }
+struct PairSum {
+  __device__ static Pair2 ident() { return {0.0f, 0.0f}; }
+  __device__ static Pair2 comb(Pair2 a, Pair2 b) {
+    const float s = a.x + b.x, bb = s - a.x;
+    return {s, ((a.x - (s - bb)) + (b.x - bb)) + (a.e + b.e)};
+  }
+};
+
 // Totals over a warp of K accumulators a lane, K <= 32, by folding: a step
 // halves the lanes' distance and the accumulators a lane still carries (it
 // sends one half to its partner and keeps the other), so K sums cost about
@@ -55,13 +72,13 @@ __device__ __forceinline__ bool warp_fold(const T (&a)[K], int lane, int &slot, 
 #pragma unroll
     for (int k = 0; k < cnt; ++k) {
       const T keep = hi ? v[k + cnt] : v[k], send = hi ? v[k] : v[k + cnt];
-      v[k] = C::comb(keep, __shfl_xor_sync(0xffffffffu, send, off));
+      v[k] = C::comb(keep, shfl_xor_any(send, off));
     }
     if (hi) base += cnt;
   }
   T x = v[0];
 #pragma unroll
-  for (int o = 16 / P; o > 0; o /= 2) x = C::comb(x, __shfl_xor_sync(0xffffffffu, x, o));
+  for (int o = 16 / P; o > 0; o /= 2) x = C::comb(x, shfl_xor_any(x, o));
   slot = base;
   total = x;
   return (lane & (32 / P - 1)) == 0 && base < K;
@@ -228,6 +245,28 @@ template <class Op>
 struct op_thread_setup<Op, std::void_t<decltype(Op::kThreadSetup)>>
     : std::integral_constant<bool, Op::kThreadSetup> {};
 
+// An Op with `static constexpr bool kSharedCtx = true` reads its set-up from
+// shared memory where it uses it: for set-ups of many values, which would
+// otherwise take a register each.
+template <class Op, class = void>
+struct op_shared_ctx : std::false_type {};
+template <class Op>
+struct op_shared_ctx<Op, std::void_t<decltype(Op::kSharedCtx)>> : std::integral_constant<bool, Op::kSharedCtx> {};
+
+// An Op may ask for a number of resident blocks per SM (`static constexpr int
+// kMinBlocks`), which bounds its registers.
+template <class Op, class = void>
+struct op_min_blocks : std::integral_constant<int, 1> {};
+template <class Op>
+struct op_min_blocks<Op, std::void_t<decltype(Op::kMinBlocks)>> : std::integral_constant<int, Op::kMinBlocks> {};
+
+// An Op may fix its blocks per SM (`static constexpr int kGridPerSm`, at most
+// what an SM holds), so that its sums have one order in every form.
+template <class Op, class = void>
+struct op_grid_per_sm : std::integral_constant<int, 0> {};
+template <class Op>
+struct op_grid_per_sm<Op, std::void_t<decltype(Op::kGridPerSm)>> : std::integral_constant<int, Op::kGridPerSm> {};
+
 // An Op with a nested `Stage` has one of them in the last block's shared
 // memory: stage_load(stage, tid, nthreads) runs before that block combines
 // the partials, and finalize takes the stage as a fourth argument.
@@ -251,15 +290,16 @@ __device__ __forceinline__ void pass_body_f(const Op &op, uint32_t n, PassScratc
   if (!op.enabled()) return;
   __shared__ double tot[K];
   __shared__ int is_last;
-  typename Op::Ctx ctx;
+  __shared__ typename Op::Ctx sctx;
+  typename Op::Ctx rctx;
   if constexpr (op_thread_setup<Op>::value) {
-    ctx = op.setup();
+    rctx = op.setup();
   } else {
-    __shared__ typename Op::Ctx sctx;
     if (threadIdx.x == 0) sctx = op.setup();
     __syncthreads();
-    ctx = sctx;
+    if constexpr (!op_shared_ctx<Op>::value) rctx = sctx;
   }
+  const typename Op::Ctx &ctx = op_shared_ctx<Op>::value ? sctx : rctx;
   constexpr int MF = op_max_from<Op>::value;
   static_assert(MF == K || op_fast<Op>::value, "max slots need the FP32 combine");
   static_assert(!op_stage<Op>::value || op_fast<Op>::value, "a stage needs the FP32 combine");
@@ -350,12 +390,18 @@ __device__ __forceinline__ void pass_body_f(const Op &op, uint32_t n, PassScratc
     }
   } else {
     __shared__ double sm[combine_rows<K>()][K];
+    if constexpr (std::is_same_v<C, SumComb>) {
+      // pairs (sum, rounding errors): an emittance is a difference of products
+      // of these sums, which a correlated beam amplifies a hundredfold
+      Pair2 v[K], t;
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-      float v = acc[k];
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) v = C::comb(v, __shfl_down_sync(0xffffffffu, v, off));
-      if (lane == 0) sm[warp][k] = (double)v;
+      for (int k = 0; k < K; ++k) v[k] = {acc[k], 0.0f};
+      int slot;
+      if (warp_fold<PairSum>(v, lane, slot, t)) sm[warp][slot] = (double)t.x + (double)t.e;
+    } else {
+      int slot;
+      float v;
+      if (warp_fold<C>(acc, lane, slot, v)) sm[warp][slot] = (double)v;
     }
     __syncthreads();
     if (threadIdx.x < K) {
@@ -379,7 +425,7 @@ __device__ __forceinline__ void pass_body_f(const Op &op, uint32_t n, PassScratc
 }
 
 template <class Op>
-__global__ void __launch_bounds__(kBlock) pass_kernel_f(Op op, uint32_t n, PassScratch scr) {
+__global__ void __launch_bounds__(kBlock, op_min_blocks<Op>::value) pass_kernel_f(Op op, uint32_t n, PassScratch scr) {
   pass_body_f(op, n, scr, blockIdx.x, gridDim.x);
 }
 
@@ -391,7 +437,7 @@ struct PassSeg {
   PassScratch scr;
 };
 template <class Op, int B>
-__global__ void __launch_bounds__(kBlock) pass_kernel_f_seg(const __grid_constant__ SegArgs<PassSeg<Op>, B> a) {
+__global__ void __launch_bounds__(kBlock, op_min_blocks<Op>::value) pass_kernel_f_seg(const __grid_constant__ SegArgs<PassSeg<Op>, B> a) {
   uint32_t bid, nblk;
   const PassSeg<Op> &p = a.p[seg_find(a, blockIdx.x, bid, nblk)];
   pass_body_f(p.op, p.n, p.scr, bid, nblk);
@@ -418,8 +464,14 @@ inline void launch_pass_f_grid(const Op &op, uint32_t n, PassScratch scr, cudaSt
 // fewer, fuller blocks keep that tail short; each thread walks more
 // particles in batches instead.  With the FP32 combine, every block the SMs
 // hold at once (up to the scratch's kMaxPassBlocks).
-inline int pass_blocks_f(uint32_t n, int per_sm = 2) {
-  uint32_t b = (n + kPassBatch * kBlock - 1) / (kPassBatch * kBlock);
+// A pass that takes a particle at a time (batch 1) spreads a small beam over
+// the SMs, a particle a thread up to one block on each; beyond that its blocks
+// hold four a thread as the others' do (more blocks make a lone beam no
+// faster and cost beams that share the SMs their reductions: a scan of 32
+// beams 24.6 -> 26.3 ms with a particle a thread throughout).
+inline int pass_blocks_f(uint32_t n, int per_sm = 2, int batch = kPassBatch) {
+  uint32_t b = (uint32_t)(((uint64_t)n + kPassBatch * kBlock - 1) / (kPassBatch * kBlock));
+  if (batch == 1) b = std::max(b, std::min<uint32_t>((uint32_t)(((uint64_t)n + kBlock - 1) / kBlock), 152u));
   if (b < 1) b = 1;
   const uint32_t cap = std::min<uint32_t>((uint32_t)per_sm * 152u, (uint32_t)kMaxPassBlocks);
   if (b > cap) b = cap;
@@ -438,9 +490,9 @@ inline int pass_resident() {
 template <class Op>
 inline void launch_pass_f(const Op &op, uint32_t n, PassScratch scr, cudaStream_t s, uint32_t cap = 0,
                           const char *site = "pass") {
-  int per_sm = op_fast<Op>::value ? pass_resident<Op>() : 2;
+  int per_sm = op_grid_per_sm<Op>::value ? op_grid_per_sm<Op>::value : op_fast<Op>::value ? pass_resident<Op>() : 2;
   if (cap && (uint32_t)per_sm > cap) per_sm = (int)cap;
-  launch_pass_f_grid(op, n, scr, s, (uint32_t)pass_blocks_f(n, per_sm), site);
+  launch_pass_f_grid(op, n, scr, s, (uint32_t)pass_blocks_f(n, per_sm, op_fast<Op>::value ? op_batch<Op>::value : kPassBatch), site);
 }
 
 // FP32 version of rel_phase for offsets that are already small

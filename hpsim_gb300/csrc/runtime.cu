@@ -1070,6 +1070,7 @@ struct Ctx {
   hps_beamline_t bl;
   hps_scheff_t sc;
   bool kicked = false;  // a SCHEFF kick of this simulation call has been issued
+  PushQueue *q = nullptr;  // FP32 beams: the range's queue of element maps
 };
 
 const double *P(hps_beamline_t bl, uint32_t i) { return bl->params[i].data(); }
@@ -1128,20 +1129,24 @@ ScKickArgs kick_args(Ctx &c, double length) {
 // valid from four particles on (blck_size/4 > 0, n > 2).
 struct Fuse32 {
   bool on;
-  PushFuse pre, post;
+  PushFuse plain, pre, post;
 };
 Fuse32 fuse32(Ctx &c) {
   Fuse32 z{};
   hps_beam_t b = c.b;
+  z.plain.mode = PUSH_PLAIN;
+  z.plain.q = c.q;
   const uint64_t stride = (uint64_t)b->grid_size * (b->blck_size / 4);
   z.on = f32(b) && c.s->sc_on && c.sc && b->n >= 4 && stride != 0 && (stride & (stride - 1)) == 0;
   if (!z.on) return z;
   z.pre.mode = PUSH_SCSTATS;
+  z.pre.q = c.q;
   z.pre.scr = b->scr;
   z.pre.sc = c.sc->d;
   z.pre.t = c.sc->t;
   z.pre.t.fld2 = nullptr;
   z.post.mode = PUSH_AFTER_KICK;
+  z.post.q = c.q;
   z.post.sc = c.sc->d;
   z.post.t = c.sc->t;
   z.post.t.fld2 = nullptr;
@@ -1149,16 +1154,16 @@ Fuse32 fuse32(Ctx &c) {
   return z;
 }
 
-// the PUSH_SCSTATS form for the half before a kick of the given length
-const PushFuse *pre_for(Ctx &c, const Fuse32 &z, double length, PushFuse *out) {
-  if (!z.on) return nullptr;
+// the form of the half before a kick of the given length
+const PushFuse &pre_for(Ctx &c, const Fuse32 &z, double length, PushFuse *out) {
+  if (!z.on) return z.plain;
   *out = z.pre;
   const ScKickArgs a = kick_args(c, length);
   out->h = sc32_host(c.b->d, a);
   out->freq = a.freq;
   out->frac = a.frac;
   out->s_last = c.kicked;  // results depend on the call's inputs only
-  return out;
+  return *out;
 }
 
 // fused: what the PUSH_SCSTATS half left of the statistics, and the mesh;
@@ -1167,6 +1172,7 @@ void sc_apply(Ctx &c, double length, bool fused = false) {
   if (!(c.s->sc_on && c.sc)) return;
   c.kicked = true;
   hps_beam_t b = c.b;
+  push32_flush(c.q);
   const ScKickArgs a = kick_args(c, length);
   if (f32(b)) {
     sc32_configure();
@@ -1191,6 +1197,7 @@ void sc_apply(Ctx &c, double length, bool fused = false) {
 void prep_gap(Ctx &c, const GapArgs &g) {
   hps_beam_t b = c.b;
   if (b->freq != g.frequency) {
+    push32_flush(c.q);
     c.s->wavelen = CLIGHT / g.frequency;
     double ratio = g.frequency / b->freq;
     b->current *= g.frequency / b->freq;
@@ -1202,6 +1209,7 @@ void prep_gap(Ctx &c, const GapArgs &g) {
 
 void monitor_at(Ctx &c, uint32_t i) {
   hps_beam_t b = c.b;
+  push32_flush(c.q);
   const ScState *sc = (c.s->sc_on && c.sc) ? c.sc->d : nullptr;
   double *dst = c.s->mon_dev + (size_t)i * HPS_NMON;
   if (f32(b)) PHASE(HPS_PROF_MONITOR, beam32_monitor(b->d, sc, dst, i, b->scr, b->stream));
@@ -1219,9 +1227,9 @@ hps_status visit(Ctx &c, uint32_t i) {
   cudaStream_t st = b->stream;
   uint32_t eid = s->cur_id;
   const Fuse32 z = fuse32(c);
-  const PushFuse *post = z.on ? &z.post : nullptr;
+  const PushFuse &post = z.on ? z.post : z.plain;
   PushFuse pre_buf;
-  auto pre = [&](double length) { return pre_for(c, z, length, &pre_buf); };
+  auto pre = [&](double length) -> const PushFuse & { return pre_for(c, z, length, &pre_buf); };
   // a half that runs behind the kick is timed as the kick
   auto post_cls = [&](int cls) { return z.on ? (int)HPS_PROF_SC_KICK : cls; };
   switch (bl->types[i]) {
@@ -1327,7 +1335,7 @@ hps_status visit(Ctx &c, uint32_t i) {
       break;
     }
     case HPS_ELEM_ROTATION:
-      PHASE(HPS_PROF_OTHER, f ? push32_rotation(d, p[HPS_P_ROT_ANGLE], st) : push_rotation(d, p[HPS_P_ROT_ANGLE], st));
+      PHASE(HPS_PROF_OTHER, f ? push32_rotation(d, p[HPS_P_ROT_ANGLE], st, z.plain) : push_rotation(d, p[HPS_P_ROT_ANGLE], st));
       break;
     case HPS_ELEM_SPCHCOMP:
       if (s->sc_on && c.sc) c.sc->fraction = p[HPS_P_SPC_FRACTION];
@@ -1335,6 +1343,7 @@ hps_status visit(Ctx &c, uint32_t i) {
     case HPS_ELEM_APERTURE_C:
     case HPS_ELEM_APERTURE_R:
       if (p[HPS_P_APT_IN] == 0.0) break;
+      push32_flush(c.q);
       PHASE(HPS_PROF_OTHER, beam_update_loss(d, b->scr, st);
             f ? beam32_update_avg_xy(d, b->scr, st) : beam_update_avg_xy(d, b->scr, st);
             f ? push32_aperture(d, bl->types[i] == HPS_ELEM_APERTURE_R, p, eid, st)
@@ -1345,7 +1354,7 @@ hps_status visit(Ctx &c, uint32_t i) {
     case HPS_ELEM_STEERER: {
       double blh = p[HPS_P_STR_BLH], blv = p[HPS_P_STR_BLV];
       if (blh > 1e-10 || blv > 1e-10)
-        PHASE(HPS_PROF_OTHER, f ? push32_steerer(d, blh, blv, st) : push_steerer(d, blh, blv, st));
+        PHASE(HPS_PROF_OTHER, f ? push32_steerer(d, blh, blv, st, z.plain) : push_steerer(d, blh, blv, st));
       break;
     }
     case HPS_ELEM_BUNCHER: {
@@ -1354,7 +1363,7 @@ hps_status visit(Ctx &c, uint32_t i) {
       s->wavelen = CLIGHT / bf;
       PHASE(HPS_PROF_OTHER,
             f ? push32_buncher(d, s->wavelen, s->design_w, bf, p[HPS_P_BUN_VOLTAGE], p[HPS_P_BUN_PHASE],
-                               p[HPS_P_APERTURE], bf / b->freq, eid, st)
+                               p[HPS_P_APERTURE], bf / b->freq, eid, st, z.plain)
               : push_buncher(d, s->wavelen, s->design_w, bf, p[HPS_P_BUN_VOLTAGE], p[HPS_P_BUN_PHASE],
                              p[HPS_P_APERTURE], bf / b->freq, eid, st));
       break;
@@ -1374,17 +1383,35 @@ hps_status visit(Ctx &c, uint32_t i) {
   return HPS_OK;
 }
 
-// SimulationEngine::Simulate, simulation_engine.cpp:447-469
-hps_status run_range(Ctx &c, int start_index, int end_index, bool monitor) {
+// SimulationEngine::Simulate, simulation_engine.cpp:447-469.  host_sync: the
+// solver's interval and mesh are read back after every element.
+hps_status run_range(Ctx &c, int start_index, int end_index, bool monitor, bool host_sync = false) {
   hps_sim_t s = c.s;
+  const PushQueueHandle queue = f32(c.b) ? push32_queue(!s->prof_on && !host_sync) : PushQueueHandle();
+  c.q = queue.get();
+  auto done = [&](hps_status st) {
+    push32_flush(c.q);
+    c.q = nullptr;
+    return st;
+  };
   for (int i = 0; i <= end_index; ++i) {
     if (i >= start_index || c.bl->types[i] == HPS_ELEM_SPCHCOMP) {
       s->cur_id = (uint32_t)i;
       hps_status st = visit(c, (uint32_t)i);
-      if (st) return st;
+      if (st) return done(st);
       if (monitor) monitor_at(c, (uint32_t)i);
+      if (host_sync) {
+        ScState h;
+        cudaError_t e = cudaMemcpyAsync(&h, c.sc->d, sizeof(h), cudaMemcpyDeviceToHost, c.b->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(c.b->stream);
+        if (e != cudaSuccess) return done(fail(HPS_ERR_CUDA, cudaGetErrorString(e)));
+        c.sc->interval = h.interval;
+        c.sc->nx = h.nx;
+        c.sc->nz = h.nz;
+      }
     }
   }
+  done(HPS_OK);
   return last_launch_status("simulate");
 }
 
@@ -1664,22 +1691,8 @@ hps_status hps_sim_simulate(hps_sim_t s, int32_t start, int32_t end) {
     if (e) return e;
     CK(cudaGraphLaunch(sim->graph.exec, st));
   } else {
-    for (int i = 0; i <= p.end_index; ++i) {
-      if (i >= p.start_index || c.bl->types[i] == HPS_ELEM_SPCHCOMP) {
-        sim->cur_id = (uint32_t)i;
-        e = visit(c, (uint32_t)i);
-        if (e) return e;
-        if (p.monitor) monitor_at(c, (uint32_t)i);
-        if (p.host_sync) {
-          ScState h;
-          CK(cudaMemcpyAsync(&h, c.sc->d, sizeof(h), cudaMemcpyDeviceToHost, st));
-          CK(cudaStreamSynchronize(st));
-          c.sc->interval = h.interval;
-          c.sc->nx = h.nx;
-          c.sc->nz = h.nz;
-        }
-      }
-    }
+    e = run_range(c, p.start_index, p.end_index, p.monitor, p.host_sync);
+    if (e) return e;
   }
   CK(cudaEventRecord(sim->ev1, st));
   e = last_launch_status("simulate");

@@ -55,33 +55,32 @@ __device__ inline float wrap_turns(float d) {
 // kick particle p (live, not longitudinally lost) whose relative phase is
 // phi; returns the fields changed.  Quotients whose denominators are
 // bounded away from zero and overflow use the two-ulp reciprocal-multiply
-// (__fdividef), the square roots of the common path the hardware
+// (div_fast), the square roots of the common path the hardware
 // approximation (sqrt_fast).
 __device__ inline uint32_t kick_particle(Part &p, float phi, const KickEnv &e) {
   const float dw = p.w;
   const float g = fmaf(dw, e.r.minv, e.r.g);
   const float gm = g + 1.0f;
   const float bgz = sqrt_fast(g * (g + 2.0f));
-  float bgx = bgz * p.xp, bgy = bgz * p.yp;
-  const float dgc = (dw + e.dwc) * e.r.minv;  // gm - gamma_c
-  const float s0 = __fdividef(dgc * (gm + e.gmg), e.gmg * (bgz + e.beta * gm));
+    const float dgc = (dw + e.dwc) * e.r.minv;  // gm - gamma_c
+  const float s0 = div_fast(dgc * (gm + e.gmg), e.gmg * fmaf(e.beta, gm, bgz));
   const float xxbar = p.x - e.xbar, yybar = p.y - e.ybar;
-  float rr = sqrt_fast(xxbar * xxbar * e.inv_epsq + yybar * yybar * e.epsq);
+  float rr = sqrt_fast(fmaf(xxbar * xxbar, e.inv_epsq, yybar * yybar * e.epsq));
   if (rr == 0.0f) rr = 1.0e-8f;
-  const float inv_rr = __fdividef(1.0f, rr);
+  const float inv_rr = rcp_fast(rr);
   const float xovr = xxbar * e.xfac * inv_rr, yovr = yybar * e.yfac * inv_rr;
-  float z = -e.c2 * wrap_turns(phi - e.phimc);
+  float z = __fmul_rn(-e.c2, wrap_turns(phi - e.phimc));
   float cbgr, cbgzs;
   if (rr > e.rmesh || fabsf(z) > e.hl) {
     z = -e.c2 * (phi - e.phimc);
-    float d = sqrtf(z * z + rr * rr);
+    float d = sqrtf(fmaf(z, z, rr * rr));
     float invd3 = 1.0f / (d * d * d);
     float rod3 = rr * invd3, zod3 = z * invd3;
     for (uint32_t nb = 1; nb <= e.adj; ++nb) {
       float xi = (float)nb;
       for (int lr = 0; lr < 2; ++lr) {
         const float sft = z + xi * e.pl;
-        d = sqrtf(sft * sft + rr * rr);
+        d = sqrtf(fmaf(sft, sft, rr * rr));
         invd3 = 1.0f / (d * d * d);
         rod3 += rr * invd3;
         zod3 += sft * invd3;
@@ -91,11 +90,11 @@ __device__ inline uint32_t kick_particle(Part &p, float phi, const KickEnv &e) {
     cbgr = e.cbgcoef * rod3;
     cbgzs = e.cbgcoef * zod3;
   } else {
-    const float ri = rr * e.inv_dr;
+    const float ri = __fmul_rn(rr, e.inv_dr);
     const uint32_t i = 1 + (int)ri;
     const float a = ri - (float)(i - 1);
     const float bb = 1.0f - a;
-    const float zi = (z + e.hl) * e.inv_dzg;
+    const float zi = __fmul_rn(z + e.hl, e.inv_dzg);
     const uint32_t j = 1 + (int)zi;
     const float c = zi - (float)(j - 1);
     const float d = 1.0f - c;
@@ -105,27 +104,30 @@ __device__ inline uint32_t kick_particle(Part &p, float phi, const KickEnv &e) {
     if (l >= e.tbl_sz || l < 1) l = e.tbl_sz - 1;
     if (m < 1) m = 1;
     const float2 fl = e.fld[l], fl1 = e.fld[l - 1], fm = e.fld[m], fm1 = e.fld[m - 1];
-    cbgr = e.er_c3 * (d * (a * fl.x + bb * fl1.x) + c * (a * fm.x + bb * fm1.x));
-    cbgzs = e.ez_c3 * (d * (a * fl.y + bb * fl1.y) + c * (a * fm.y + bb * fm1.y));
+    cbgr = e.er_c3 * fmaf(d, fmaf(a, fl.x, bb * fl1.x), c * fmaf(a, fm.x, bb * fm1.x));
+    cbgzs = e.ez_c3 * fmaf(d, fmaf(a, fl.y, bb * fl1.y), c * fmaf(a, fm.y, bb * fm1.y));
   }
-  bgx += cbgr * xovr;
-  bgy += cbgr * yovr;
+  // the same bits in every kernel, as the element maps (push32_maps.cuh)
+  const float bgx = fmaf(bgz, p.xp, cbgr * xovr), bgy = fmaf(bgz, p.yp, cbgr * yovr);
   // bgzf = gamma_c (p* + dp + beta_c (1 + (p* + dp)^2 / 2)) taken as
   // bgz + (bgzf - bgz): the change is formed without cancellation and bgz
   // comes straight from the particle's energy
   const float s2 = s0 * s0;
-  const float dbgz = e.gmg * (cbgzs + e.beta * (0.5f * cbgzs * (2.0f * s0 + cbgzs) +
-                                                __fdividef(s2 * s2, 4.0f * (1.0f + 0.5f * s2 + sqrt_fast(1.0f + s2)))));
-  const float bgzf = bgz + dbgz;
+  const float dbgz =
+      e.gmg * fmaf(e.beta,
+                   fmaf(0.5f * cbgzs, fmaf(2.0f, s0, cbgzs),
+                        div_fast(s2 * s2, 4.0f * (fmaf(0.5f, s2, 1.0f) + sqrt_fast(1.0f + s2)))),
+                   cbgzs);
+  const float bgzf = __fadd_rn(bgz, dbgz);
   if (bgzf <= 0.0f) {
     p.lo = 9999u;
     return WR_LOSS;
   }
-  const float inv_f = __fdividef(1.0f, bgzf);
+  const float inv_f = rcp_fast(bgzf);
   p.xp = bgx * inv_f;
   p.yp = bgy * inv_f;
   const float w = e.r.w + dw;
-  p.w = dw + __fdividef(w * (gm + 1.0f) * dbgz, gm * bgz);
+  p.w = fmaf(w * (gm + 1.0f) * dbgz, rcp_fast(gm * bgz), dw);
   return WR_XP | WR_YP | WR_W;
 }
 
