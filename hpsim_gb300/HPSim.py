@@ -586,10 +586,8 @@ class SpaceCharge:
 
     def set_contraction(self, kernel):
         """Contraction kernel of FP32 beams (not in the reference's API):
-        'tensor' (split-BF16 tcgen05 products where the mesh allows) or
-        'cuda' (the FP32 ring convolution on CUDA cores).  A solver that is
-        not told takes the faster one for its mesh: CUDA cores up to
-        nr * nz = 8192, tensor cores above."""
+        'tensor' (the default: split-BF16 tcgen05 products where the mesh
+        allows) or 'cuda' (the FP32 ring convolution on CUDA cores)."""
         call("hps_scheff_set", self._h, 10, {"tensor": 0.0, "cuda": 1.0}[kernel])
 
     def set_surrogate_kernel(self, kernel):

@@ -364,174 +364,5 @@ inline void contract_configure() {
   contract_seg_configure<T, SegCap<MeshSeg>::value>();
 }
 
-// ---- FP32 tables, 32 source radii at a time: the wide form ------------------
-// A block takes kWideRows = 33 field rows of one field radius: 4 blocks for
-// the 129 rows of a 32 x 128 mesh, 132 blocks in all, one per SM, so every
-// SM stages one table (64 KB from L2) where the general form's 297 blocks of
-// 16 rows staged two.  Three groups of 11 points x four quarters of the
-// source rows = 12 warps; a lane keeps one source radius.  Per source row a
-// warp loads one table pair and one charge for 11 packed multiply-adds
-// (fma.rn.f32x2: both field components at once), so the row walk is bound by
-// the FMA pipe, not by shared memory.  The 22 sums of a warp end with a
-// folding tree (31 shuffles; a tree per sum takes 110) and the quarters are
-// added in order.  Bound: staging latency and the FMA pipe, about 1 us each.
-constexpr int kWideP = 11;                       // field points per warp
-constexpr int kWideG = 3;                        // point groups per block
-constexpr int kWideQ = 4;                        // warps sharing a group's source rows
-constexpr int kWideRows = kWideP * kWideG;       // field rows per block
-constexpr int kWideThreads = kWideG * kWideQ * 32;
-
-__device__ __forceinline__ float2 fma_pair(float2 a, float2 b, float2 c) {
-  float2 d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;"
-      : "=l"(*(unsigned long long *)&d)
-      : "l"(*(unsigned long long *)&a), "l"(*(unsigned long long *)&b), "l"(*(unsigned long long *)&c));
-  return d;
-}
-
-inline size_t contract_wide_smem(uint32_t nz) { return (size_t)nz * 32 * (2 * sizeof(float2) + sizeof(float2)); }
-// meshes of the wide form: source radii in whole warps, the two-sided table
-// of 32 of them within a CTA's shared memory (192 KB at nz = 256), and no bin
-// left out of any point's sum (contract_lim)
-inline bool contract_wide_ok(uint32_t nx, uint32_t nz) {
-  return nx % 32 == 0 && nz >= 32 && nz <= 256 && (nz & (nz - 1)) == 0;
-}
-
-__device__ __forceinline__ void contract_wide_body(const ScState *sc, const ScTables &t, uint32_t nx, uint32_t nz,
-                                                   uint32_t rp, uint32_t by) {
-  if (!sc->remesh || sc->sur_accepted || sc->nx != nx || sc->nz != nz) return;
-  extern __shared__ __align__(16) unsigned char contract_raw[];
-  __shared__ float part[kWideQ][kWideRows * 2];
-  float2 *gz = (float2 *)contract_raw;  // [k + nz - 1][32]: g(k), E_z with its sign
-  float2 *qs = gz + 2 * nz * 32;        // [zs][32]: the charge twice
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int grp = warp / kWideQ, quarter = warp % kWideQ;
-  const int zp0 = (int)by * kWideRows + grp * kWideP;
-  const int za = (int)(quarter * nz / kWideQ), zb = (int)((quarter + 1) * nz / kWideQ);
-  const float2 *G = CTab<float>::slice(t, rp, nx * nz);
-  float2 acc[kWideP];
-#pragma unroll
-  for (int j = 0; j < kWideP; ++j) acc[j] = make_float2(0.0f, 0.0f);
-  for (uint32_t rs0 = 0; rs0 < nx; rs0 += 32) {
-    __syncthreads();
-    // two radii a load, every load of a thread's share before its first store
-    constexpr int kStage = 6;
-    const uint32_t npair = nz * 16;
-    for (uint32_t e0 = threadIdx.x; e0 < npair; e0 += kStage * kWideThreads) {
-      float4 gv[kStage];
-      ulonglong2 bv[kStage];
-#pragma unroll
-      for (int u = 0; u < kStage; ++u) {
-        const uint32_t e = e0 + u * kWideThreads, at = (e >> 4) * nx + rs0 + 2 * (e & 15);
-        if (e < npair) {
-          gv[u] = __ldg((const float4 *)(G + at));
-          bv[u] = __ldg((const ulonglong2 *)(t.bin_fx + at));
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < kStage; ++u) {
-        const uint32_t e = e0 + u * kWideThreads, z = e >> 4, r = 2 * (e & 15);
-        if (e < npair) {
-          *(float4 *)(gz + (nz + z) * 32 + r) = gv[u];                                                  // k = z + 1
-          *(float4 *)(gz + (nz - 1 - z) * 32 + r) = make_float4(gv[u].x, -gv[u].y, gv[u].z, -gv[u].w);  // k = -z
-          const float q0 = CTab<float>::charge(bv[u].x), q1 = CTab<float>::charge(bv[u].y);
-          *(float4 *)(qs + z * 32 + r) = make_float4(q0, q0, q1, q1);
-        }
-      }
-    }
-    __syncthreads();
-    if (zp0 > (int)nz) continue;
-    // ring slot (j - u) mod R holds g(zp0 + j - zs), u = zs - zs0; the slot
-    // (R - 1 - u) mod R is free at row zs and takes g(zp0 - zs - 1)
-    constexpr int R = kWideP + 1;
-    float2 ring[R];
-    const float2 *h = gz + lane;
-#pragma unroll
-    for (int j = 0; j < kWideP; ++j) ring[j] = h[(nz - 1 + min(zp0 + j - za, (int)nz)) * 32];
-    const float2 *hp = h + ((int)nz - 1 + zp0 - za - 1) * 32;  // g(zp0 - zs - 1) at zs = za
-    const float2 *qp = qs + za * 32 + lane;
-    for (int zs0 = za; zs0 < zb; zs0 += R, qp += R * 32, hp -= R * 32) {
-#pragma unroll
-      for (int u = 0; u < R; ++u) {
-        if (zs0 + u >= zb) break;
-        if (zs0 + u + 1 < zb) ring[(R - 1 - u) % R] = hp[-u * 32];
-        const float2 q = qp[u * 32];
-#pragma unroll
-        for (int j = 0; j < kWideP; ++j) acc[j] = fma_pair(q, ring[(j - u + R) % R], acc[j]);
-      }
-    }
-  }
-  // the sums over the lanes: at each step a lane keeps one half of its sums
-  // and hands the other to its partner; lane l ends with sum number l
-  float v[32];
-#pragma unroll
-  for (int j = 0; j < 16; ++j) {
-    v[2 * j] = j < kWideP ? acc[j < kWideP ? j : 0].x : 0.0f;
-    v[2 * j + 1] = j < kWideP ? acc[j < kWideP ? j : 0].y : 0.0f;
-  }
-#pragma unroll
-  for (int half = 16; half > 0; half >>= 1) {
-    const bool up = lane & half;
-#pragma unroll
-    for (int i = 0; i < half; ++i) {
-      const float keep = up ? v[i + half] : v[i], send = up ? v[i] : v[i + half];
-      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, half);
-    }
-  }
-  if (lane < 2 * kWideP) part[quarter][grp * 2 * kWideP + lane] = v[0];
-  __syncthreads();
-  if (threadIdx.x < kWideRows * 2) {
-    const uint32_t zp = by * kWideRows + threadIdx.x / 2;
-    if (zp <= nz)
-      t.ffld2[2 * ((size_t)zp * (nx + 1) + rp) + (threadIdx.x & 1)] =
-          ((part[0][threadIdx.x] + part[1][threadIdx.x]) + part[2][threadIdx.x]) + part[3][threadIdx.x];
-  }
-}
-
-// grid (nr + 1, ceil((nz + 1) / kWideRows))
-__global__ void __launch_bounds__(kWideThreads, 1) k_contract_wide(const ScState *sc, ScTables t, uint32_t nx,
-                                                                   uint32_t nz) {
-  contract_wide_body(sc, t, nx, nz, blockIdx.x, blockIdx.y);
-}
-template <int B>
-__global__ void __launch_bounds__(kWideThreads, 1)
-    k_contract_wide_seg(const __grid_constant__ SegArgs<MeshSeg, B> a, uint32_t nx, uint32_t nz) {
-  const MeshSeg &p = a.p[blockIdx.z];
-  contract_wide_body(p.sc, p.t, nx, nz, blockIdx.x, blockIdx.y);
-}
-inline dim3 contract_wide_grid(uint32_t nx, uint32_t nz, uint32_t beams = 1) {
-  return dim3(nx + 1, (nz + 1 + kWideRows - 1) / kWideRows, beams);
-}
-inline void contract_wide_merge(const std::vector<const Rec *> &recs, SegFork &, cudaStream_t st, cudaStream_t) {
-  uint32_t dims[2];
-  std::memcpy(dims, recs[0]->p.data() + sizeof(MeshSeg), sizeof(dims));
-  std::vector<Rec> heads(recs.size());  // the MeshSeg heads of the records
-  std::vector<const Rec *> hp(recs.size());
-  for (size_t k = 0; k < recs.size(); ++k) {
-    heads[k].p.assign(recs[k]->p.begin(), recs[k]->p.begin() + sizeof(MeshSeg));
-    hp[k] = &heads[k];
-  }
-  seg_chunks<MeshSeg>(hp, [&](const auto &a, uint32_t) {
-    k_contract_wide_seg<std::decay_t<decltype(a)>::kB>
-        <<<contract_wide_grid(dims[0], dims[1], a.nb), kWideThreads, contract_wide_smem(dims[1]), st>>>(a, dims[0],
-                                                                                                      dims[1]);
-  });
-}
-inline void contract_wide_launch(const ScState *sc, const ScTables &t, uint32_t nx, uint32_t nz, cudaStream_t st) {
-  if (recorder()) {
-    struct { MeshSeg m; uint32_t dims[2]; } p{{sc, t}, {nx, nz}};
-    record("contract_wide", &contract_wide_merge, 0, p, (uint64_t)nx << 32 | nz);
-    return;
-  }
-  k_contract_wide<<<contract_wide_grid(nx, nz), kWideThreads, contract_wide_smem(nz), st>>>(sc, t, nx, nz);
-}
-inline void contract_wide_configure() {
-  const int most = (int)contract_wide_smem(256);
-  cudaFuncSetAttribute(k_contract_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-  cudaFuncSetAttribute(k_contract_wide_seg<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-  cudaFuncSetAttribute(k_contract_wide_seg<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-  cudaFuncSetAttribute(k_contract_wide_seg<SegCap<MeshSeg>::value>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-}
-
 }  // namespace
 }  // namespace hps

@@ -234,9 +234,6 @@ void sc32_configure();
 // the tensor-core contraction (contract_tc.cuh): meshes it takes, and the
 // bytes of its folded split-BF16 Green's table and of its partial fields
 bool sc32_tc_mesh(uint32_t nr, uint32_t nz);
-// meshes that a solver left to choose solves on CUDA cores (contract.cuh's
-// wide form) although the tensor cores could take them
-bool sc32_cuda_faster(uint32_t nr, uint32_t nz);
 size_t sc32_tc_bytes(uint32_t nr, uint32_t nz, size_t *partial_bytes);
 void contract32(const ScState *sc, const ScTables &t, uint32_t nx_max, uint32_t nz_max, bool mesh_fixed,
                 cudaStream_t st);

@@ -105,7 +105,6 @@ struct hps_scheff_s {
   SurNet *sur = nullptr;  // field surrogate, owned
   int sur_kernel = 1;     // its layers: 0 tensor cores where the layer allows, 1 CUDA cores (faster at batch 1)
   int contraction = 0;    // FP32 beams: 0 tensor cores where the mesh allows, 1 CUDA cores
-  bool contraction_auto = true;  // not set by the caller: tensor cores only on meshes where they are the faster ones
 };
 
 // The host-side state of a simulator that a range advances (engine, beam
@@ -839,8 +838,7 @@ static void scheff_free_tables(hps_scheff_t s) {
 }
 
 // the tensor-core contraction's buffers for the largest mesh (FP32 beams),
-// when that mesh allows it and the solver does not ask for CUDA cores (nor,
-// left to choose, finds them faster there)
+// when that mesh allows it and the solver does not ask for CUDA cores
 static hps_status scheff_alloc_tc(hps_scheff_t s) {
   if (s->t.tcg) cudaFree(s->t.tcg);
   if (s->t.tcp) cudaFree(s->t.tcp);
@@ -848,7 +846,6 @@ static hps_status scheff_alloc_tc(hps_scheff_t s) {
   s->t.tcp = nullptr;
   s->t.tc_nr = s->t.tc_nz = 0;
   if (s->contraction != 0 || !sc32_tc_mesh(s->nx_max, s->nz_max)) return HPS_OK;
-  if (s->contraction_auto && sc32_cuda_faster(s->nx_max, s->nz_max)) return HPS_OK;
   size_t pb = 0;
   const size_t gb = sc32_tc_bytes(s->nx_max, s->nz_max, &pb);
   unsigned char *g = nullptr;
@@ -919,10 +916,9 @@ hps_status hps_scheff_set(hps_scheff_t s, int param, double v) {
     case 5: s->fraction = v; break;
     case 10: {
       if (v != 0.0 && v != 1.0) return fail(HPS_ERR_INVALID, "scheff_set: contraction kernel is 0 or 1");
-      if ((int)v == s->contraction && !s->contraction_auto) return HPS_OK;
+      if ((int)v == s->contraction) return HPS_OK;
       CK(cudaDeviceSynchronize());
       s->contraction = (int)v;
-      s->contraction_auto = false;
       hps_status st = scheff_alloc_tc(s);
       if (st) return st;
       break;
@@ -2071,15 +2067,12 @@ struct Shape {
   uint32_t dep_per_sm, sweep_cap, dep_agg, dep_threads;
 };
 
-// the contraction kernel a solver runs: its choice, or the one it found faster
-int contraction_of(hps_scheff_t s) { return s->contraction_auto ? (s->t.tcg ? 0 : 1) : s->contraction; }
-
 hps_status shape_apply(hps_sim_t s, const Shape &sh) {
   s->dep_per_sm = sh.dep_per_sm;
   s->sweep_cap = sh.sweep_cap;
   s->dep_agg = sh.dep_agg;
   s->dep_threads = sh.dep_threads;
-  if (s->sc && contraction_of(s->sc) != sh.contraction) {
+  if (s->sc && s->sc->contraction != sh.contraction) {
     hps_status e = hps_scheff_set(s->sc, 10, (double)sh.contraction);
     if (e) return e;
   }
@@ -2112,7 +2105,7 @@ std::string tune_key(hps_sim_t s, const char *what) {
 template <class Run, class Restore>
 hps_status tune_search(const std::vector<hps_sim_t> &sims, bool fp32, bool tc_ok, int reps, Run run,
                        Restore restore, Shape *best_out, std::vector<double> *times) {
-  Shape best{sims[0]->sc ? contraction_of(sims[0]->sc) : 0, sims[0]->dep_per_sm, sims[0]->sweep_cap,
+  Shape best{sims[0]->sc ? sims[0]->sc->contraction : 0, sims[0]->dep_per_sm, sims[0]->sweep_cap,
              sims[0]->dep_agg, sims[0]->dep_threads};
   if (!fp32) { *best_out = best; return HPS_OK; }
   auto measure = [&](const Shape &sh, double *ms) -> hps_status {
@@ -2282,7 +2275,7 @@ hps_status hps_batch_autotune(hps_batch_t bt, int32_t start, int32_t end, int32_
 
 hps_status hps_sim_get_shape(hps_sim_t s, int32_t *shape_out) {
   if (!s || !shape_out) return fail(HPS_ERR_INVALID, "sim_get_shape: bad argument");
-  shape_out[0] = s->sc ? contraction_of(s->sc) : 0;
+  shape_out[0] = s->sc ? s->sc->contraction : 0;
   shape_out[1] = (int32_t)s->dep_per_sm;
   shape_out[2] = (int32_t)s->sweep_cap;
   shape_out[3] = (int32_t)s->dep_agg;

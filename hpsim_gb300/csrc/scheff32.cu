@@ -877,22 +877,12 @@ void sc32_configure() {
     cudaFuncSetAttribute(k32_deposit_seg<SegCap<DepSeg>::value>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)kMaxHistSmem);
     contract_configure<float>();
-    contract_wide_configure();
     const cudaError_t e = contract_tc_configure();
     if (e != cudaSuccess) set_error(HPS_ERR_CUDA, cudaGetErrorString(e));
   });
 }
 
 bool sc32_tc_mesh(uint32_t nr, uint32_t nz) { return tc_mesh_ok(nr, nz); }
-// The tensor cores' product carries a Toeplitz expansion, three split-BF16
-// products and a second launch that sums the per-radius partials; it pays
-// once the sum itself is large.  Measured per kick, whole kick (us), wide
-// form against tensor cores: 1,048,576 particles 61.7 : 70.2 at 32 x 128,
-// 73.8 : 78.0 at 32 x 256, 76.4 : 79.8 at 64 x 128, 125.7 : 107.1 at
-// 64 x 256; 20,011 particles 30.6 : 38.3, 43.4 : 47.2, 45.6 : 48.5,
-// 82.8 : 62.5.  The sum's work grows with (nr nz)^2, so the line is at
-// nr nz = 8192.
-bool sc32_cuda_faster(uint32_t nr, uint32_t nz) { return contract_wide_ok(nr, nz) && nr * nz <= 8192; }
 size_t sc32_tc_bytes(uint32_t nr, uint32_t nz, size_t *partial_bytes) {
   *partial_bytes = tc_partial_bytes(nr, nz);
   return tc_table_bytes(nr, nz);
@@ -900,8 +890,7 @@ size_t sc32_tc_bytes(uint32_t nr, uint32_t nz, size_t *partial_bytes) {
 
 // UpdateFldTbl2KernelDouble for FP32 tables: the tensor-core kernels when
 // the solver holds their buffers for the largest mesh it takes, the FP32
-// ring convolution otherwise (its wide form where the kick's mesh is known
-// on the host and allows it).  Each returns at once when the other one is
+// ring convolution otherwise.  Each returns at once when the other one is
 // the one for the kick's mesh; mesh_fixed (the kick's mesh is the largest
 // one, decided on the host) leaves out the one that cannot run.
 void contract32(const ScState *sc, const ScTables &t, uint32_t nx_max, uint32_t nz_max, bool mesh_fixed,
@@ -912,10 +901,7 @@ void contract32(const ScState *sc, const ScTables &t, uint32_t nx_max, uint32_t 
     contract_tc_launch(sc, t, nx_max, nz_max, st);
     if (!rec) note_launch(2);
   }
-  if (!tc && mesh_fixed && contract_wide_ok(nx_max, nz_max)) {
-    contract_wide_launch(sc, t, nx_max, nz_max, st);
-    if (!rec) note_launch();
-  } else if (!tc || !mesh_fixed) {
+  if (!tc || !mesh_fixed) {
     contract_launch<float>(sc, t, nx_max, nz_max, st);
     if (!rec) note_launch();
   }
@@ -962,7 +948,7 @@ hps_status hps_scheff_field_f32_kernel(uint32_t nr, uint32_t nz, const double *b
     return (hps_status)set_error(HPS_ERR_UNSUPPORTED,
                                  "scheff_field_f32: the tensor-core contraction takes nz in 128..512 and nr in "
                                  "16..64 (powers of two)");
-  const bool tc = kernel == 2 || (kernel == 0 && tc_mesh_ok(nr, nz) && !sc32_cuda_faster(nr, nz));
+  const bool tc = kernel == 2 || (kernel == 0 && tc_mesh_ok(nr, nz));
   sc32_configure();
   size_t nb = (size_t)nr * nz, n1 = (size_t)(nr + 1) * nr * nz * 2, n2 = (size_t)(nz + 1) * (nr + 1) * 2;
   ScState *sc = nullptr;

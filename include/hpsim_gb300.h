@@ -204,8 +204,7 @@ hps_status hps_scheff_destroy(hps_scheff_t s);
  * No reference counterpart: 10 the contraction kernel of FP32 beams (0, the
  * default: split-BF16 tensor cores where the mesh allows -- nz a power of
  * two in 128..512, nr in 16..64 -- else the FP32 ring convolution; 1: the
- * ring convolution always; never set: the ring convolution up to nr nz =
- * 8192, where it is the faster one, else as 0); read-only: 11 the solver holds the tensor-core
+ * ring convolution always); read-only: 11 the solver holds the tensor-core
  * buffers, 12 a bounded wait of the tensor-core kernel gave up (1).
  * 13 the attached surrogate's layers: 0 on the tensor cores where the
  * layer's shape allows (c_out <= 128, c_in a power of two, w_in even), 1
@@ -254,8 +253,7 @@ hps_status hps_scheff_field_noalloc(uint32_t nr, uint32_t nz, const double *bins
  * that its error against the FP64 table can be stated. */
 hps_status hps_scheff_field_f32(uint32_t nr, uint32_t nz, const double *bins, const double *mesh, double *field);
 /* hps_scheff_field_f32 with the contraction kernel chosen: 0 the one FP32
- * beams use for the mesh (the tensor cores where the mesh allows and nr nz
- * is above 8192), 1 the
+ * beams use for the mesh (the tensor cores where the mesh allows), 1 the
  * FP32 ring convolution on CUDA cores, 2 the split-BF16 tensor-core product
  * (tcgen05; nz a power of two in 128..512, nr in 16..64, else
  * HPS_ERR_UNSUPPORTED).  Same computation as UpdateFinalFldTblKernelCall,
