@@ -5,9 +5,9 @@
 // space_charge.cpp) and SimulationEngine (src/simulation/src/
 // simulation_engine.{cpp,cu}).  All particle work is issued on the beam's
 // CUDA stream; a simulate() call issues a fixed launch sequence (the
-// space-charge decisions live on the device), which is captured once into a
-// CUDA graph and replayed while the lattice and the engine's host state are
-// unchanged.
+// space-charge decisions live on the device): kernel by kernel the first time
+// its inputs are seen, captured into a CUDA graph the second time and replayed
+// while the lattice and the engine's host state are unchanged.
 #include <algorithm>
 #include <atomic>
 #include <cctype>
@@ -123,6 +123,7 @@ struct GraphEntry {
   uint64_t serial = 0;          // bumped at every capture
   HostState after{};            // host state after the range
   uint64_t nkernels = 0;        // kernels in the captured graph
+  uint64_t ran = 0;             // key of the last range that was launched kernel by kernel
 };
 
 struct hps_sim_s {
@@ -1521,6 +1522,38 @@ void host_put(hps_sim_t s, const HostState &h) {
   if (s->sc) { s->sc->fraction = h.fraction; s->sc->interval = h.interval; }
 }
 
+// Whether visiting the range may end in a lattice error: the neighbours that
+// the gaps' visitors ask for, taken on the strict side.
+bool range_may_fail(const RunPlan &p) {
+  const hps_beamline_t bl = p.c.bl;
+  for (int i = 0; i <= p.end_index; ++i) {
+    const int type = bl->types[i], before = T(bl, (int64_t)i - 1), after = T(bl, (int64_t)i + 1);
+    if (i < p.start_index && type != HPS_ELEM_SPCHCOMP) continue;
+    if (type < HPS_ELEM_DRIFT || type > HPS_ELEM_DIPOLE) return true;
+    if (type == HPS_ELEM_RFGAP_DTL && (i == 0 || before != HPS_ELEM_QUAD || after != HPS_ELEM_QUAD)) return true;
+    if (type == HPS_ELEM_RFGAP_CCL && (i == p.start_index || before != HPS_ELEM_RFGAP_CCL) &&
+        after != HPS_ELEM_RFGAP_CCL && after != HPS_ELEM_RFGAP_DTL)
+      return true;
+  }
+  return false;
+}
+
+// Whether the range is launched kernel by kernel instead of as a graph: the
+// first time its inputs are seen.  A graph pays from the second replay on: a
+// capture costs the host as much as the launches themselves, and its
+// instantiation and the old one's destruction three times that (0.8 ms for the
+// 40 kicks of the quad channel, as long as the GPU works on 20,000 particles),
+// all before the GPU starts.  A program that changes a set point before every
+// pass never comes back to a graph; one that repeats a pass gets it at the
+// second.  A range that may end in an error is captured, so that nothing has
+// run when it does.
+bool launch_directly(const RunPlan &p) {
+  GraphEntry &g = p.c.s->graph;
+  if ((g.exec && g.key == p.key) || g.ran == p.key || range_may_fail(p)) return false;
+  g.ran = p.key;
+  return true;
+}
+
 // The simulator's graph for the plan: the cached one when the host state
 // matches (the host state then moves to the end of the range, as a replay
 // does), else a new capture (which moves it while recording).  The graph is
@@ -1681,12 +1714,13 @@ hps_status hps_sim_simulate(hps_sim_t s, int32_t start, int32_t end) {
   hps_sim_t sim = s;
   Ctx &c = p.c;
   cudaStream_t st = c.b->stream;
-  CK(cudaEventRecord(sim->ev0, st));
-  if (p.graph) {
+  if (p.graph && !launch_directly(p)) {
     e = prepare_graph(p);
     if (e) return e;
+    CK(cudaEventRecord(sim->ev0, st));
     CK(cudaGraphLaunch(sim->graph.exec, st));
   } else {
+    CK(cudaEventRecord(sim->ev0, st));
     e = run_range(c, p.start_index, p.end_index, p.monitor, p.host_sync);
     if (e) return e;
   }
@@ -2099,8 +2133,8 @@ std::string tune_key(hps_sim_t s, const char *what) {
 // The search: coordinate descent over the four knobs (contraction kernel,
 // then deposit blocks per SM, then sweep blocks per SM, then aggregated
 // deposit adds), each candidate
-// timed as the median of `reps` runs after one untimed run (which captures
-// its graph), every run from the snapshot.  run() simulates and returns the
+// timed as the median of `reps` runs after two untimed runs (the second
+// captures its graph), every run from the snapshot.  run() simulates and returns the
 // device time in ms.
 template <class Run, class Restore>
 hps_status tune_search(const std::vector<hps_sim_t> &sims, bool fp32, bool tc_ok, int reps, Run run,
@@ -2114,13 +2148,13 @@ hps_status tune_search(const std::vector<hps_sim_t> &sims, bool fp32, bool tc_ok
       if (e) return e;
     }
     std::vector<double> v;
-    for (int r = 0; r <= reps; ++r) {
+    for (int r = 0; r <= reps + 1; ++r) {
       hps_status e = restore();
       if (e) return e;
       double t = 0.0;
       e = run(&t);
       if (e) return e;
-      if (r > 0) v.push_back(t);
+      if (r > 1) v.push_back(t);
     }
     std::sort(v.begin(), v.end());
     *ms = v[v.size() / 2];
