@@ -14,7 +14,7 @@
 // the 127 + nz offsets that tile needs, in chunks of 64, N = 2 (nr + 1)
 // rounded up to a multiple of 16 (the padding rows of B are zero).  The
 // last field row zp = nz needs offsets k = 1 .. nz only, which are all in
-// the last tile's chunks: that tile's producer threads sum it from the B
+// the last tile's chunks: that tile's last four warps sum it from the B
 // tiles while they are staged, one row of B (one (rp, component)) each.
 //
 // Precision: split BF16.  Both operands are written as hi = bf16(x), lo =
@@ -30,12 +30,24 @@
 // zero-padded column, which the producer warps copy with 16-byte shared-
 // memory loads from 8 shifted copies of it and store swizzled.
 //
-// Warp roles (160 threads): warps 0-3 build the A tiles and issue the bulk
-// copies, then read the accumulator back (warp w owns TMEM lanes 32w..);
-// warp 4 allocates the tensor memory and one of its threads issues the MMAs
-// and commits them to the stage's "empty" barrier.  Every wait is bounded
-// (about a second); a wait that gives up sets the solver's error word, and
-// the CTA drains its copies and MMAs before it frees the tensor memory.
+// Warp roles (416 threads): warps 0-3 build the hi half of the A tiles and
+// warps 4-7 the lo half (thread 0 issues the bulk copies), then both read the
+// accumulator back (a warp owns TMEM lanes 32 (warp mod 4)..); warp 8
+// allocates the tensor memory and one of its threads issues the MMAs and
+// commits them to the stage's "empty" barrier; warps 9-12 sum the last field
+// row.  Every wait is bounded (about a second); a wait that gives up sets the
+// solver's error word, and the CTA drains its copies and MMAs before it frees
+// the tensor memory.
+//
+// A CTA's time is its chain of latencies (the charge column, its shifted
+// copies, a chunk's A tile, the MMAs, the accumulator's way out), not the
+// product.  One set of producers that also summed the last row between two
+// chunks, with three stages, took 9.8 us at 32 x 128 and 17.7 at 64 x 256;
+// the halves of A side by side, the last row on warps of its own and a stage
+// per chunk where they fit take 7.6 and 13.8.  (Slices of the columns on the
+// SMs that 32 CTAs leave idle took 7.3 at 32 x 128, and made a batch of 32
+// beams 14% slower: every slice builds A again.)  No accumulator's order of
+// terms depends on any of this.
 //
 // The per-radius partial tiles (and last-row partials) are summed in a
 // fixed order by k_tc_reduce: results are deterministic.
@@ -54,8 +66,10 @@ namespace {
 
 constexpr int kTcM = 128;           // field rows per tile (MMA M)
 constexpr int kTcKC = 64;           // offsets per chunk (one 128-byte swizzle row of BF16)
-constexpr int kTcThreads = 160;     // 4 producer / epilogue warps + 1 MMA warp
-constexpr int kTcProducers = 128;
+constexpr int kTcThreads = 416;     // 8 producer / epilogue warps, 1 MMA warp, 4 last-row warps
+constexpr int kTcProducers = 256;   // threads that write A
+constexpr int kTcBuilders = 384;    // threads that write the shifted charge copies
+constexpr int kTcStages = 4;
 constexpr size_t kTcSmemMax = 227 * 1024;
 
 // meshes the tensor-core path takes: nz a multiple of the tile height, N
@@ -90,11 +104,13 @@ __host__ __device__ inline size_t tc_stage_bytes(uint32_t BT) { return 2 * 16384
 
 inline TcDims tc_dims(uint32_t nr, uint32_t nz) {
   TcDims d{};
-  d.nr = nr; d.nz = nz; d.N = tc_n(nr); d.cols = tc_tmem_cols(d.N); d.NC = 2 * nz / kTcKC; d.CPT = nz / kTcKC + 2;
+  d.nr = nr; d.nz = nz; d.N = tc_n(nr); d.NC = 2 * nz / kTcKC; d.CPT = nz / kTcKC + 2;
   d.BT = d.N * 128; d.L = nz + 264; d.tiles = nz / kTcM;
+  d.cols = tc_tmem_cols(d.N);
   // 256 bytes are left for the kernel's static shared memory (barriers)
   const size_t fixed = 1024 + (size_t)16 * d.L * 2 + (size_t)nz * 4 + 256;
-  d.S = fixed + 3 * tc_stage_bytes(d.BT) <= kTcSmemMax ? 3 : 2;
+  d.S = 2;
+  while (d.S < (uint32_t)kTcStages && d.S < d.CPT && fixed + (d.S + 1) * tc_stage_bytes(d.BT) <= kTcSmemMax) ++d.S;
   d.smem = fixed + d.S * tc_stage_bytes(d.BT);
   return d;
 }
@@ -148,31 +164,32 @@ __device__ __forceinline__ void contract_tc_body(const ScState *sc, const ScTabl
                                                  uint32_t tile, uint32_t rs) {
   if (!tc_go(sc, t)) return;
   extern __shared__ unsigned char tc_raw[];
-  __shared__ uint64_t full[3], empty[3], done;
+  __shared__ uint64_t full[kTcStages], empty[kTcStages], done;
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
   const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t N = d.N, nz = d.nz, nr = d.nr, S = d.S, BT = d.BT, L = d.L;
   // 1024-byte aligned stage buffers, then the shifted charge copies and the column
   unsigned char *sm = (unsigned char *)(((uintptr_t)tc_raw + 1023) & ~(uintptr_t)1023);
-  const size_t stage = tc_stage_bytes(BT);
+  const size_t stage = tc_stage_bytes(d.BT);
   __nv_bfloat16 *cp = (__nv_bfloat16 *)(sm + S * stage);  // [h][s][L]
   float *qc = (float *)(sm + S * stage + (size_t)16 * L * 2);
   volatile int *abort = &abort_flag;
+  // the last tile's last-row warps also read its B tiles
+  const bool last_row = tile + 1 == d.tiles;
 
   // the charge column first: its loads overlap the set-up below
-  if (warp < 4)
-    for (uint32_t zs = tid; zs < nz; zs += kTcProducers) qc[zs] = tc_charge(__ldg(t.bin_fx + zs * nr + rs));
+  for (uint32_t zs = tid; zs < nz; zs += kTcThreads) qc[zs] = tc_charge(__ldg(t.bin_fx + zs * nr + rs));
   if (tid == 0) {
     for (uint32_t s = 0; s < S; ++s) {
       mbar_init(&full[s], kTcProducers + 1);
-      mbar_init(&empty[s], 1);
+      mbar_init(&empty[s], last_row ? 5 : 1);
     }
     mbar_init(&done, 1);
     abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 4) {
+  if (warp == 8) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem(&tmem_slot)),
                  "r"(d.cols)
                  : "memory");
@@ -183,26 +200,24 @@ __device__ __forceinline__ void contract_tc_body(const ScState *sc, const ScTabl
   tc_fence_after();
   const uint32_t tmem = tmem_slot;
   const uint32_t c0 = 2 * tile, nch = d.CPT;  // this tile's chunks of the folded range
+  const unsigned char *gsrc = (const unsigned char *)t.tcg + (size_t)rs * d.NC * 2 * BT;
+  auto fetch = [&](uint32_t i) {  // chunk i's B tiles
+    const uint32_t s = i % S;
+    unsigned char *st = sm + s * stage + 2 * 16384;
+    const unsigned char *src = gsrc + (size_t)(c0 + i) * 2 * BT;
+    mbar_arrive_tx(&full[s], 2 * BT);
+    bulk_g2s(st, src, BT, &full[s]);
+    bulk_g2s(st + BT, src + BT, BT, &full[s]);
+  };
   bool issued_mma = false;
 
-  if (warp < 4) {
-    // ---- producers: the B tiles of the first stages in flight, the charge
-    // column's shifted copies, then per chunk the A tile (and the B tile of
-    // the chunks after the first S) ----
-    const unsigned char *gsrc = (const unsigned char *)t.tcg + (size_t)rs * d.NC * 2 * BT;
-    if (tid == 0) {
-      for (uint32_t i = 0; i < S && i < nch; ++i) {
-        unsigned char *st = sm + i * stage;
-        mbar_arrive_tx(&full[i], 2 * BT);
-        const unsigned char *src = gsrc + (size_t)(c0 + i) * 2 * BT;
-        bulk_g2s(st + 2 * 16384, src, BT, &full[i]);
-        bulk_g2s(st + 2 * 16384 + BT, src + BT, BT, &full[i]);
-      }
-    }
+  if (warp != 8) {
+    if (tid == 0)
+      for (uint32_t i = 0; i < S && i < nch; ++i) fetch(i);
     // copy s, element x holds R(x + s - 128), R(v) = q(nz - 1 - v) inside the
     // mesh; eight elements per 16-byte store (L is a multiple of 8)
-    const uint32_t groups = L / 8;
-    for (uint32_t e = tid; e < 8 * groups; e += kTcProducers) {
+    const uint32_t groups = L / 8, bt = warp < 8 ? tid : tid - 32;
+    for (uint32_t e = bt; e < 8 * groups; e += kTcBuilders) {
       const uint32_t s = e / groups, x0 = (e % groups) * 8;
       __align__(16) __nv_bfloat16 hv[8], lv[8];
 #pragma unroll
@@ -215,71 +230,71 @@ __device__ __forceinline__ void contract_tc_body(const ScState *sc, const ScTabl
       *(uint4 *)(cp + s * L + x0) = *(const uint4 *)hv;
       *(uint4 *)(cp + (8 + s) * L + x0) = *(const uint4 *)lv;
     }
-    asm volatile("bar.sync 1, 128;" ::: "memory");
-    const uint32_t m = tid;  // the A row this thread writes
-    // the last tile's threads also sum the last field row from B rows tid
-    // and tid + 128 (n < N) of the chunks of offsets 1 .. nz
-    const bool last_row = tile + 1 == d.tiles;
-    float lr0 = 0.0f, lr1 = 0.0f;
+    asm volatile("bar.sync 1, 384;" ::: "memory");
+  }
+  if (warp < 8) {
+    // ---- producers: per chunk one half of the A tile (thread 0: the B tile
+    // of the chunks after the first S) ----
+    const uint32_t m = tid & 127, h = tid >> 7;  // the A row this thread writes, hi or lo
     for (uint32_t i = 0; i < nch && !*abort; ++i) {
       const uint32_t s = i % S, use = i / S;
       if (use > 0 && !mbar_wait(&empty[s], (use - 1) & 1, abort)) break;
-      unsigned char *st = sm + s * stage;
-      if (tid == 0 && use > 0) {
-        mbar_arrive_tx(&full[s], 2 * BT);
-        const unsigned char *src = gsrc + (size_t)(c0 + i) * 2 * BT;
-        bulk_g2s(st + 2 * 16384, src, BT, &full[s]);
-        bulk_g2s(st + 2 * 16384 + BT, src + BT, BT, &full[s]);
-      }
+      if (tid == 0 && use > 0) fetch(i);
       // row m of the chunk: R(W .. W + 63), W = 64 i - m (+128 into the copies)
       const int wp = 64 * (int)i - (int)m + 128;
       const int sh = wp & 7, base = wp - sh;
-      const uint4 *hi = (const uint4 *)(cp + sh * L + base);
-      const uint4 *lo = (const uint4 *)(cp + (8 + sh) * L + base);
-      unsigned char *ah = st + (m >> 3) * 1024 + (m & 7) * 128;
-      unsigned char *al = ah + 16384;
+      const uint4 *src = (const uint4 *)(cp + (8 * h + sh) * L + base);
+      unsigned char *a = sm + s * stage + h * 16384 + (m >> 3) * 1024 + (m & 7) * 128;
 #pragma unroll
-      for (uint32_t jj = 0; jj < 8; ++jj) {
-        const uint32_t off = ((jj ^ (m & 7)) & 7) << 4;
-        *(uint4 *)(ah + off) = hi[jj];
-        *(uint4 *)(al + off) = lo[jj];
-      }
+      for (uint32_t jj = 0; jj < 8; ++jj) *(uint4 *)(a + (((jj ^ (m & 7)) & 7) << 4)) = src[jj];
       fence_async_smem();
       mbar_arrive(&full[s]);
-      const uint32_t c = c0 + i;  // this chunk's offsets: kidx = 64 c + j
-      if (last_row && c * kTcKC >= nz) {
-        // B landed (the phase also needs the tile's bytes); offset kidx
-        // k = kidx - (nz - 1) takes the charge of row zs = 2 nz - 1 - kidx
-        if (!mbar_wait(&full[s], use & 1, abort)) break;
-        const unsigned char *bh = st + 2 * 16384, *bl = bh + BT;
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          const uint32_t n = tid + 128 * half;
-          if (n >= N) continue;
-          const uint32_t row = (n >> 3) * 1024 + (n & 7) * 128;
-          float acc = 0.0f;
-#pragma unroll
-          for (uint32_t jj = 0; jj < 8; ++jj) {
-            const uint32_t off = row + (((jj ^ (n & 7)) & 7) << 4);
-            const uint4 vh = *(const uint4 *)(bh + off), vl = *(const uint4 *)(bl + off);
-            const __nv_bfloat16 *h8 = (const __nv_bfloat16 *)&vh, *l8 = (const __nv_bfloat16 *)&vl;
-#pragma unroll
-            for (uint32_t u = 0; u < 8; ++u) {
-              const uint32_t zs = 2 * nz - 1 - (c * kTcKC + 8 * jj + u);
-              acc = fmaf(qc[zs], __bfloat162float(h8[u]) + __bfloat162float(l8[u]), acc);
-            }
-          }
-          if (half == 0) lr0 += acc;
-          else lr1 += acc;
-        }
-      }
     }
-    if (last_row && !*abort) {
-      // rows n < N only: a thread beyond them would write into the next
-      // radius's partials
-      float *pl = t.tcp + (size_t)d.tiles * nr * N * kTcM + (size_t)rs * N;
-      if (tid < N) pl[tid] = lr0;
-      if (tid + 128 < N) pl[tid + 128] = lr1;
+  } else if (warp > 8) {
+    // ---- the last field row, from B rows r and r + 128 (below N) in the
+    // chunks of offsets 1 .. nz ----
+    if (last_row) {
+      const uint32_t r = tid - 288;
+      float lr0 = 0.0f, lr1 = 0.0f;
+      for (uint32_t i = 0; i < nch && !*abort; ++i) {
+        const uint32_t s = i % S, use = i / S;
+        const uint32_t c = c0 + i;  // this chunk's offsets: kidx = 64 c + j
+        if (!mbar_wait(&full[s], use & 1, abort)) break;
+        if (c * kTcKC >= nz) {
+          // offset kidx, k = kidx - (nz - 1), takes the charge of row
+          // zs = 2 nz - 1 - kidx
+          const unsigned char *bh = sm + s * stage + 2 * 16384, *bl = bh + BT;
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            const uint32_t n = r + 128 * half;
+            if (n >= N) continue;
+            const uint32_t row = (n >> 3) * 1024 + (n & 7) * 128;
+            float acc = 0.0f;
+#pragma unroll
+            for (uint32_t jj = 0; jj < 8; ++jj) {
+              const uint32_t off = row + (((jj ^ (n & 7)) & 7) << 4);
+              const uint4 vh = *(const uint4 *)(bh + off), vl = *(const uint4 *)(bl + off);
+              const __nv_bfloat16 *h8 = (const __nv_bfloat16 *)&vh, *l8 = (const __nv_bfloat16 *)&vl;
+#pragma unroll
+              for (uint32_t u = 0; u < 8; ++u) {
+                const uint32_t zs = 2 * nz - 1 - (c * kTcKC + 8 * jj + u);
+                acc = fmaf(qc[zs], __bfloat162float(h8[u]) + __bfloat162float(l8[u]), acc);
+              }
+            }
+            if (half == 0) lr0 += acc;
+            else lr1 += acc;
+          }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&empty[s]);
+      }
+      if (!*abort) {
+        // rows n < N only: a thread beyond them would write into the next
+        // radius's partials
+        float *pl = t.tcp + (size_t)d.tiles * nr * N * kTcM + (size_t)rs * N;
+        if (r < N) pl[r] = lr0;
+        if (r + 128 < N) pl[r + 128] = lr1;
+      }
     }
   } else if (lane == 0) {
     // ---- the MMA thread ----
@@ -304,13 +319,14 @@ __device__ __forceinline__ void contract_tc_body(const ScState *sc, const ScTabl
   }
 
   // ---- epilogue: the accumulator to this (tile, radius) partial ----
-  if (warp < 4) {
+  if (warp < 8) {
     const bool ok = !*abort && mbar_wait(&done, 0, abort);
     if (ok) {
       tc_fence_after();
-      float *out = t.tcp + ((size_t)(tile * nr + rs) * N) * kTcM + 32 * warp + lane;
-      const uint32_t tl = tmem + ((32 * warp) << 16);
-      for (uint32_t c = 0; c < N; c += 16) {
+      const uint32_t lanes = 32 * (warp & 3);
+      float *out = t.tcp + ((size_t)(tile * nr + rs) * N) * kTcM + lanes + lane;
+      const uint32_t tl = tmem + (lanes << 16);
+      for (uint32_t c = 16 * (warp >> 2); c < N; c += 32) {
         float v[16];
         tc_ld16(tl + c, v);
 #pragma unroll
@@ -325,7 +341,7 @@ __device__ __forceinline__ void contract_tc_body(const ScState *sc, const ScTabl
     // land (both finish on their own within microseconds), then free the
     // tensor memory
     if (tid == 0) atomicOr((unsigned int *)&((ScState *)sc)->tc_error, 1u);
-    if (warp == 4 && lane == 0 && issued_mma) {
+    if (warp == 8 && lane == 0 && issued_mma) {
       tc_commit(&done);
       int dummy = 0;
       (void)mbar_wait(&done, 0, &dummy);
@@ -335,7 +351,7 @@ __device__ __forceinline__ void contract_tc_body(const ScState *sc, const ScTabl
     }
     __syncthreads();
   }
-  if (warp == 4) {
+  if (warp == 8) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(d.cols) : "memory");
   }
