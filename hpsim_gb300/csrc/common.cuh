@@ -109,7 +109,7 @@ struct Sc32Host {
 
 struct ScTables {
   unsigned long long *bin_fx;  // fixed-point deposit, nz_max*nx_max
-  double *fld1;                // (nx+1)*nx*nz (x,y interleaved)
+  double *fld1;                // (nx+1)*nz*nx (x,y interleaved)
   double *fld2;                // (nz+1)*(nx+1) (x,y interleaved)
   float *ffld1, *ffld2;        // FP32 variants (FP32 beams)
   Sc32Consts *c32;             // FP32 beams: constants of the current kick

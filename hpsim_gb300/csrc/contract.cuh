@@ -36,16 +36,11 @@ constexpr int kContractThreads = kCG * kCH * 32;
 // an FP64 128-row mesh (two CTAs per SM; lanes run over source radii)
 constexpr int kContractSmem = 96 * 1024;
 
-// the FP32 and FP64 tables: pair type, table layout, charge conversion
+// the FP32 and FP64 tables ([rp][dz][rs], rs fastest): pair type, charge conversion
 template <class T> struct CTab;
 template <> struct CTab<float> {
   using V = float2;
-  // FP32 Green's table [rp][dz][rs] (ScTables::ffld1)
-  static __device__ const V *slice(const ScTables &t, uint32_t rp, uint32_t fld) {
-    return (const V *)t.ffld1 + (size_t)rp * fld;
-  }
-  static __device__ size_t at(uint32_t z, uint32_t rs, uint32_t nx, uint32_t) { return (size_t)z * nx + rs; }
-  static constexpr bool kZFast = false;  // consecutive table entries run over rs
+  static __device__ const V *table(const ScTables &t) { return (const V *)t.ffld1; }
   // 2^-36 fixed-point charge through two 32-bit conversions (a 64-bit
   // integer conversion runs on the FP64 pipe)
   static __device__ float charge(unsigned long long v) {
@@ -58,12 +53,7 @@ template <> struct CTab<float> {
 };
 template <> struct CTab<double> {
   using V = double2;
-  // FP64 Green's table [rp][rs][dz] (ScTables::fld1)
-  static __device__ const V *slice(const ScTables &t, uint32_t rp, uint32_t fld) {
-    return (const V *)t.fld1 + (size_t)rp * fld;
-  }
-  static __device__ size_t at(uint32_t z, uint32_t rs, uint32_t, uint32_t nz) { return (size_t)rs * nz + z; }
-  static constexpr bool kZFast = true;   // consecutive table entries run over dz
+  static __device__ const V *table(const ScTables &t) { return (const V *)t.fld1; }
   static __device__ double charge(unsigned long long v) { return (double)(long long)v * kBinInvScale; }
   static __device__ double *out(const ScTables &t) { return t.fld2; }
 };
@@ -132,7 +122,7 @@ __device__ __forceinline__ void contract_block(const ScState *sc, const ScTables
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int grp = warp / kCH, half = warp % kCH;
   const uint32_t za = half * nz / kCH, zb = (half + 1) * nz / kCH;  // this warp's source rows
-  const V *G = CTab<T>::slice(t, rp, fld_sz);
+  const V *G = CTab<T>::table(t) + (size_t)rp * fld_sz;
   T axs[S][kCP], azs[S][kCP];
 #pragma unroll
   for (int sl = 0; sl < S; ++sl)
@@ -152,8 +142,8 @@ __device__ __forceinline__ void contract_block(const ScState *sc, const ScTables
       for (int u = 0; u < kStage; ++u) {
         const uint32_t e = e0 + u * blockDim.x;
         if (e < ntile) {
-          const uint32_t z = CTab<T>::kZFast ? e % nz : e / ntr, r = CTab<T>::kZFast ? e / nz : e % ntr;
-          gv[u] = __ldg(G + CTab<T>::at(z, rs0 + r, nx, nz));
+          const uint32_t z = e / ntr, r = e % ntr;
+          gv[u] = __ldg(G + (size_t)z * nx + rs0 + r);
           bv[u] = __ldg(t.bin_fx + z * nx + rs0 + r);
         }
       }
@@ -161,7 +151,7 @@ __device__ __forceinline__ void contract_block(const ScState *sc, const ScTables
       for (int u = 0; u < kStage; ++u) {
         const uint32_t e = e0 + u * blockDim.x;
         if (e < ntile) {
-          const uint32_t z = CTab<T>::kZFast ? e % nz : e / ntr, r = CTab<T>::kZFast ? e / nz : e % ntr;
+          const uint32_t z = e / ntr, r = e % ntr;
           if (M) {
             gz[(nz + z) * tr + r] = gv[u];                               // k = z + 1
             gz[(nz - 1 - z) * tr + r] = cpair<T, V>(gv[u].x, -gv[u].y);  // k = -z

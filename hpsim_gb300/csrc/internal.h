@@ -111,8 +111,6 @@ void sc_mesh(const DevBeam &b, ScState *sc, const ScTables &t, const ScKickArgs 
              cudaStream_t st, const SurNet *sur = nullptr);
 void sc_kick(const DevBeam &b, ScState *sc, const ScTables &t, const ScKickArgs &a, cudaStream_t st);
 void beam_update_stat_for_sc(const DevBeam &b, PassScratch s, cudaStream_t st);
-// Green's table (k_green) for a solver whose state says "remesh"
-void sc_green(const ScState *sc, const ScTables &t, uint32_t num_part, double cur_ov_mc2, cudaStream_t st);
 
 // ---- SCHEFF field surrogate (nn.cu, surrogate.cu) ------------------------
 // dims = {batch, c_in, c_out, h_in, w_in, stride, up}; skip may be null

@@ -16,6 +16,7 @@
 #include "../../include/hpsim_gb300.h"
 #include "internal.h"
 #include "contract.cuh"
+#include "contract64.cuh"
 #include "reduce.cuh"
 #include "scheff_common.cuh"
 
@@ -177,11 +178,37 @@ __global__ void k_decide_only(DevBeam b, ScState *sc, ScTables t, double freq, d
   zero_mesh_tables(sc, t, threadIdx.x, blockDim.x);
 }
 
-// UpdateFldTbl1Kernel, space_charge_kernel.cu:39-100 (one thread per table
-// entry; rows rs >= (nr/by)*by are not written, as in the reference's grid);
-// not needed when a field surrogate's field was accepted
-__global__ void k_green(const ScState *sc, ScTables t, uint32_t num_part, double cur_ov_mc2) {
+// UpdateFldTbl1Kernel, space_charge_kernel.cu:39-100 (rows rs >= (nr/by)*by
+// are not written, as in the reference's grid); not needed when a field
+// surrogate's field was accepted.  Bound by the FP64 pipe: an entry costs one
+// quotient, one reciprocal root and one logarithm; the source radii's root and
+// 1 / (2 rp) are taken once a block.  1 - m with m = 4 rs rp / (b + d^2) is
+// formed as (c + d^2) / (b + d^2) where it is small, which does not cancel.
+// A block of 16 warps an SM takes consecutive entries, so that no SM waits
+// for another's last round (two blocks of 8 warps with a grid stride left
+// 13% of the rounds empty at 32 x 128).  32 x 128: 38.5 -> 26.5 us, with one adjacent
+// bunch 88 -> 57.5.
+struct Green64 {
+  double er, ez;
+};
+__device__ __forceinline__ void green64_add(Green64 &s, double rs2mrp2, double b, double c, double rsrp4, double hrp,
+                                            double d) {
+  const double d2 = d * d, cd = c + d2;
+  const double r = rsqrt(b + d2), r2 = r * r, m = rsrp4 * r2;
+  const double g = m < 0.5 ? 1.0 - m : cd * r2;
+  const double h = log(g);
+  const double ee = 1.0 + g * (0.4630106 - 0.2452740 * h + g * (0.1077857 - 0.04125321 * h));
+  const double ek = 1.38629436 - 0.5 * h + g * (0.1119697 - 0.1213486 * h + g * (0.07253230 - 0.02887472 * h));
+  const double q = ee / cd;
+  s.er += (ek - (rs2mrp2 + d2) * q) * r * hrp;
+  s.ez += d * q * r;
+}
+constexpr int kGreenThreads = 512;
+constexpr int kGreenBlocks = 152;
+__global__ void __launch_bounds__(kGreenThreads, 1) k_green(const ScState *sc, ScTables t, uint32_t num_part,
+                                                            double cur_ov_mc2) {
   if (!sc->remesh || sc->sur_accepted) return;
+  extern __shared__ double green_r[];  // rs of each source radius, then 1 / (2 rp) of each field radius (0 on axis)
   const uint32_t nr = sc->nx, nz = sc->nz;
   const uint32_t by = (512 / nz < nr) ? 512 / nz : nr;
   const uint32_t nrs = by ? (nr / by) * by : 0;
@@ -193,49 +220,34 @@ __global__ void k_green(const ScState *sc, ScTables t, uint32_t num_part, double
   const double wave_len = CLIGHT / r_freq;
   const double pl = r_beta * gm * wave_len;
   const double c1 = 5721.67 * cur_ov_mc2 / (r_freq * 1e6 * (double)num_part);
-  for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
-    uint32_t tz = e % nz;
-    uint32_t k = (e / nz) % nrs;
-    uint32_t rpi = e / (nz * nrs);
-    double rs = sqrt(0.5 * (k * k + (k + 1) * (k + 1))) * dr;
-    double zs = 0.5 * dzg;
-    double zp = (tz + 1) * dzg;
-    double rp = rpi * dr;
-    double d = zp - zs;
-    double d2 = d * d;
-    double c = (rp - rs) * (rp - rs);
-    double b = (rp + rs) * (rp + rs);
-    double rsrp = rs * rp;
-    double a = 4.0 * rsrp / (b + d2);
-    double g = 1.0 - a;
-    double h = log(g);
-    double ee = 1.0 + g * (0.4630106 - 0.2452740 * h + g * (0.1077857 - 0.04125321 * h));
-    double ek = 1.38629436 - 0.5 * h + g * (0.1119697 - 0.1213486 * h + g * (0.07253230 - 0.02887472 * h));
-    double er1 = 0.0;
-    a = sqrt(b + d2);
-    double rs2mrp2 = (rs * rs - rp * rp);
-    if (rp != 0.0) er1 = (ek - (rs2mrp2 + d2) * ee / (c + d2)) / (2.0 * rp * a);
-    double ez1 = d * ee / (a * (c + d2));
-    for (uint32_t i = 1; i <= adj; ++i) {
-      double xi = i;
-      for (int j = 0; j < 2; ++j) {
-        double d1 = d - xi * pl;
-        d2 = d1 * d1;
-        a = 4.0 * rsrp / (b + d2);
-        g = 1.0 - a;
-        h = log(g);
-        ee = 1.0 + g * (0.4630106 - 0.2452740 * h + g * (0.1077857 - 0.04125321 * h));
-        ek = 1.38629436 - 0.5 * h + g * (0.1119697 - 0.1213486 * h + g * (0.07253230 - 0.02887472 * h));
-        a = sqrt(b + d2);
-        if (rp != 0.0) er1 += (ek - (rs2mrp2 + d2) * ee / (c + d2)) / (2.0 * rp * a);
-        ez1 += d1 * ee / (a * (c + d2));
-        xi = -xi;
-      }
-    }
-    size_t cnt = (size_t)rpi * nr * nz + (size_t)k * nz + tz;
-    t.fld1[2 * cnt] = c1 * er1;
-    t.fld1[2 * cnt + 1] = c1 * ez1;
+  for (uint32_t k = threadIdx.x; k < nr; k += blockDim.x) {
+    green_r[k] = sqrt(0.5 * (k * k + (k + 1) * (k + 1))) * dr;
+    green_r[nr + k + 1] = 0.5 / ((k + 1) * dr);
+    if (k == 0) green_r[nr] = 0.0;
   }
+  __syncthreads();
+  const uint32_t share = ((total + gridDim.x - 1) / gridDim.x + 31) / 32 * 32;
+  const uint32_t e0 = blockIdx.x * share, e1 = min(total, e0 + share);
+  for (uint32_t e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
+    const uint32_t k = e % nrs, tz = (e / nrs) % nz, rpi = e / (nz * nrs);
+    const double rs = green_r[k], hrp = green_r[nr + rpi];
+    const double zs = 0.5 * dzg, zp = (tz + 1) * dzg, rp = rpi * dr, d = zp - zs;
+    const double c = (rp - rs) * (rp - rs), b = (rp + rs) * (rp + rs), rsrp4 = 4.0 * (rs * rp);
+    const double rs2mrp2 = rs * rs - rp * rp;
+    Green64 s{0.0, 0.0};
+    green64_add(s, rs2mrp2, b, c, rsrp4, hrp, d);
+    for (uint32_t i = 1; i <= adj; ++i) {
+      const double sft = i * pl;
+      green64_add(s, rs2mrp2, b, c, rsrp4, hrp, d - sft);
+      green64_add(s, rs2mrp2, b, c, rsrp4, hrp, d + sft);
+    }
+    // stored [rp][dz][rs], rs fastest, for the contraction's lanes
+    ((double2 *)t.fld1)[((size_t)rpi * nz + tz) * nr + k] = make_double2(c1 * s.er, c1 * s.ez);
+  }
+}
+void green64_launch(const ScState *sc, const ScTables &t, uint32_t nr_max, uint32_t num_part, double cur_ov_mc2,
+                    cudaStream_t st) {
+  k_green<<<kGreenBlocks, kGreenThreads, (2 * (size_t)nr_max + 1) * sizeof(double), st>>>(sc, t, num_part, cur_ov_mc2);
 }
 
 __device__ inline void dep_add(unsigned long long *h, int k, double v) {
@@ -446,12 +458,18 @@ void sc_stats(const DevBeam &b, ScState *sc, const ScTables &t, const ScKickArgs
 }
 
 // UpdateFldTbl2KernelDouble (space_charge_kernel.cu:472-568) on the FP64
-// tables: contract.cuh's ring-convolution kernel, grid and shared memory
-// sized for the largest mesh the solver takes
-void contract64(const ScState *sc, const ScTables &t, uint32_t nx_max, uint32_t nz_max, cudaStream_t st) {
+// tables: contract64.cuh's kernel where the kick's mesh is known on the host
+// and one it takes, contract.cuh's general one, sized for the largest mesh
+// the solver takes, otherwise
+void contract64(const ScState *sc, const ScTables &t, uint32_t nx_max, uint32_t nz_max, bool mesh_fixed,
+                cudaStream_t st) {
   static PerDevice configured;
-  configured.once([] { contract_configure<double>(); });
-  contract_launch<double>(sc, t, nx_max, nz_max, st);
+  configured.once([] {
+    contract_configure<double>();
+    contract64_configure();
+  });
+  if (mesh_fixed && contract64_ok(nx_max, nz_max)) contract64_launch(sc, t, nx_max, nz_max, st);
+  else contract_launch<double>(sc, t, nx_max, nz_max, st);
 }
 
 void sc_mesh(const DevBeam &b, ScState *sc, const ScTables &t, const ScKickArgs &a, PassScratch s,
@@ -462,7 +480,7 @@ void sc_mesh(const DevBeam &b, ScState *sc, const ScTables &t, const ScKickArgs 
   // field surrogate the deposit comes first, and an accepted surrogate field
   // makes the Green's table and the contraction return at once
   if (!sur) {
-    k_green<<<2 * 152, kBlock, 0, st>>>(sc, t, b.n, a.current * a.frac / b.mass);
+    green64_launch(sc, t, a.nx_max, b.n, a.current * a.frac / b.mass, st);
     note_launch();
   }
   if (a.deposit_ok) {
@@ -471,10 +489,10 @@ void sc_mesh(const DevBeam &b, ScState *sc, const ScTables &t, const ScKickArgs 
   }
   if (sur) {
     sur_solve(b, sc, t, a, *sur, st);
-    k_green<<<2 * 152, kBlock, 0, st>>>(sc, t, b.n, a.current * a.frac / b.mass);
+    green64_launch(sc, t, a.nx_max, b.n, a.current * a.frac / b.mass, st);
     note_launch();
   }
-  contract64(sc, t, a.nx_max, a.nz_max, st);
+  contract64(sc, t, a.nx_max, a.nz_max, a.mesh_fixed, st);
   note_launch();
 }
 
@@ -483,13 +501,6 @@ void sc_kick(const DevBeam &b, ScState *sc, const ScTables &t, const ScKickArgs 
     k_kick<<<grid_for(b.n), kBlock, 0, st>>>(b, sc, t, a.length, a.current, a.skip_stride);
     note_launch();
   }
-}
-
-// Green's table in FP64 for the FP32 solver too: its elliptic-integral fits
-// difference two O(1) terms into an O(r^2/d^2) far field
-void sc_green(const ScState *sc, const ScTables &t, uint32_t num_part, double cur_ov_mc2, cudaStream_t st) {
-  k_green<<<2 * 152, kBlock, 0, st>>>(sc, t, num_part, cur_ov_mc2);
-  note_launch();
 }
 
 // the limit only grows, per device (the attribute is per device)
@@ -546,8 +557,8 @@ cudaError_t sc_field_solve(ScState *sc, unsigned long long *fx, double *fld1, do
   t.bin_fx = fx;
   t.fld1 = fld1;
   t.fld2 = fld2;
-  k_green<<<2 * 152, kBlock, 0, st>>>(sc, t, (uint32_t)mesh[4], mesh[5]);
-  contract64(sc, t, nr, nz, st);
+  green64_launch(sc, t, nr, (uint32_t)mesh[4], mesh[5], st);
+  contract64(sc, t, nr, nz, true, st);
   note_launch(4);
   return cudaGetLastError();
 }
