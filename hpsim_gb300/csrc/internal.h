@@ -43,6 +43,13 @@ struct PerDevice {
   }
 };
 
+// a fork of a beam's stream: kernels on `side` between ev_fork and ev_join
+// run beside the kernels on `main` (a parallel branch of a captured graph)
+struct Fork {
+  cudaStream_t main, side;
+  cudaEvent_t ev_fork, ev_join;
+};
+
 // ---- beam reductions and small beam kernels (beam_ops.cu) -------------
 void beam_update_loss(const DevBeam &b, PassScratch s, cudaStream_t st);
 void beam_update_lloss_count(const DevBeam &b, PassScratch s, cudaStream_t st);
@@ -108,7 +115,7 @@ void sc_stats(const DevBeam &b, ScState *sc, const ScTables &t, const ScKickArgs
               cudaStream_t st);
 struct SurNet;
 void sc_mesh(const DevBeam &b, ScState *sc, const ScTables &t, const ScKickArgs &a, PassScratch s,
-             cudaStream_t st, const SurNet *sur = nullptr);
+             cudaStream_t st, const SurNet *sur = nullptr, const Fork *fork = nullptr);
 void sc_kick(const DevBeam &b, ScState *sc, const ScTables &t, const ScKickArgs &a, cudaStream_t st);
 void beam_update_stat_for_sc(const DevBeam &b, PassScratch s, cudaStream_t st);
 
@@ -152,7 +159,7 @@ int sur_build(SurNet &n, int n_layers, const int32_t *arch, int gmean_after, con
 // accepted into the field table (the FP32 one with fp32 != 0) or left to the
 // contraction
 void sur_solve(const DevBeam &b, ScState *sc, const ScTables &t, const ScKickArgs &a, const SurNet &n,
-               cudaStream_t st, int fp32 = 0);
+               cudaStream_t st, int fp32, const Fork *fork);
 int sur_read(const SurNet &n, double *accepted, double *rejected, double *residual);
 // layers on the tensor cores; whether a tensor-core layer's wait gave up
 int sur_conv_state(const SurNet &n, int *tc_layers, unsigned int *err);
@@ -237,13 +244,8 @@ void contract32(const ScState *sc, const ScTables &t, uint32_t nx_max, uint32_t 
                 cudaStream_t st);
 void sc32_stats(const DevBeam &b, ScState *sc, const ScTables &t, const ScKickArgs &a, PassScratch s,
                 cudaStream_t st);
-// a fork of a beam's stream: kernels on `side` between ev_fork and ev_join
-// run beside the kernels on `main` (a parallel branch of a captured graph)
-struct Fork {
-  cudaStream_t main, side;
-  cudaEvent_t ev_fork, ev_join;
-};
-// fork (may be null): the Green's table runs beside the deposit
+// fork (may be null): the Green's table runs beside the deposit, a field
+// surrogate's spot solve beside its network
 void sc32_mesh(const DevBeam &b, ScState *sc, const ScTables &t, const ScKickArgs &a, PassScratch s,
                cudaStream_t st, const SurNet *sur = nullptr, const Fork *fork = nullptr);
 void sc32_kick(const DevBeam &b, ScState *sc, const ScTables &t, const ScKickArgs &a, cudaStream_t st);

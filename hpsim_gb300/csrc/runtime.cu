@@ -1186,7 +1186,7 @@ void sc_apply(Ctx &c, double length, bool fused = false) {
   ScTables t = c.sc->t;
   t.ffld2 = nullptr;  // FP64 beams use fld2
   PHASE(HPS_PROF_SC_STATS, sc_stats(b->d, c.sc->d, t, a, b->scr, b->stream));
-  PHASE(HPS_PROF_SC_MESH, sc_mesh(b->d, c.sc->d, t, a, b->scr, b->stream, c.sc->sur));
+  PHASE(HPS_PROF_SC_MESH, sc_mesh(b->d, c.sc->d, t, a, b->scr, b->stream, c.sc->sur, &b->fork));
   PHASE(HPS_PROF_SC_KICK, sc_kick(b->d, c.sc->d, t, a, b->stream));
 }
 

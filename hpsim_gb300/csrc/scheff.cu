@@ -255,6 +255,84 @@ __device__ inline void dep_add(unsigned long long *h, int k, double v) {
   if (q) atomicAdd(h + k, (unsigned long long)q);
 }
 
+// What all particles of a kick share, formed once a block by one warp: the
+// independent quotients on a lane each (one FP64 quotient's latency for all of
+// them), where every thread used to form them for its one or two particles,
+// a third of these kernels' FP64 instructions.
+struct Kick64 {
+  double gmg, epsq, inv_epsq, xfac, yfac, xbar, ybar, phimc, c2, pl;
+  double dr, inv_dr, dzg, inv_dzg, hl;
+  double beta, inv_mass, c3, cbg, er_c3, ez_c3;  // the kick's alone
+  uint32_t nx, nz, adj;
+};
+// KICK: the mesh as the kick sees it (ratio-scaled); else as the deposit does
+template <bool KICK>
+__device__ __forceinline__ void kick64_consts(Kick64 &K, const DevBeam &bm, const ScState *sc, double length,
+                                              double current) {
+  __shared__ double q[10];
+  const int lane = threadIdx.x;
+  if (lane < 32) {
+    const BeamStats &st = *bm.st;
+    const double beta = sc->beta, gmg = rsqrt(1.0 - beta * beta), xs = st.st[X_SIG_GOOD], ys = st.st[Y_SIG_GOOD];
+    const double rr = KICK ? sc->ratio_r : 1.0, rz = KICK ? sc->ratio_z : 1.0;
+    const double dr = sc->dr * rr, dzg = sc->dz * gmg * rz;
+    double num = 1.0, den = 1.0;
+    switch (lane) {
+      case 0: num = xs; den = ys; break;
+      case 1: num = ys; den = xs; break;
+      case 2: num = CLIGHT; den = sc->freq; break;
+      case 3: den = dr; break;
+      case 4: den = dzg; break;
+      case 5: num = length; den = beta * gmg; break;
+      case 6: den = bm.mass; break;
+      case 7: num = 5721.67 * (current * sc->frac); den = sc->freq * 1e6 * (double)bm.n * bm.mass; break;
+      case 8: num = sc->ratio_q; den = sc->ratio_r * sc->ratio_z * sc->ratio_g * sc->ratio_g; break;
+      case 9: num = sc->ratio_q; den = sc->ratio_z * sc->ratio_z; break;
+      default: break;
+    }
+    const double v = num / den;
+    if (lane < 10) q[lane] = v;
+    __syncwarp();
+    if (lane == 0) {
+      K.gmg = gmg;
+      K.epsq = q[0];
+      K.inv_epsq = q[1];
+      K.xbar = st.st[X_AVG_GOOD];
+      K.ybar = st.st[Y_AVG_GOOD];
+      K.phimc = st.st[PHI_AVG_R];
+      K.pl = beta * gmg * q[2];
+      K.c2 = K.pl * (1.0 / TWOPI);
+      K.dr = dr;
+      K.inv_dr = q[3];
+      K.dzg = dzg;
+      K.inv_dzg = q[4];
+      K.nx = sc->nx;
+      K.nz = sc->nz;
+      K.adj = sc->adj;
+      K.hl = K.nz * 0.5 * dzg;
+      if (KICK) {
+        K.xfac = 2.0 / (q[0] + 1.0);
+        K.yfac = q[0] * K.xfac;
+        K.beta = beta;
+        K.inv_mass = q[6];
+        K.c3 = q[5];
+        K.cbg = q[7] * q[5] * PI * 0.5 * sc->num_on_mesh;
+        K.er_c3 = q[8] * q[5];
+        K.ez_c3 = q[9] * q[5];
+      }
+    }
+  }
+  __syncthreads();
+}
+
+__device__ __forceinline__ double wrap_turns64(double d) {
+  for (int guard = 0; (d > PI || d < -PI) && guard < 1000000; ++guard) {
+    if (d > 0.0) d -= TWOPI;
+    else d += TWOPI;
+  }
+  return d;
+}
+
 // DistributeParticleKernel, space_charge_kernel.cu:123-224: each block
 // deposits into its own histogram in shared memory (integer weights), then
 // adds it to the global table; integer sums make the table independent of
@@ -262,56 +340,43 @@ __device__ inline void dep_add(unsigned long long *h, int k, double v) {
 __global__ void k_deposit(DevBeam bm, ScState *sc, ScTables t) {
   if (!sc->remesh) return;
   extern __shared__ unsigned long long hist[];
+  __shared__ Kick64 K;
   const uint32_t nx = sc->nx, nz = sc->nz, nb = nx * nz;
   for (uint32_t k = threadIdx.x; k < nb; k += blockDim.x) hist[k] = 0ull;
-  __syncthreads();
-  const BeamStats &st = *bm.st;
-  const double phimc = st.st[PHI_AVG_R], xbar = st.st[X_AVG_GOOD], ybar = st.st[Y_AVG_GOOD];
-  const double epsq = st.st[X_SIG_GOOD] / st.st[Y_SIG_GOOD];
-  const double r_beta = sc->beta, r_freq = sc->freq;
-  const double gm = rsqrt(1.0 - r_beta * r_beta);
-  const double dr = sc->dr, dzg = sc->dz * gm;
-  const double wave_len = CLIGHT / r_freq;
-  const double hl = nz * 0.5 * dzg;
-  const double c2 = r_beta * gm * wave_len / TWOPI;
+  kick64_consts<false>(K, bm, sc, 0.0, 0.0);
+  const double dr = K.dr, drdr = dr * dr, inv_drdr = K.inv_dr * K.inv_dr;
   uint32_t cnt = 0;
   for (uint32_t np = blockIdx.x * blockDim.x + threadIdx.x; np < bm.n; np += gridDim.x * blockDim.x) {
     if (!(bm.loss[np] == 0u && bm.lloss[np] == 0u)) continue;
-    double x = bm.x[np], y = bm.y[np], z = bm.phi_r[np];
-    double rsq_sh = (x - xbar) * (x - xbar) / epsq + (y - ybar) * (y - ybar) * epsq;
-    int i = (int)(sqrt(rsq_sh) / dr + 1);
+    const double dx = bm.x[np] - K.xbar, dy = bm.y[np] - K.ybar;
+    const double rsq_sh = dx * dx * K.inv_epsq + dy * dy * K.epsq;
+    const int i = (int)(sqrt(rsq_sh) * K.inv_dr + 1);
     if (!(i >= 1 && (uint32_t)i <= nx)) continue;
-    double ddz = z - phimc;
-    for (int guard = 0; (ddz > PI || ddz < -PI) && guard < 1000000; ++guard) {
-      if (ddz > 0.0) ddz -= TWOPI;
-      else ddz += TWOPI;
-    }
-    z = -c2 * ddz;
-    if (!(fabs(z) < hl)) continue;
-    double zz = z + hl;
-    int jm1 = (int)(zz / dzg + 1);
+    const double z = -K.c2 * wrap_turns64(bm.phi_r[np] - K.phimc);
+    if (!(fabs(z) < K.hl)) continue;
+    const double zz = z + K.hl;
+    const int jm1 = (int)(zz * K.inv_dzg + 1);
     int i1 = i + 1;
-    double drdr = dr * dr;
     if (rsq_sh < 0.5 * drdr * (double)(i * i + (i - 1) * (i - 1))) i1 = i - 1;
     if (i1 < 1) i1 = 1;
     if (i1 > (int)nx) i1 = nx;
     int j1 = jm1 + 1;
-    if (zz < (jm1 - 1 + 0.5) * dzg) j1 = jm1 - 1;
+    if (zz < (jm1 - 1 + 0.5) * K.dzg) j1 = jm1 - 1;
     if (j1 < 1) j1 = 1;
     if (j1 > (int)nz) j1 = nz;
     if (jm1 < 1 || jm1 > (int)nz) continue;  // cannot happen for |z| < hl
     double a;
     if (i1 == i) a = 1.0;
     else {
-      double sqrtmp = sqrt(4.0 * rsq_sh / drdr - 1.0);
-      double rminsq = 0.25 * drdr * (sqrtmp - 1.0) * (sqrtmp - 1.0);
-      double rmaxsq = rminsq + sqrtmp * drdr;
-      if (i1 < i) a = (rmaxsq - (i - 1) * (i - 1) * drdr) / (rmaxsq - rminsq);
-      else a = ((i1 - 1) * (i1 - 1) * drdr - rminsq) / (rmaxsq - rminsq);
+      // radii in units of dr: rmax^2 - rmin^2 = q = sqrt(4 r^2 - 1)
+      const double q2 = 4.0 * rsq_sh * inv_drdr - 1.0, iq = rsqrt(q2), q = q2 * iq;
+      const double rmin2 = 0.25 * (q - 1.0) * (q - 1.0);
+      if (i1 < i) a = (rmin2 + q - (double)((i - 1) * (i - 1))) * iq;
+      else a = ((double)((i1 - 1) * (i1 - 1)) - rmin2) * iq;
     }
     double cc = 1.0;
-    if (j1 != jm1) cc = (zz - (j1 - 1 + 0.5) * dzg) / ((jm1 - j1) * dzg);
-    double bb = 1.0 - a, d = 1.0 - cc;
+    if (j1 != jm1) cc = (zz - (j1 - 1 + 0.5) * K.dzg) * (j1 < jm1 ? K.inv_dzg : -K.inv_dzg);
+    const double bb = 1.0 - a, d = 1.0 - cc;
     int k = (jm1 - 1) * nx + i;
     dep_add(hist, k - 1, a * cc);
     k += i1 - i;
@@ -336,61 +401,37 @@ __global__ void k_deposit(DevBeam bm, ScState *sc, ScTables t) {
 // grid-stride loop `while (indx > 0 && ...)` ends thread 0 before its first
 // particle, so particles whose index is a multiple of its launch's thread
 // count (skip_stride) are never kicked; the same set is skipped here.
+// Per particle: three roots, two reciprocals (nine quotients and three roots
+// before).  65,536 particles: kick 38 -> 20.6 us, deposit 26.7 -> 16.9.
 __global__ void k_kick(DevBeam bm, const ScState *sc, ScTables t, double length, double current,
                        uint64_t skip_stride) {
-  const uint32_t nx = sc->nx, nz = sc->nz;
-  const double r_beta = sc->beta, r_freq = sc->freq, r_mass = bm.mass;
-  const double r_current = current * sc->frac;
-  const double rr = sc->ratio_r, rz = sc->ratio_z, rq = sc->ratio_q, rg = sc->ratio_g;
-  const BeamStats &st = *bm.st;
-  const double phimc = st.st[PHI_AVG_R], xbar = st.st[X_AVG_GOOD], ybar = st.st[Y_AVG_GOOD];
-  const double epsq = st.st[X_SIG_GOOD] / st.st[Y_SIG_GOOD];
-  const double gmg = rsqrt(1.0 - r_beta * r_beta);
-  const double dr = sc->dr * rr;
-  const double dzg = sc->dz * gmg * rz;
-  const double wave_len = CLIGHT / r_freq;
-  const double hl = nz * 0.5 * dzg;
-  const double c1 = 5721.67 * r_current / (r_freq * 1e6 * (double)bm.n * r_mass);
-  const double c2 = r_beta * gmg * wave_len / TWOPI;
-  const double c3 = length / (r_beta * gmg);
-  const double xfac = 2.0 / (epsq + 1.0);
-  const double yfac = epsq * xfac;
-  const uint32_t adj = sc->adj, onm = sc->num_on_mesh;
-  const uint32_t tbl_sz = (nx + 1) * (nz + 1);
+  __shared__ Kick64 K;
+  kick64_consts<true>(K, bm, sc, length, current);
+  const uint32_t nx = K.nx, nz = K.nz, tbl_sz = (nx + 1) * (nz + 1);
   const double *fld = t.fld2;
   for (uint32_t indx = blockIdx.x * blockDim.x + threadIdx.x; indx < bm.n; indx += gridDim.x * blockDim.x) {
     if (indx % skip_stride == 0) continue;
     if (!(bm.loss[indx] == 0u && bm.lloss[indx] == 0u)) continue;
-    double x = bm.x[indx], y = bm.y[indx], xp = bm.xp[indx], yp = bm.yp[indx];
-    double phi = bm.phi_r[indx], w = bm.w[indx];
+    const double x = bm.x[indx], y = bm.y[indx], phi = bm.phi_r[indx], w = bm.w[indx];
+    const double g = w * K.inv_mass, gm = g + 1.0, bgz = sqrt(g * (g + 2.0));
+    double bgx = bgz * bm.xp[indx], bgy = bgz * bm.yp[indx];
+    double bgzstar = K.gmg * (bgz - K.beta * gm);
+    const double xxbar = x - K.xbar, yybar = y - K.ybar;
+    const double r2 = xxbar * xxbar * K.inv_epsq + yybar * yybar * K.epsq;
+    const double inv_r = r2 == 0.0 ? 1.0e8 : rsqrt(r2), r = r2 == 0.0 ? 1.0e-8 : r2 * inv_r;
+    const double xovr = xxbar * K.xfac * inv_r, yovr = yybar * K.yfac * inv_r;
+    double z = -K.c2 * wrap_turns64(phi - K.phimc);
     double cbgr, cbgzs;
-    double gm = w / r_mass + 1.0;
-    double bgz = sqrt((gm - 1.0) * (gm + 1.0));
-    double bgx = bgz * xp;
-    double bgy = bgz * yp;
-    double bgzstar = gmg * (bgz - r_beta * gm);
-    double xxbar = x - xbar, yybar = y - ybar;
-    double r = sqrt(xxbar * xxbar / epsq + yybar * yybar * epsq);
-    if (r == 0.0) r = 1.0e-8;
-    double xovr = xxbar * xfac / r;
-    double yovr = yybar * yfac / r;
-    double ddz = phi - phimc;
-    for (int guard = 0; (ddz > PI || ddz < -PI) && guard < 1000000; ++guard) {
-      if (ddz > 0.0) ddz -= TWOPI;
-      else ddz += TWOPI;
-    }
-    double z = -c2 * ddz;
-    if (r > nx * dr || fabs(z) > hl) {
-      z = -c2 * (phi - phimc);
+    if (r > nx * K.dr || fabs(z) > K.hl) {
+      z = -K.c2 * (phi - K.phimc);
       double d = sqrt(z * z + r * r);
       double invd3 = 1.0 / (d * d * d);
       double rod3 = r * invd3;
       double zod3 = z * invd3;
-      double pl = r_beta * gmg * wave_len;
-      for (uint32_t nb = 1; nb <= adj; ++nb) {
+      for (uint32_t nb = 1; nb <= K.adj; ++nb) {
         int xi = (int)nb;
         for (int lr = 1; lr <= 2; ++lr) {
-          double sft = z + xi * pl;
+          double sft = z + xi * K.pl;
           d = sqrt(sft * sft + r * r);
           invd3 = 1.0 / (d * d * d);
           rod3 += r * invd3;
@@ -398,38 +439,35 @@ __global__ void k_kick(DevBeam bm, const ScState *sc, ScTables t, double length,
           xi = -xi;
         }
       }
-      double cbgcoef = c1 * c3 * PI * 0.5 * onm;
-      cbgr = cbgcoef * rod3;
-      cbgzs = cbgcoef * zod3;
+      cbgr = K.cbg * rod3;
+      cbgzs = K.cbg * zod3;
     } else {
-      uint32_t i = 1 + (int)(r / dr);
-      double a = r / dr - (i - 1.0);
-      double bb = 1.0 - a;
-      uint32_t j = 1 + (int)((z + hl) / dzg);
-      double c = (z + hl) / dzg - (j - 1.0);
-      double d = 1.0 - c;
+      const double ri = r * K.inv_dr, zi = (z + K.hl) * K.inv_dzg;
+      const uint32_t i = 1 + (int)ri;
+      const double a = ri - (i - 1.0), bb = 1.0 - a;
+      const uint32_t j = 1 + (int)zi;
+      const double c = zi - (j - 1.0), d = 1.0 - c;
       uint32_t l = (j - 1) * (nx + 1) + i;
       uint32_t m = l + (nx + 1);
       if (m >= tbl_sz) m = tbl_sz - 1;
       // l leaves the table only for r == nx*dr with z == hl, or NaN input
       if (l >= tbl_sz || l < 1) l = tbl_sz - 1;
       if (m < 1) m = 1;
-      double er_ratio = rq / (rr * rz * rg * rg);
-      double ez_ratio = rq / (rz * rz);
-      cbgr = er_ratio * c3 * (d * (a * fld[2 * l] + bb * fld[2 * (l - 1)]) + c * (a * fld[2 * m] + bb * fld[2 * (m - 1)]));
-      cbgzs = ez_ratio * c3 * (d * (a * fld[2 * l + 1] + bb * fld[2 * (l - 1) + 1]) +
-                               c * (a * fld[2 * m + 1] + bb * fld[2 * (m - 1) + 1]));
+      cbgr = K.er_c3 * (d * (a * fld[2 * l] + bb * fld[2 * (l - 1)]) + c * (a * fld[2 * m] + bb * fld[2 * (m - 1)]));
+      cbgzs = K.ez_c3 * (d * (a * fld[2 * l + 1] + bb * fld[2 * (l - 1) + 1]) +
+                         c * (a * fld[2 * m + 1] + bb * fld[2 * (m - 1) + 1]));
     }
     bgx += cbgr * xovr;
     bgy += cbgr * yovr;
     bgzstar += cbgzs;
-    double gstar = 1.0 + 0.5 * bgzstar * bgzstar;
-    double bgzf = gmg * (bgzstar + r_beta * gstar);
+    const double gstar = 1.0 + 0.5 * bgzstar * bgzstar;
+    const double bgzf = K.gmg * (bgzstar + K.beta * gstar);
     if (bgzf <= 0.0) bm.loss[indx] = 9999u;
     else {
-      bm.xp[indx] = bgx / bgzf;
-      bm.yp[indx] = bgy / bgzf;
-      bm.w[indx] *= 1.0 + (gm + 1.0) * (bgzf - bgz) / (gm * bgz);
+      const double inv_f = 1.0 / bgzf;
+      bm.xp[indx] = bgx * inv_f;
+      bm.yp[indx] = bgy * inv_f;
+      bm.w[indx] = w * (1.0 + (gm + 1.0) * (bgzf - bgz) / (gm * bgz));
     }
   }
 }
@@ -473,7 +511,7 @@ void contract64(const ScState *sc, const ScTables &t, uint32_t nx_max, uint32_t 
 }
 
 void sc_mesh(const DevBeam &b, ScState *sc, const ScTables &t, const ScKickArgs &a, PassScratch s,
-             cudaStream_t st, const SurNet *sur) {
+             cudaStream_t st, const SurNet *sur, const Fork *fork) {
   launch_pass(OpAdjMesh{b, sc}, b.n, s, st);
   note_launch();
   // mesh kernels are sized for the largest mesh this solver can take; with a
@@ -488,7 +526,7 @@ void sc_mesh(const DevBeam &b, ScState *sc, const ScTables &t, const ScKickArgs 
     note_launch();
   }
   if (sur) {
-    sur_solve(b, sc, t, a, *sur, st);
+    sur_solve(b, sc, t, a, *sur, st, 0, fork);
     green64_launch(sc, t, a.nx_max, b.n, a.current * a.frac / b.mass, st);
     note_launch();
   }

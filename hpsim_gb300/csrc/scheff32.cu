@@ -834,7 +834,7 @@ void sc32_mesh(const DevBeam &b, ScState *sc, const ScTables &t, const ScKickArg
       launch_k(k32_green_deposit, dim3(ndep), dim3(dthreads), q.smem ? hb : 0, st, b, sc, u, q, ndep, 0u);
       note_launch();
     }
-    sur_solve(b, sc, u, a, *sur, st, 1);
+    sur_solve(b, sc, u, a, *sur, st, 1, fork);
     k32_green<<<ngreen, kBlock, 0, st>>>(sc, u);
     note_launch();
   } else if (fork && ndep) {

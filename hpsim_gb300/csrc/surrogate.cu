@@ -5,7 +5,8 @@
 //   k_sur_input   charge / total and log cell aspect as the network input
 //                 (BF16), the field scale, the acceptance flag cleared;
 //   the network   its 3x3 convolution layers (nn.cu) with the skip additions
-//                 fused and the plane-mean broadcast, on a batch of one;
+//                 fused and the plane-mean broadcast, on a batch of one, and
+//                 beside it on the beam's side stream
 //   k_sur_spot    the plain method's field (the sum over every bin of charge
 //                 times the Green's function, evaluated in FP32) at the
 //                 mesh's last row and column, which the network does not
@@ -13,7 +14,7 @@
 //   k_sur_fit     the network's E_r and E_z corrected by gains (constant
 //                 plus linear across the mesh) fitted at the sample points,
 //                 and their relative residual there against the tolerance;
-//   k_sur_write   when accepted, the field table gets the corrected interior
+//                 when accepted, the field table gets the corrected interior
 //                 and the spot-solved boundary, and the solver state says
 //                 so: the FP64 Green's table and the contraction then return
 //                 at once.
@@ -28,13 +29,14 @@
 #include "../../include/hpsim_gb300.h"
 #include "green32.cuh"
 #include "internal.h"
+#include "reduce.cuh"
 
 namespace hps {
 
 namespace {
 
 constexpr int kSurBlock = 256;
-constexpr int kFitBlock = 64;
+constexpr int kFitBlock = 128;  // two warps for each field component
 constexpr int kInBlocks = 16;
 
 struct SurDev {
@@ -43,7 +45,6 @@ struct SurDev {
   double scale;        // field = network output * scale
   double c1, dzg, dr;  // Green's-table scale, bunch-frame cell length, radial cell size
   double residual;     // relative residual of the last check
-  double cf[6];        // field = output * (cf0 + cf1 z + cf2 r) for E_r, cf3.. for E_z
   uint32_t n_accepted, n_rejected;
   unsigned int conv_err;  // a tensor-core layer's bounded wait gave up
 };
@@ -80,12 +81,13 @@ __device__ inline void spot_point(uint32_t k, uint32_t nr, uint32_t nz, uint32_t
 // kInBlocks blocks: each sums the whole charge table (a few microseconds of
 // loads, not worth a second launch) and normalises its share; block 0
 // records the kick's scalars
+// c1: the Green's-table scale of an FP64 beam
 // fp32: the kick of an FP32 beam (mesh and Green's-table scale from the FP32
 // kick constants, as the FP32 Green's table takes them)
 __global__ void __launch_bounds__(kSurBlock) k_sur_input(ScState *sc, ScTables t, SurDev *sd, __nv_bfloat16 *x,
                                                          uint32_t nr, uint32_t nz, double out_scale,
-                                                         uint32_t num_part, double cur_ov_mc2, int fp32) {
-  __shared__ unsigned long long red[kSurBlock];
+                                                         double c1, int fp32) {
+  __shared__ unsigned long long red[kSurBlock / 32];
   __shared__ int go;
   __shared__ float qs;
   __shared__ __nv_bfloat16 la;
@@ -103,43 +105,49 @@ __global__ void __launch_bounds__(kSurBlock) k_sur_input(ScState *sc, ScTables t
   const uint32_t nb = nr * nz;
   unsigned long long a = 0;
   for (uint32_t k = threadIdx.x; k < nb; k += blockDim.x) a += t.bin_fx[k];
-  red[threadIdx.x] = a;
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x / 32] = a;
   __syncthreads();
-  for (int off = blockDim.x / 2; off > 0; off >>= 1) {
-    if (threadIdx.x < off) red[threadIdx.x] += red[threadIdx.x + off];
-    __syncthreads();
+  if (threadIdx.x % 32 == 0) {  // every warp's first lane has the sum
+    a = 0;
+    for (int w = 0; w < kSurBlock / 32; ++w) a += red[w];
   }
-  if (threadIdx.x == 0) {
-    if (fp32) {
+  __syncthreads();
+  if (threadIdx.x == 0) red[0] = a;
+  // the network's inputs are BF16 and FP32 numbers: FP32 arithmetic (in FP64 a
+  // dependent quotient costs a third of a microsecond, a logarithm one); the
+  // field's scale stays FP64
+  if (!fp32 && threadIdx.x == 0) {
+    const float b2 = (float)sc->beta * (float)sc->beta;
+    qs = a ? (float)nb / (float)(long long)a : 0.0f;
+    la = __float2bfloat16_rn(logf((float)sc->dz * rsqrtf(1.0f - b2) / (float)sc->dr));
+  }
+  if (!fp32 && threadIdx.x == 32 && blockIdx.x == 0) {
+    const double dzg = sc->dz * rsqrt(1.0 - sc->beta * sc->beta), total = (double)(long long)a * kBinInvScale;
+    sd->active = total > 0.0;
+    sd->total = total;
+    sd->scale = c1 * total / (out_scale * sc->dr * dzg);
+    sd->c1 = c1;
+    sd->dzg = dzg;
+    sd->dr = sc->dr;
+  }
+  if (fp32 && threadIdx.x == 0) {
+    {
       // FP32 arithmetic throughout (an FP64 divide costs about a microsecond)
       const Sc32Consts &k = *t.c32;
-      const float dr = k.dr0, dzg = k.dzg0, c1 = k.green_c1;
+      const float dr = k.dr0, dzg = k.dzg0, c1f = k.green_c1;
       if (blockIdx.x == 0) {
         const float total = (float)(long long)red[0] * 1.4551915228366852e-11f;  // 2^-36
         sd->active = total > 0.0f;
         sd->total = total;
-        sd->scale = c1 * total / ((float)out_scale * dr * dzg);
-        sd->c1 = c1;
+        sd->scale = c1f * total / ((float)out_scale * dr * dzg);
+        sd->c1 = c1f;
         sd->dzg = dzg;
         sd->dr = dr;
       }
       qs = red[0] ? (float)nb / (float)(long long)red[0] : 0.0f;
       la = __float2bfloat16_rn(logf(dzg / dr));
-    } else {
-      const double dzg = sc->dz * rsqrt(1.0 - sc->beta * sc->beta);
-      if (blockIdx.x == 0) {
-        const double total = (double)(long long)red[0] * kBinInvScale;
-        const double c1 = 5721.67 * cur_ov_mc2 / (sc->freq * 1e6 * (double)num_part);
-        sd->active = total > 0.0;
-        sd->total = total;
-        sd->scale = c1 * total / (out_scale * sc->dr * dzg);
-        sd->c1 = c1;
-        sd->dzg = dzg;
-        sd->dr = sc->dr;
-      }
-      // charge / total * nb in bin units: the fixed-point integers times nb / sum
-      qs = red[0] ? (float)((double)nb / (double)(long long)red[0]) : 0.0f;
-      la = __float2bfloat16_rn((float)log(dzg / sc->dr));
     }
   }
   __syncthreads();
@@ -190,28 +198,6 @@ __global__ void __launch_bounds__(kSurBlock) k_sur_spot(const ScState *sc, const
   if (threadIdx.x == 0) spot[blockIdx.x] = make_double2(sd->c1 * rx[0], sd->c1 * rz[0]);
 }
 
-// each v[j] summed over the block -- a fixed shuffle tree per warp, then the
-// warps in order -- and returned to every thread in v; red holds K values
-// per warp
-template <int K>
-__device__ inline void block_sum(double *red, double (&v)[K]) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-#pragma unroll
-  for (int j = 0; j < K; ++j)
-    for (int off = 16; off > 0; off >>= 1) v[j] += __shfl_down_sync(0xffffffffu, v[j], off);
-  if (lane == 0)
-#pragma unroll
-    for (int j = 0; j < K; ++j) red[warp * K + j] = v[j];
-  __syncthreads();
-#pragma unroll
-  for (int j = 0; j < K; ++j) {
-    double a = red[j];
-    for (int w = 1; w < nw; ++w) a += red[w * K + j];
-    v[j] = a;
-  }
-  __syncthreads();
-}
-
 // the solution of the symmetric 3x3 system m c = y (m packed as m00 m01 m02
 // m11 m12 m22) by Cramer's rule; false when m is numerically singular
 __device__ inline bool solve3(const double *m, const double *y, double *c) {
@@ -237,88 +223,98 @@ __device__ inline float rhat(uint32_t rp, uint32_t nr) { return ((float)rp + 0.5
 // spot-solved values (a global amplitude error and gains varying linearly
 // across the mesh are removed; a singular fit keeps the amplitude factor
 // alone).  The relative residual of the corrected field at the samples
-// decides; the coefficients and the decision go to the solver state.
-__global__ void __launch_bounds__(kFitBlock) k_sur_fit(ScState *sc, SurDev *sd, const __nv_bfloat16 *out,
+// decides; block 0 leaves the decision in the solver state.  Every block takes
+// the same fit, and when the field is accepted writes its share of it into the
+// field table (the FP32 table of an FP32 beam): the corrected network field
+// inside, the spot-solved values on the last row and column.
+__global__ void __launch_bounds__(kFitBlock) k_sur_fit(ScState *sc, SurDev *sd, ScTables t, const __nv_bfloat16 *out,
                                                        const double2 *spot, uint32_t nr, uint32_t nz,
-                                                       uint32_t n_samples, double tol) {
+                                                       uint32_t n_samples, double tol, int fp32) {
   if (!sd->active) return;
-  __shared__ double red[18 * (kFitBlock / 32)];
+  constexpr int kHalf = kFitBlock / 2, kWarps = kHalf / 32;
+  __shared__ double red[2][9 * kWarps], sums[2][9], cf[2][3];
+  __shared__ int accept;
   const double scale = sd->scale;
   const uint32_t nb = nr * nz, base = nr + 1 + nz;
-  // per component: the normal matrix (6) and right-hand side (3)
-  double fit[18];
+  // a half of the block per component; the normal matrix (6) and right-hand
+  // side (3): the lanes' sums, then a thread per sum over the warps
+  const int comp = threadIdx.x / kHalf, ht = threadIdx.x % kHalf, lane = threadIdx.x & 31, hw = ht / 32;
+  double f[9];
 #pragma unroll
-  for (int j = 0; j < 18; ++j) fit[j] = 0.0;
-  for (uint32_t k = threadIdx.x; k < n_samples; k += blockDim.x) {
+  for (int j = 0; j < 9; ++j) f[j] = 0.0;
+  for (uint32_t k = ht; k < n_samples; k += kHalf) {
     uint32_t zp, rp;
     spot_point(base + k, nr, nz, sc->n_solves, zp, rp);
     const double2 e = spot[base + k];
-    const double zh = zhat(zp, nz), rh = rhat(rp, nr);
-#pragma unroll
-    for (int comp = 0; comp < 2; ++comp) {
-      const double en = (double)__bfloat162float(out[comp * nb + zp * nr + rp]) * scale;
-      const double bs[3] = {en, en * zh, en * rh};
-      double *f = fit + 9 * comp;
-      f[0] += bs[0] * bs[0]; f[1] += bs[0] * bs[1]; f[2] += bs[0] * bs[2];
-      f[3] += bs[1] * bs[1]; f[4] += bs[1] * bs[2]; f[5] += bs[2] * bs[2];
-      const double ex = comp ? e.y : e.x;
-      f[6] += bs[0] * ex; f[7] += bs[1] * ex; f[8] += bs[2] * ex;
-    }
+    const double zh = zhat(zp, nz), rh = rhat(rp, nr), ex = comp ? e.y : e.x;
+    const double en = (double)__bfloat162float(out[comp * nb + zp * nr + rp]) * scale;
+    const double b1 = en * zh, b2 = en * rh;
+    f[0] += en * en; f[1] += en * b1; f[2] += en * b2;
+    f[3] += b1 * b1; f[4] += b1 * b2; f[5] += b2 * b2;
+    f[6] += en * ex; f[7] += b1 * ex; f[8] += b2 * ex;
   }
-  block_sum(red, fit);
-  double cf[2][3];
-#pragma unroll
-  for (int comp = 0; comp < 2; ++comp) {
-    const double *f = fit + 9 * comp;
-    if (!solve3(f, f + 6, cf[comp])) {
-      cf[comp][0] = f[0] > 0.0 ? f[6] / f[0] : 1.0;
+  int slot;
+  double total;
+  if (warp_fold<SumComb>(f, lane, slot, total)) red[comp][hw * 9 + slot] = total;
+  __syncthreads();
+  if (ht < 9) {
+    double a = red[comp][ht];
+    for (int w = 1; w < kWarps; ++w) a += red[comp][w * 9 + ht];
+    sums[comp][ht] = a;
+  }
+  __syncthreads();
+  if (ht == 0) {
+    const double *m = sums[comp];
+    if (!solve3(m, m + 6, cf[comp])) {
+      cf[comp][0] = m[0] > 0.0 ? m[6] / m[0] : 1.0;
       cf[comp][1] = cf[comp][2] = 0.0;
     }
   }
+  __syncthreads();
   double r[2] = {0.0, 0.0};  // residual, reference
-  for (uint32_t k = threadIdx.x; k < n_samples; k += blockDim.x) {
+  for (uint32_t k = ht; k < n_samples; k += kHalf) {
     uint32_t zp, rp;
     spot_point(base + k, nr, nz, sc->n_solves, zp, rp);
     const double2 e = spot[base + k];
-    const double zh = zhat(zp, nz), rh = rhat(rp, nr);
-    const double er = (double)__bfloat162float(out[zp * nr + rp]) * scale *
-                      (cf[0][0] + cf[0][1] * zh + cf[0][2] * rh);
-    const double ez = (double)__bfloat162float(out[nb + zp * nr + rp]) * scale *
-                      (cf[1][0] + cf[1][1] * zh + cf[1][2] * rh);
-    r[0] += (er - e.x) * (er - e.x) + (ez - e.y) * (ez - e.y);
-    r[1] += e.x * e.x + e.y * e.y;
+    const double ex = comp ? e.y : e.x;
+    const double d = (double)__bfloat162float(out[comp * nb + zp * nr + rp]) * scale *
+                         (cf[comp][0] + cf[comp][1] * zhat(zp, nz) + cf[comp][2] * rhat(rp, nr)) - ex;
+    r[0] += d * d;
+    r[1] += ex * ex;
   }
-  block_sum(red, r);
-  if (threadIdx.x != 0) return;
-  // the ratio in FP32 (the test needs a few digits; FP64 divide and square
-  // root take microseconds on this GPU)
-  const bool f32 = r[1] > 1e-30 && r[1] < 1e30 && r[0] < 1e30;
-  const double res = r[1] > 0.0 ? (f32 ? (double)sqrtf((float)r[0] / (float)r[1]) : sqrt(r[0] / r[1]))
-                                 : (r[0] > 0.0 ? 1.0 : 0.0);
-  const bool ok = res <= tol;
-  sd->residual = res;
-  if (ok) sd->n_accepted += 1;
-  else sd->n_rejected += 1;
-  for (int j = 0; j < 6; ++j) sd->cf[j] = scale * cf[j / 3][j % 3];
-  sc->sur_accepted = ok;
-}
-
-// an accepted field into the field table (the FP32 table of an FP32 beam):
-// the corrected network field inside, the spot-solved values on the last row
-// and column
-__global__ void __launch_bounds__(kSurBlock) k_sur_write(const ScState *sc, ScTables t, const SurDev *sd,
-                                                         const __nv_bfloat16 *out, const double2 *spot, uint32_t nr,
-                                                         uint32_t nz, int fp32) {
-  if (!sd->active || !sc->sur_accepted) return;
-  const uint32_t nrow = nr + 1, nb = nr * nz;
+  if (warp_fold<SumComb>(r, lane, slot, total)) red[0][2 * (threadIdx.x / 32) + slot] = total;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    r[0] = r[1] = 0.0;
+    for (int w = 0; w < kFitBlock / 32; ++w) {
+      r[0] += red[0][2 * w];
+      r[1] += red[0][2 * w + 1];
+    }
+    // the ratio in FP32 (the test needs a few digits; FP64 divide and square
+    // root take microseconds on this GPU)
+    const bool f32 = r[1] > 1e-30 && r[1] < 1e30 && r[0] < 1e30;
+    const double res = r[1] > 0.0 ? (f32 ? (double)sqrtf((float)r[0] / (float)r[1]) : sqrt(r[0] / r[1]))
+                                   : (r[0] > 0.0 ? 1.0 : 0.0);
+    accept = res <= tol;
+    for (int j = 0; j < 6; ++j) cf[j / 3][j % 3] *= scale;
+    if (blockIdx.x == 0) {
+      sd->residual = res;
+      if (accept) sd->n_accepted += 1;
+      else sd->n_rejected += 1;
+      sc->sur_accepted = accept;
+    }
+  }
+  __syncthreads();
+  if (!accept) return;
+  const uint32_t nrow = nr + 1;
   const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= (nz + 1) * nrow) return;
   const uint32_t zp = p / nrow, rp = p % nrow;
   double2 e;
   if (zp < nz && rp < nr) {
     const double zh = zhat(zp, nz), rh = rhat(rp, nr);
-    e.x = (double)__bfloat162float(out[zp * nr + rp]) * (sd->cf[0] + sd->cf[1] * zh + sd->cf[2] * rh);
-    e.y = (double)__bfloat162float(out[nb + zp * nr + rp]) * (sd->cf[3] + sd->cf[4] * zh + sd->cf[5] * rh);
+    e.x = (double)__bfloat162float(out[zp * nr + rp]) * (cf[0][0] + cf[0][1] * zh + cf[0][2] * rh);
+    e.y = (double)__bfloat162float(out[nb + zp * nr + rp]) * (cf[1][0] + cf[1][1] * zh + cf[1][2] * rh);
   } else {
     e = spot[zp == nz ? rp : nr + 1 + zp];
   }
@@ -339,10 +335,19 @@ SurNet::~SurNet() {
 }
 
 void sur_solve(const DevBeam &bm, ScState *sc, const ScTables &t, const ScKickArgs &a, const SurNet &n,
-               cudaStream_t st, int fp32) {
+               cudaStream_t st, int fp32, const Fork *fork) {
   SurDev *sd = (SurDev *)n.d;
-  k_sur_input<<<kInBlocks, kSurBlock, 0, st>>>(sc, t, sd, (__nv_bfloat16 *)n.x, n.nr, n.nz, n.out_scale, bm.n,
-                                               a.current * a.frac / bm.mass, fp32);
+  k_sur_input<<<kInBlocks, kSurBlock, 0, st>>>(sc, t, sd, (__nv_bfloat16 *)n.x, n.nr, n.nz, n.out_scale,
+                                               5721.67 * (a.current * a.frac / bm.mass) / (a.freq * 1e6 * (double)bm.n), fp32);
+  // the spot solve beside the network: both need the input's scalars only
+  const uint32_t npts = n.nr + 1 + n.nz + n.n_samples;
+  cudaStream_t side = fork ? fork->side : st;
+  if (fork) {
+    cudaEventRecord(fork->ev_fork, st);
+    cudaStreamWaitEvent(side, fork->ev_fork, 0);
+  }
+  k_sur_spot<<<npts, kSurBlock, 0, side>>>(sc, t, sd, (double2 *)n.spot, n.nr, n.nz);
+  if (fork) cudaEventRecord(fork->ev_join, side);
   const void *cur = n.x;
   for (size_t l = 0; l < n.arch.size(); ++l) {
     const int32_t *dims = n.dims.data() + 7 * l;
@@ -354,14 +359,12 @@ void sur_solve(const DevBeam &bm, ScState *sc, const ScTables &t, const ScKickAr
     if ((int)l == n.gmean_after) nn_gmean_forward(n.act[l], dims[2], n.hw[l], st);
     cur = n.act[l];
   }
-  const uint32_t npts = n.nr + 1 + n.nz + n.n_samples;
-  k_sur_spot<<<npts, kSurBlock, 0, st>>>(sc, t, sd, (double2 *)n.spot, n.nr, n.nz);
+  if (fork) cudaStreamWaitEvent(st, fork->ev_join, 0);
   const __nv_bfloat16 *out = (const __nv_bfloat16 *)n.act.back();
-  k_sur_fit<<<1, kFitBlock, 0, st>>>(sc, sd, out, (const double2 *)n.spot, n.nr, n.nz, n.n_samples, n.tol);
   const uint32_t nf = (n.nz + 1) * (n.nr + 1);
-  k_sur_write<<<(nf + kSurBlock - 1) / kSurBlock, kSurBlock, 0, st>>>(sc, t, sd, out, (const double2 *)n.spot,
-                                                                      n.nr, n.nz, fp32);
-  note_launch(4);
+  k_sur_fit<<<(nf + kFitBlock - 1) / kFitBlock, kFitBlock, 0, st>>>(sc, sd, t, out, (const double2 *)n.spot, n.nr, n.nz,
+                                                                    n.n_samples, n.tol, fp32);
+  note_launch(3);
 }
 
 int sur_build(SurNet &n, int n_layers, const int32_t *arch, int gmean_after, const int32_t *skip,
