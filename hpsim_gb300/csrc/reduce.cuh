@@ -36,23 +36,6 @@ struct MaxComb {  // MaxR2PhiReduceKernel starts from 0 (beam_kernel.cu:809-810)
   __device__ static float comb(float a, float b) { return a < b ? b : a; }
 };
 
-// a sum as a float and the float of its rounding errors (two-sum, Knuth)
-struct Pair2 {
-  float x, e;
-};
-__device__ __forceinline__ Pair2 shfl_xor_any(Pair2 v, int off) {
-  return {__shfl_xor_sync(0xffffffffu, v.x, off), __shfl_xor_sync(0xffffffffu, v.e, off)};
-}
-template <class T>
-__device__ __forceinline__ T shfl_xor_any(T v, int off) { return __shfl_xor_sync(0xffffffffu, v, off); }
-struct PairSum {
-  __device__ static Pair2 ident() { return {0.0f, 0.0f}; }
-  __device__ static Pair2 comb(Pair2 a, Pair2 b) {
-    const float s = a.x + b.x, bb = s - a.x;
-    return {s, ((a.x - (s - bb)) + (b.x - bb)) + (a.e + b.e)};
-  }
-};
-
 // Totals over a warp of K accumulators a lane, K <= 32, by folding: a step
 // halves the lanes' distance and the accumulators a lane still carries (it
 // sends one half to its partner and keeps the other), so K sums cost about
@@ -72,13 +55,13 @@ __device__ __forceinline__ bool warp_fold(const T (&a)[K], int lane, int &slot, 
 #pragma unroll
     for (int k = 0; k < cnt; ++k) {
       const T keep = hi ? v[k + cnt] : v[k], send = hi ? v[k] : v[k + cnt];
-      v[k] = C::comb(keep, shfl_xor_any(send, off));
+      v[k] = C::comb(keep, __shfl_xor_sync(0xffffffffu, send, off));
     }
     if (hi) base += cnt;
   }
   T x = v[0];
 #pragma unroll
-  for (int o = 16 / P; o > 0; o /= 2) x = C::comb(x, shfl_xor_any(x, o));
+  for (int o = 16 / P; o > 0; o /= 2) x = C::comb(x, __shfl_xor_sync(0xffffffffu, x, o));
   slot = base;
   total = x;
   return (lane & (32 / P - 1)) == 0 && base < K;
@@ -390,18 +373,12 @@ __device__ __forceinline__ void pass_body_f(const Op &op, uint32_t n, PassScratc
     }
   } else {
     __shared__ double sm[combine_rows<K>()][K];
-    if constexpr (std::is_same_v<C, SumComb>) {
-      // pairs (sum, rounding errors): an emittance is a difference of products
-      // of these sums, which a correlated beam amplifies a hundredfold
-      Pair2 v[K], t;
 #pragma unroll
-      for (int k = 0; k < K; ++k) v[k] = {acc[k], 0.0f};
-      int slot;
-      if (warp_fold<PairSum>(v, lane, slot, t)) sm[warp][slot] = (double)t.x + (double)t.e;
-    } else {
-      int slot;
-      float v;
-      if (warp_fold<C>(acc, lane, slot, v)) sm[warp][slot] = (double)v;
+    for (int k = 0; k < K; ++k) {
+      float v = acc[k];
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) v = C::comb(v, __shfl_down_sync(0xffffffffu, v, off));
+      if (lane == 0) sm[warp][k] = (double)v;
     }
     __syncthreads();
     if (threadIdx.x < K) {
@@ -468,10 +445,12 @@ inline void launch_pass_f_grid(const Op &op, uint32_t n, PassScratch scr, cudaSt
 // the SMs, a particle a thread up to one block on each; beyond that its blocks
 // hold four a thread as the others' do (more blocks make a lone beam no
 // faster and cost beams that share the SMs their reductions: a scan of 32
-// beams 24.6 -> 26.3 ms with a particle a thread throughout).
+// beams 24.6 -> 26.3 ms with a particle a thread throughout).  Up to 1,024
+// particles one block without a grid-wide sum is as fast (558 against 552 us
+// for eight kicks).
 inline int pass_blocks_f(uint32_t n, int per_sm = 2, int batch = kPassBatch) {
   uint32_t b = (uint32_t)(((uint64_t)n + kPassBatch * kBlock - 1) / (kPassBatch * kBlock));
-  if (batch == 1) b = std::max(b, std::min<uint32_t>((uint32_t)(((uint64_t)n + kBlock - 1) / kBlock), 152u));
+  if (batch == 1 && n > 4 * kBlock) b = std::max(b, std::min<uint32_t>((uint32_t)(((uint64_t)n + kBlock - 1) / kBlock), 152u));
   if (b < 1) b = 1;
   const uint32_t cap = std::min<uint32_t>((uint32_t)per_sm * 152u, (uint32_t)kMaxPassBlocks);
   if (b > cap) b = cap;
