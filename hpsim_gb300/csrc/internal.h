@@ -236,6 +236,8 @@ void beam32_to_double(const DevBeam &b, int coord, double *out, cudaStream_t st)
 void beam32_update_stat_for_sc(const DevBeam &b, PassScratch s, cudaStream_t st);
 
 void sc32_configure();
+// deposit blocks per SM on a mesh of nr x nz
+uint32_t sc32_deposit_per_sm(uint32_t nr, uint32_t nz);
 // the tensor-core contraction (contract_tc.cuh): meshes it takes, and the
 // bytes of its folded split-BF16 Green's table and of its partial fields
 bool sc32_tc_mesh(uint32_t nr, uint32_t nz);

@@ -153,7 +153,7 @@ struct hps_sim_s {
   double last_ms = 0.0;
   // launch shapes of the FP32 kernels (hps_sim_autotune picks them)
   uint32_t sweep_cap = 0;   // particle sweeps: blocks per SM (0: all the SM holds)
-  uint32_t dep_per_sm = 3;  // deposit: blocks per SM
+  uint32_t dep_per_sm = 0;  // deposit: blocks per SM (0: by the mesh)
   uint32_t dep_agg = 0;     // deposit: warp-aggregated histogram adds
   uint32_t dep_threads = 256;  // deposit: threads per block
 };
@@ -1098,6 +1098,12 @@ int T(hps_beamline_t bl, int64_t i) {
   return (i >= 0 && i < (int64_t)bl->types.size()) ? bl->types[i] : 0;
 }
 
+// deposit blocks per SM: the simulator's choice, else by the mesh
+uint32_t deposit_per_sm(hps_sim_t s) {
+  if (s->dep_per_sm) return s->dep_per_sm;
+  return s->sc ? sc32_deposit_per_sm(s->sc->nx_max, s->sc->nz_max) : 3u;
+}
+
 // the arguments of one SCHEFF kick of the given length
 ScKickArgs kick_args(Ctx &c, double length) {
   hps_beam_t b = c.b;
@@ -1114,7 +1120,7 @@ ScKickArgs kick_args(Ctx &c, double length) {
   a.nz_max = c.sc->nz_max;
   a.adj_possible = c.sc->adj_bunch != 0;
   a.mesh_fixed = c.sc->mesh_w == 0.0 && c.sc->nx == c.sc->nx_max && c.sc->nz == c.sc->nz_max;
-  a.dep_per_sm = c.s->dep_per_sm;
+  a.dep_per_sm = deposit_per_sm(c.s);
   a.dep_agg = c.s->dep_agg;
   a.dep_threads = c.s->dep_threads;
   return a;
@@ -2139,7 +2145,7 @@ std::string tune_key(hps_sim_t s, const char *what) {
 template <class Run, class Restore>
 hps_status tune_search(const std::vector<hps_sim_t> &sims, bool fp32, bool tc_ok, int reps, Run run,
                        Restore restore, Shape *best_out, std::vector<double> *times) {
-  Shape best{sims[0]->sc ? sims[0]->sc->contraction : 0, sims[0]->dep_per_sm, sims[0]->sweep_cap,
+  Shape best{sims[0]->sc ? sims[0]->sc->contraction : 0, deposit_per_sm(sims[0]), sims[0]->sweep_cap,
              sims[0]->dep_agg, sims[0]->dep_threads};
   if (!fp32) { *best_out = best; return HPS_OK; }
   auto measure = [&](const Shape &sh, double *ms) -> hps_status {
@@ -2310,7 +2316,7 @@ hps_status hps_batch_autotune(hps_batch_t bt, int32_t start, int32_t end, int32_
 hps_status hps_sim_get_shape(hps_sim_t s, int32_t *shape_out) {
   if (!s || !shape_out) return fail(HPS_ERR_INVALID, "sim_get_shape: bad argument");
   shape_out[0] = s->sc ? s->sc->contraction : 0;
-  shape_out[1] = (int32_t)s->dep_per_sm;
+  shape_out[1] = (int32_t)deposit_per_sm(s);
   shape_out[2] = (int32_t)s->sweep_cap;
   shape_out[3] = (int32_t)s->dep_agg;
   shape_out[4] = (int32_t)s->dep_threads;

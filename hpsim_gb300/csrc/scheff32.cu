@@ -737,7 +737,24 @@ DepQ dep_quant(uint32_t n, int grid, uint32_t threads, size_t hist_bytes) {
 
 constexpr size_t kMaxHistSmem = 96 * 1024;
 
+// whole clusters of deposit blocks, at most per_sm an SM
+uint32_t deposit_grid(uint32_t n, uint32_t threads, uint32_t per_sm) {
+  const uint32_t b = std::min<uint32_t>((uint32_t)(((uint64_t)n + threads - 1) / threads), per_sm * 152u);
+  return (b + kDepCluster - 1) / kDepCluster * kDepCluster;
+}
+
 }  // namespace
+
+// Three blocks an SM, two where the histogram is 32 KB or more: there clearing
+// the histograms and summing them over the cluster is what a third block adds
+// (64 x 256: 1,000,000 particles through five CCL tanks 7.53 ms with three,
+// 6.81 with two, 7.53 with four; six beams of 262,144 9.04, 8.26, 9.65;
+// 16,777,216 particles 9.99, 9.35, 9.32; 32 x 128: 1,048,576 particles
+// through 331 elements 20.98, 22.19, 22.97).
+uint32_t sc32_deposit_per_sm(uint32_t nr, uint32_t nz) {
+  const size_t hb = (size_t)nr * nz * sizeof(int);
+  return hb < 32 * 1024 || hb > kMaxHistSmem ? 3 : 2;
+}
 
 void beam32_update_stat_for_sc(const DevBeam &b, PassScratch s, cudaStream_t st) {
   if (b.n <= 2) return;
@@ -803,12 +820,13 @@ void sc32_mesh(const DevBeam &b, ScState *sc, const ScTables &t, const ScKickArg
   DepQ q{};
   const uint32_t dthreads = a.dep_threads ? a.dep_threads : 256u;  // deposit block size
   if (a.deposit_ok) {
-    // dep_per_sm blocks per SM at most (three unless tuned), in whole clusters
-    ndep = std::min<uint32_t>((b.n + dthreads - 1) / dthreads, (a.dep_per_sm ? a.dep_per_sm : 3u) * 152u);
-    ndep = (ndep + kDepCluster - 1) / kDepCluster * kDepCluster;
+    ndep = deposit_grid(b.n, dthreads, a.dep_per_sm);
     hb = (size_t)a.nx_max * a.nz_max * sizeof(int);
     if (hb > kMaxHistSmem) hb = 0;
-    q = dep_quant(b.n, (int)ndep, dthreads, hb);
+    // two blocks an SM take the fixed-point scale of three: a block's share is
+    // at most twice as large (one round of particles instead of two, else 5/3),
+    // and a bin's sum stays below 2^31 where the scale leaves it at 2^30
+    q = dep_quant(b.n, (int)deposit_grid(b.n, dthreads, a.dep_per_sm == 2 ? 3 : a.dep_per_sm), dthreads, hb);
     q.agg = a.dep_agg ? 1 : 0;
   }
   // Green's table entries of the largest mesh, a few per thread on one block
