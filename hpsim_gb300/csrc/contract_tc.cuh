@@ -359,6 +359,7 @@ __device__ __forceinline__ void contract_tc_body(const ScState *sc, const ScTabl
 
 // grid (tiles, nr): tile blockIdx.x of field rows, source radius blockIdx.y
 __global__ void __launch_bounds__(kTcThreads, 1) k_contract_tc(const ScState *sc, ScTables t, TcDims d) {
+  pdl_enter();
   contract_tc_body(sc, t, d, blockIdx.x, blockIdx.y);
 }
 // the lockstep form: grid z over the beams, one solver's tables each
@@ -420,6 +421,7 @@ __device__ __forceinline__ void tc_reduce_body(const ScState *sc, const ScTables
 }
 
 __global__ void __launch_bounds__(256) k_tc_reduce(const ScState *sc, ScTables t, TcDims d) {
+  pdl_enter();
   tc_reduce_body(sc, t, d, blockIdx.x, blockIdx.y);
 }
 template <int B>
@@ -461,16 +463,17 @@ inline void contract_tc_merge(const std::vector<const Rec *> &recs, SegFork &, c
   });
 }
 
-// both launches of a tensor-core solve on a mesh of nr x nz
-inline void contract_tc_launch(const ScState *sc, const ScTables &t, uint32_t nr, uint32_t nz, cudaStream_t st) {
+// both launches of a tensor-core solve on a mesh of nr x nz, for a beam of n particles
+inline void contract_tc_launch(const ScState *sc, const ScTables &t, uint32_t nr, uint32_t nz, uint32_t n,
+                               cudaStream_t st) {
   if (recorder()) {
     struct { MeshSeg m; uint32_t dims[2]; } p{{sc, t}, {nr, nz}};
     record("contract_tc", &contract_tc_merge, 0, p, (uint64_t)p.dims[0] << 32 | p.dims[1]);
     return;
   }
   const TcDims d = tc_dims(nr, nz);
-  k_contract_tc<<<dim3(d.tiles, nr), kTcThreads, d.smem, st>>>(sc, t, d);
-  k_tc_reduce<<<dim3((nz + 1 + 63) / 64, nr + 1), 256, 0, st>>>(sc, t, d);
+  launch_after(n, k_contract_tc, dim3(d.tiles, nr), dim3(kTcThreads), d.smem, st, sc, t, d);
+  launch_after(n, k_tc_reduce, dim3((nz + 1 + 63) / 64, nr + 1), dim3(256), 0, st, sc, t, d);
 }
 
 }  // namespace

@@ -242,7 +242,7 @@ uint32_t sc32_deposit_per_sm(uint32_t nr, uint32_t nz);
 // bytes of its folded split-BF16 Green's table and of its partial fields
 bool sc32_tc_mesh(uint32_t nr, uint32_t nz);
 size_t sc32_tc_bytes(uint32_t nr, uint32_t nz, size_t *partial_bytes);
-void contract32(const ScState *sc, const ScTables &t, uint32_t nx_max, uint32_t nz_max, bool mesh_fixed,
+void contract32(const ScState *sc, const ScTables &t, uint32_t nx_max, uint32_t nz_max, bool mesh_fixed, uint32_t n,
                 cudaStream_t st);
 void sc32_stats(const DevBeam &b, ScState *sc, const ScTables &t, const ScKickArgs &a, PassScratch s,
                 cudaStream_t st);

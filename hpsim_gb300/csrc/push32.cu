@@ -457,6 +457,7 @@ __device__ __forceinline__ void kick_push_body(const DevBeam &b, const ScState *
 template <class Map>
 __global__ void __launch_bounds__(kBlock) k32_kick_push(DevBeam b, const ScState *sc, ScTables t, RefK rk,
                                                        uint64_t skip_mask, Map m, Shift sh) {
+  pdl_enter();
   kick_push_body(b, sc, t, rk, skip_mask, m, sh, blockIdx.x, gridDim.x);
 }
 
@@ -562,8 +563,8 @@ void launch_kick_push(const DevBeam &b, const PushFuse &pf, const RefK &rk, cons
            KickPushSeg<Map>{b, (const ScState *)pf.sc, pf.t, rk, pf.skip_mask, m, sh});
     return;
   }
-  launch_k(k32_kick_push<Map>, dim3(grid), dim3(kBlock), 0, st, b, (const ScState *)pf.sc, pf.t, rk, pf.skip_mask, m,
-           sh);
+  launch_after(b.n, k32_kick_push<Map>, dim3(grid), dim3(kBlock), 0, st, b, (const ScState *)pf.sc, pf.t, rk,
+               pf.skip_mask, m, sh);
   note_launch();
 }
 

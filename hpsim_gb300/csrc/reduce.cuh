@@ -403,6 +403,7 @@ __device__ __forceinline__ void pass_body_f(const Op &op, uint32_t n, PassScratc
 
 template <class Op>
 __global__ void __launch_bounds__(kBlock, op_min_blocks<Op>::value) pass_kernel_f(Op op, uint32_t n, PassScratch scr) {
+  pdl_enter();
   pass_body_f(op, n, scr, blockIdx.x, gridDim.x);
 }
 
@@ -433,7 +434,7 @@ inline void launch_pass_f_grid(const Op &op, uint32_t n, PassScratch scr, cudaSt
     record(site, &pass_merge<Op>, blocks, PassSeg<Op>{op, n, scr});
     return;
   }
-  launch_k(pass_kernel_f<Op>, dim3(blocks), dim3(kBlock), 0, s, op, n, scr);
+  launch_after(n, pass_kernel_f<Op>, dim3(blocks), dim3(kBlock), 0, s, op, n, scr);
 }
 
 // With the FP64 combine, at most two blocks per SM: the last block sums

@@ -346,6 +346,7 @@ __device__ __forceinline__ void stat_body(const StatArgs &a, uint32_t bid, uint3
 }
 
 __global__ void __cluster_dims__(kStatCluster, 1, 1) __launch_bounds__(kStatThreads) k32_stat_sweeps(StatArgs a) {
+  pdl_enter();
   stat_body(a, blockIdx.x, gridDim.x);
 }
 // lockstep form: every beam's clusters in one flat launch
@@ -655,6 +656,7 @@ __device__ void deposit_blocks(const DevBeam &bm, ScState *sc, const ScTables &t
 // multiples of the cluster size, so no cluster mixes the two).
 __global__ void __cluster_dims__(kDepCluster, 1, 1) __launch_bounds__(kDepBlockMax)
     k32_green_deposit(DevBeam bm, ScState *sc, ScTables t, DepQ q, uint32_t ndep, uint32_t ngreen) {
+  pdl_enter();
   if (!sc->remesh) return;
   if (blockIdx.x < ndep) deposit_blocks(bm, sc, t, q, blockIdx.x, ndep);
   else green_blocks(sc, t, blockIdx.x - ndep, ngreen);
@@ -804,7 +806,7 @@ void sc32_stats_after_push(const DevBeam &b, ScState *sc, const ScTables &t, con
     record("stats_fallback", &stat_merge, blocks, k);
     return;
   }
-  k32_stat_sweeps<<<blocks, kStatThreads, 0, st>>>(k);
+  launch_after(b.n, k32_stat_sweeps, dim3(blocks), dim3(kStatThreads), 0, st, k);
   note_launch();
 }
 
@@ -841,9 +843,10 @@ void sc32_mesh(const DevBeam &b, ScState *sc, const ScTables &t, const ScKickArg
     }
     record("green", &green_merge, 4u * ngreen, MeshSeg{sc, u});
     record("deposit", &deposit_merge, ndep, DepSeg{b, sc, u, q, hb, dthreads}, dthreads);
-    contract32(sc, u, a.nx_max, a.nz_max, a.mesh_fixed, st);
+    contract32(sc, u, a.nx_max, a.nz_max, a.mesh_fixed, b.n, st);
     return;
   }
+  const bool forked = sur || (fork && ndep && !(ndep <= 152u && q.smem && 5 * hb <= 200 * 1024));
   if (sur) {
     // field surrogate: the deposit alone, the network and its check, then
     // the Green's table and the contraction, which return at once when the
@@ -855,7 +858,7 @@ void sc32_mesh(const DevBeam &b, ScState *sc, const ScTables &t, const ScKickArg
     sur_solve(b, sc, u, a, *sur, st, 1, fork);
     k32_green<<<ngreen, kBlock, 0, st>>>(sc, u);
     note_launch();
-  } else if (fork && ndep) {
+  } else if (forked) {
     // the Green's table on the side stream, beside the deposit: it needs no
     // shared memory, so its blocks take the warp slots the deposit's
     // shared-memory histograms leave free (in one launch they would queue
@@ -869,10 +872,15 @@ void sc32_mesh(const DevBeam &b, ScState *sc, const ScTables &t, const ScKickArg
     cudaStreamWaitEvent(st, fork->ev_join, 0);
     note_launch(2);
   } else {
-    launch_k(k32_green_deposit, dim3(ndep + ngreen), dim3(dthreads), q.smem ? hb : 0, st, b, sc, u, q, ndep, ngreen);
+    // one launch: also for beams whose deposit leaves every SM room for four
+    // blocks of the Green's table, which then need no fork, no second launch
+    // and no join (20,011 particles, a set-point change: 2.26 -> 2.17 ms)
+    const uint32_t ng = fork && ndep ? 4u * ngreen : ngreen;
+    launch_after(b.n, k32_green_deposit, dim3(ndep + ng), dim3(dthreads), q.smem ? hb : 0, st, b, sc, u, q, ndep, ng);
     note_launch();
   }
-  contract32(sc, u, a.nx_max, a.nz_max, a.mesh_fixed, st);
+  // behind a join the contraction waits for both branches as a whole
+  contract32(sc, u, a.nx_max, a.nz_max, a.mesh_fixed, forked ? UINT32_MAX : b.n, st);
 }
 
 void sc32_kick(const DevBeam &b, ScState *sc, const ScTables &t, const ScKickArgs &a, cudaStream_t st) {
@@ -911,12 +919,12 @@ size_t sc32_tc_bytes(uint32_t nr, uint32_t nz, size_t *partial_bytes) {
 // ring convolution otherwise.  Each returns at once when the other one is
 // the one for the kick's mesh; mesh_fixed (the kick's mesh is the largest
 // one, decided on the host) leaves out the one that cannot run.
-void contract32(const ScState *sc, const ScTables &t, uint32_t nx_max, uint32_t nz_max, bool mesh_fixed,
+void contract32(const ScState *sc, const ScTables &t, uint32_t nx_max, uint32_t nz_max, bool mesh_fixed, uint32_t n,
                 cudaStream_t st) {
   const bool tc = t.tcg != nullptr && t.tc_nr == nx_max && t.tc_nz == nz_max;
   const bool rec = recorder() != nullptr;
   if (tc) {
-    contract_tc_launch(sc, t, nx_max, nz_max, st);
+    contract_tc_launch(sc, t, nx_max, nz_max, n, st);
     if (!rec) note_launch(2);
   }
   if (!tc || !mesh_fixed) {
@@ -1008,7 +1016,7 @@ hps_status hps_scheff_field_f32_kernel(uint32_t nr, uint32_t nz, const double *b
     }
     k32_green<<<4 * 152, kBlock>>>(sc, t);
     note_launch(3);
-    contract32(sc, t, nr, nz, true, 0);
+    contract32(sc, t, nr, nz, true, UINT32_MAX, 0);
     e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpy(&tc_error, &sc->tc_error, 4, cudaMemcpyDeviceToHost);
   }
