@@ -12,11 +12,12 @@
 //    1/64 rate, and a dependent FP64 divide costs about a microsecond);
 //  * ahead of a kick on four or more particles, the element half before it
 //    takes every statistics sweep in its own sweep (push32.cu,
-//    OpPushScStats) and certifies that the loss test flags no particle
+//    ScStatsBase) and certifies that the loss test flags no particle
 //    and that no relative phase wraps; only when it cannot, the loss test
-//    and the moments run here in one small launch (Op32LlossScStats, whose
-//    last block sweeps the moments again when the good set changed).  The
-//    kick runs inside the element half after it;
+//    and the moments run here in one small launch (k32_stat_sweeps, whose
+//    last cluster sweeps the moments again when the good set changed).  The
+//    kick runs with the element half after it, in the sweep of the next
+//    element's half where nothing stands between;
 //  * relative phases are not stored: the deposit and the kick form
 //    wrap(phi - <phi>_good) from the phase offset and Sc32Consts::pag;
 //  * the deposit keeps a 32-bit fixed-point histogram per block in shared
