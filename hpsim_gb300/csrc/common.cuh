@@ -52,6 +52,7 @@ struct DevBeam {
   // launch shape of the FP32 particle sweeps and statistics passes: at most
   // this many blocks per SM (0: as many as the SM holds at once)
   uint32_t sweep_cap;
+  uint32_t in_batch;  // the range shares the GPU with other beams' ranges
 };
 
 // SCHEFF solver state in device memory (configuration, the adaptive-remesh

@@ -276,57 +276,35 @@ __global__ void __launch_bounds__(kBlock) k32_run(const __grid_constant__ RunArg
 // one, sc32_stats_after_push); so it does when s lies more than 4
 // sigma_phi from <phi>_good, where sigma_phi^2 as a difference of FP32
 // moments about s would lose precision.
+//
+// The sums have one order in every form of the sweep, whatever launches it:
+// that of blocks of 256 threads, two an SM at most (pass_blocks_f), in which a
+// thread adds its particles in turn (every gridDim x 256th), then the warps'
+// shuffle trees, the warps in order and the blocks as combine_slot_f takes
+// them.  The mesh's edge follows from the sums, and a particle there is kicked
+// from either side by the edge's last bit: in another order one particle in
+// some five million ended elsewhere after a few kicks at low energy.
 struct ScStatsBase {
   // 0 good count, 1 sum d (raw, for <phi>_good), 2-3 sum f, f^2 (wrapped, for
   // sigma_phi), 4-8 x, x^2, y, y^2, W of the good set; 9 sum f, 10 count of the
   // live set; 11 lloss count; 12 max |f| over the live set; 13 max phi over
   // lloss != 1.  d = phi - s, f = wrap(d).
   static constexpr int K = 14;
-  static constexpr int kMaxFrom = 12;
-  // every form of the sweep has the same blocks, so that a kick's statistics
-  // are summed in the same order whatever the sweep runs with
-  static constexpr int kBatch = 1;
-  static constexpr int kMinBlocks = 4;
-  static constexpr int kGridPerSm = 4;
-  static constexpr bool kFast = true;
-  using Comb = SumComb;
-  using Stage = Sc32Stage;
-  struct P { Part p; uint32_t ll; };
   DevBeam b;  // carries the synchronous particle after the element
   int s_last;  // s from the last kick's <phi>_good offset (else 0)
   ScState *sc;
   ScTables tb;
   double freq, frac;
   Sc32Host h;
-  __device__ bool enabled() const { return true; }
   __device__ float origin() const {
     const float e = s_last ? tb.c32->pag : 0.0f;
     return fabsf(e) < 3.14159265f ? e : 0.0f;
   }
-  __device__ P load(uint32_t i) const { return {load_part(b, i), b.lloss[i]}; }
-  __device__ void add(const Part &p, uint32_t ll, float s, float (&a)[K]) const {
-    const bool alive = p.lo == 0u, g = alive && ll == 0u;
-    const float d = p.ph - s, f = rel_phase_f(d);
-    a[0] += g ? 1.0f : 0.0f;
-    a[1] += g ? d : 0.0f;
-    a[2] += g ? f : 0.0f;
-    a[3] += g ? f * f : 0.0f;
-    a[4] += g ? p.x : 0.0f;
-    a[5] += g ? p.x * p.x : 0.0f;
-    a[6] += g ? p.y : 0.0f;
-    a[7] += g ? p.y * p.y : 0.0f;
-    a[8] += g ? p.w : 0.0f;
-    a[9] += alive ? f : 0.0f;
-    a[10] += alive ? 1.0f : 0.0f;
-    a[11] += ll != 0u ? 1.0f : 0.0f;
-    if (alive) a[12] = fmaxf(a[12], fabsf(f));
-    if (ll != 1u) a[13] = fmaxf(a[13], p.ph);
-  }
-  __device__ void stage_load(Stage &g, int tid, int nth) const {
+  __device__ void stage_load(Sc32Stage &g, int tid, int nth) const {
     sc32_stage_load(g, b, sc, tid, nth);
     if (tid == nth - 1) g.c.pag = origin();  // until the kick's constants take its place
   }
-  __device__ void finalize(const double *t, int tid, int nth, Stage &stage) const {
+  __device__ void finalize(const double *t, int tid, int nth, Sc32Stage &stage) const {
     __shared__ int ok;
     if (tid == 0) {
       BeamStats &st = stage.st;
@@ -362,18 +340,17 @@ struct ScStatsBase {
   }
 };
 
+// the form of the sweep with a map alone: advance() takes a particle through
+// it and stores what changed
 template <class Map>
 struct OpPushScStats : ScStatsBase {
-  static constexpr bool kThreadSetup = true;
   struct Ctx { float s; };
   Map m;
   Shift sh;
   __device__ Ctx setup() const { return {origin()}; }
-  __device__ void use(uint32_t i, const P &q, float (&a)[K], const Ctx &c) const {
-    Part p = q.p;
+  __device__ void advance(uint32_t i, Part &p, uint32_t, const Ctx &) const {
     const uint32_t w = step(p, m, sh);
     if (w) store_part(b, i, p, w);
-    add(p, q.ll, c.s, a);
   }
 };
 
@@ -397,7 +374,6 @@ struct PreRec {
 // block has finished its particles.
 template <class A>
 struct OpKickPushScStats : ScStatsBase {
-  static constexpr bool kSharedCtx = true;
   struct Ctx { float s; KickEnv e; };
   RefK rk;
   uint64_t skip_mask;
@@ -405,10 +381,9 @@ struct OpKickPushScStats : ScStatsBase {
   Shift sh1;
   PreRec m;
   __device__ Ctx setup() const { return {origin(), kick_env(sc, tb, rk)}; }
-  __device__ void use(uint32_t i, const P &q, float (&a)[K], const Ctx &c) const {
-    Part p = q.p;
+  __device__ void advance(uint32_t i, Part &p, uint32_t ll, const Ctx &c) const {
     uint32_t w = 0;
-    if (p.lo == 0u && q.ll == 0u && ((uint64_t)i & skip_mask) != 0)
+    if (p.lo == 0u && ll == 0u && ((uint64_t)i & skip_mask) != 0)
       w = kick_particle(p, rel_phase_f(p.ph - c.e.pag), c.e);
     w |= step(p, a1, sh1);
     switch (m.kind) {
@@ -417,9 +392,208 @@ struct OpKickPushScStats : ScStatsBase {
       default: w |= step(p, m.gap1, m.sh); break;
     }
     if (w) store_part(b, i, p, w);
-    add(p, q.ll, c.s, a);
   }
 };
+
+// what a particle adds to the sums: of the good set (zero elsewhere) and, fl,
+// of the live set
+struct SweepTerms {
+  float x, y, w, d, f, fl;
+};
+
+// Block bid of nblk.  Two blocks an SM, as the order of the sums has it, keep
+// half of an SM's issue slots busy.  A beam alone (NG = 2) therefore runs a
+// block as two groups of 256 threads that take its rounds in turn and hand
+// each other the terms through shared memory: one group keeps the sums of x, y
+// and W, the other those of the phases, and each adds the rounds in their
+// order; a thread's next particle is on its way meanwhile.  Beams that share
+// the GPU fill it together: there a block is one group (NG = 1), whose 1.3 KB
+// of shared memory fit beside another beam's field sum where 14 KB do not.
+// Microseconds, NG = 1 | 2: 16,777,216 particles through a CCL tank 11,200 |
+// 9,370, 1,048,576 through 331 elements 22,260 | 21,190, 20,011 with a set-point
+// change 1,815 | 1,705; 32 beams of 16,384 to 524,288 together 24,700 |
+// 26,110, six of 262,144 8,320 | 8,670.
+template <int NG, class Op>
+__device__ __forceinline__ void sweep_body(const Op &op, PassScratch scr, uint32_t bid, uint32_t nblk) {
+  static_assert(NG == 1 || NG == 2, "one group or two");
+  constexpr int K = Op::K, kMax = 12, kWarps = kBlock / 32;
+  __shared__ float red[kMax][kWarps];
+  __shared__ float red_max[2][NG * kWarps];
+  __shared__ uint32_t red_cnt[3][NG * kWarps];
+  __shared__ double tot[K];
+  __shared__ Sc32Stage stage;
+  __shared__ typename Op::Ctx ctx;
+  __shared__ int is_last;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, grp = tid / kBlock, t = tid % kBlock, wg = t >> 5;
+  if (tid == 0) ctx = op.setup();
+  __syncthreads();
+  const float s = ctx.s;
+  const uint32_t n = op.b.n, stride = nblk * kBlock, rounds = (n + stride - 1) / stride;
+  uint32_t good = 0, live = 0, lloss = 0;
+  float fmax_ = -INFINITY, phmax = -INFINITY;
+  auto take = [&](uint32_t i, Part &p, uint32_t ll) {
+    op.advance(i, p, ll, ctx);
+    const bool alive = p.lo == 0u, g = alive && ll == 0u;
+    const float d = p.ph - s, f = rel_phase_f(d);
+    if (alive) fmax_ = fmaxf(fmax_, fabsf(f));
+    if (ll != 1u) phmax = fmaxf(phmax, p.ph);
+    good += g;
+    live += alive;
+    lloss += ll != 0u;
+    return SweepTerms{g ? p.x : 0.0f, g ? p.y : 0.0f, g ? p.w : 0.0f, g ? d : 0.0f, g ? f : 0.0f, alive ? f : 0.0f};
+  };
+  auto add = [](float &v, float e) { v += e; };
+  auto add2 = [](float &v, float &v2, float e) {
+    v += e;
+    v2 = __fadd_rn(v2, __fmul_rn(e, e));
+  };
+  auto tree = [&](float v, int k) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+    if (lane == 0) red[k][wg] = v;
+  };
+  if constexpr (NG == 1) {
+    float a[9] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    for (uint32_t i = bid * kBlock + t; i < n; i += stride) {
+      Part p = load_part(op.b, i);
+      const SweepTerms e = take(i, p, op.b.lloss[i]);
+      add2(a[3], a[4], e.x);
+      add2(a[5], a[6], e.y);
+      add(a[7], e.w);
+      add(a[0], e.d);
+      add2(a[1], a[2], e.f);
+      add(a[8], e.fl);
+    }
+#pragma unroll
+    for (int k = 0; k < 9; ++k) tree(a[k], k + 1);
+  } else {
+    __shared__ float term[2][6][kBlock];  // what the groups hand over, in two sets
+    Part next{};
+    uint32_t next_ll = 0;
+    auto fetch = [&](uint32_t r, uint32_t i) {
+      if (r < rounds && i < n) {
+        next = load_part(op.b, i);
+        next_ll = op.b.lloss[i];
+      }
+    };
+    float a[5] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    fetch(grp, grp * stride + bid * kBlock + t);
+    for (uint32_t r = 0; r < rounds; r += 2) {
+      const uint32_t i = (r + grp) * stride + bid * kBlock + t;
+      Part p = next;
+      const uint32_t ll = next_ll;
+      fetch(r + grp + 2, i + 2 * stride);
+      SweepTerms e = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+      if (r + grp < rounds && i < n) e = take(i, p, ll);
+      // a set is written again behind the next rounds' barrier
+      float(&tm)[6][kBlock] = term[(r / 2) & 1];
+      auto sync = [&] { asm volatile("bar.sync %0, 64;" ::"r"(1 + wg) : "memory"); };
+      if (grp == 0) {
+        tm[3][t] = e.d; tm[4][t] = e.f; tm[5][t] = e.fl;
+        sync();
+        add2(a[0], a[1], e.x); add2(a[0], a[1], tm[0][t]);
+        add2(a[2], a[3], e.y); add2(a[2], a[3], tm[1][t]);
+        add(a[4], e.w); add(a[4], tm[2][t]);
+      } else {
+        tm[0][t] = e.x; tm[1][t] = e.y; tm[2][t] = e.w;
+        sync();
+        add(a[0], tm[3][t]); add(a[0], e.d);
+        add2(a[1], a[2], tm[4][t]); add2(a[1], a[2], e.f);
+        add(a[3], tm[5][t]); add(a[3], e.fl);
+      }
+    }
+    if (grp == 0) { tree(a[0], 4); tree(a[1], 5); tree(a[2], 6); tree(a[3], 7); tree(a[4], 8); }
+    else { tree(a[0], 1); tree(a[1], 2); tree(a[2], 3); tree(a[3], 9); }
+  }
+  // counts and maxima: exact in any order
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    fmax_ = fmaxf(fmax_, __shfl_xor_sync(0xffffffffu, fmax_, off));
+    phmax = fmaxf(phmax, __shfl_xor_sync(0xffffffffu, phmax, off));
+  }
+  good = __reduce_add_sync(0xffffffffu, good);
+  live = __reduce_add_sync(0xffffffffu, live);
+  lloss = __reduce_add_sync(0xffffffffu, lloss);
+  if (lane == 0) {
+    red_cnt[0][warp] = good;
+    red_cnt[1][warp] = live;
+    red_cnt[2][warp] = lloss;
+    red_max[0][warp] = fmax_;
+    red_max[1][warp] = phmax;
+  }
+  __syncthreads();
+  float *partf = (float *)scr.part;
+  if (tid < K) {
+    float v;
+    if (tid >= kMax) {
+      v = -INFINITY;
+      for (int w = 0; w < NG * kWarps; ++w) v = fmaxf(v, red_max[tid - kMax][w]);
+    } else if (tid == 0 || tid >= 10) {
+      uint32_t c = 0;
+      for (int w = 0; w < NG * kWarps; ++w) c += red_cnt[tid == 0 ? 0 : tid - 9][w];
+      v = (float)c;
+    } else {
+      v = 0.0f;
+      for (int w = 0; w < kWarps; ++w) v += red[tid][w];
+    }
+    if (nblk == 1) tot[tid] = (double)v;
+    else partf[(size_t)tid * kMaxPassBlocks + bid] = v;
+  }
+  if (nblk > 1) {
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) is_last = (atomicAdd(scr.counter, 1u) == nblk - 1);
+    __syncthreads();
+    if (!is_last) return;
+    __threadfence();
+    op.stage_load(stage, tid, blockDim.x);
+    for (int k = warp; k < K; k += NG * kWarps) {
+      const float v = combine_slot_f<SumComb, kMax>(partf, k, nblk);
+      if (lane == 0) tot[k] = (double)v;
+    }
+  } else {
+    op.stage_load(stage, tid, blockDim.x);
+  }
+  __syncthreads();
+  op.finalize(tot, tid, blockDim.x, stage);
+  __syncthreads();
+  if (tid == 0 && nblk > 1) *scr.counter = 0u;
+}
+
+template <class Op, int NG>
+__global__ void __launch_bounds__(NG *kBlock, 4 / NG) k32_sweep(Op op, PassScratch scr) {
+  pdl_enter();
+  sweep_body<NG>(op, scr, blockIdx.x, gridDim.x);
+}
+// lockstep form, one beam's share of a merged launch
+template <class Op>
+struct SweepSeg {
+  Op op;
+  PassScratch scr;
+};
+template <class Op, int B>
+__global__ void __launch_bounds__(kBlock, 4) k32_sweep_seg(const __grid_constant__ SegArgs<SweepSeg<Op>, B> a) {
+  uint32_t bid, nblk;
+  const SweepSeg<Op> &p = a.p[seg_find(a, blockIdx.x, bid, nblk)];
+  sweep_body<1>(p.op, p.scr, bid, nblk);
+}
+template <class Op>
+void sweep_merge(const std::vector<const Rec *> &recs, SegFork &, cudaStream_t st, cudaStream_t) {
+  seg_chunks<SweepSeg<Op>>(recs, [&](const auto &a, uint32_t blocks) {
+    k32_sweep_seg<Op, std::decay_t<decltype(a)>::kB><<<blocks, kBlock, 0, st>>>(a);
+  });
+}
+template <class Op>
+void launch_sweep(const Op &op, PassScratch scr, cudaStream_t st, const char *site) {
+  const DevBeam &b = op.b;
+  const uint32_t blocks = (uint32_t)pass_blocks_f(b.n, b.sweep_cap == 1 ? 1 : 2);
+  if (recorder()) {
+    record(site, &sweep_merge<Op>, blocks, SweepSeg<Op>{op, scr});
+    return;
+  }
+  if (b.in_batch) launch_after(b.n, k32_sweep<Op, 1>, dim3(blocks), dim3(kBlock), 0, st, op, scr);
+  else launch_after(b.n, k32_sweep<Op, 2>, dim3(blocks), dim3(2 * kBlock), 0, st, op, scr);
+}
 
 // ApplySpchKickKernel on the particles it kicks (alive, not longitudinally
 // lost, outside the skipped set), then the map on every live particle
@@ -628,8 +802,8 @@ template <class A>
 bool launch_kick_to_kick(PushQueue &q, const ScStatsBase &base, const PreRec &m, const PushFuse &pf, cudaStream_t st) {
   if (q.k.kind != map_kind<A>()) return false;
   q.kick = false;
-  launch_pass_f(OpKickPushScStats<A>{base, q.k.rk, q.k.pf.skip_mask, q.k.as<A>(), q.k.sh, m}, base.b.n, pf.scr, st,
-                base.b.sweep_cap, "kick_push_scstats");
+  launch_sweep(OpKickPushScStats<A>{base, q.k.rk, q.k.pf.skip_mask, q.k.as<A>(), q.k.sh, m}, pf.scr, st,
+               "kick_push_scstats");
   return true;
 }
 
@@ -669,7 +843,7 @@ void launch_map(const DevBeam &b, const Map &m, const RefK &rk, double phi0, dou
       if (!done) {
         push32_flush(&q);
         if constexpr (joins_kick<Map>() || std::is_same_v<Map, DipMap>)
-          launch_pass_f(OpPushScStats<Map>{base, m, sh}, b.n, pf.scr, st, b.sweep_cap, "push_scstats");
+          launch_sweep(OpPushScStats<Map>{base, m, sh}, pf.scr, st, "push_scstats");
       }
       if (!recorder()) note_launch();
       return;

@@ -218,50 +218,39 @@ struct op_max_from : std::integral_constant<int, Op::K> {};
 template <class Op>
 struct op_max_from<Op, std::void_t<decltype(Op::kMaxFrom)>> : std::integral_constant<int, Op::kMaxFrom> {};
 
-// An Op with `static constexpr bool kThreadSetup = true` has setup() run by
-// every thread instead of once per block: for set-ups of a load or two in
-// FP32, whose latency then overlaps the first particles' loads instead of
-// standing before them behind a barrier.
+// An Op with kFast fixes its blocks per SM (`static constexpr int kGridPerSm`):
+// the order of its sums follows from the number of blocks, and must not change
+// with the registers that a compiler gives the kernel.
 template <class Op, class = void>
-struct op_thread_setup : std::false_type {};
-template <class Op>
-struct op_thread_setup<Op, std::void_t<decltype(Op::kThreadSetup)>>
-    : std::integral_constant<bool, Op::kThreadSetup> {};
-
-// An Op with `static constexpr bool kSharedCtx = true` reads its set-up from
-// shared memory where it uses it: for set-ups of many values, which would
-// otherwise take a register each.
-template <class Op, class = void>
-struct op_shared_ctx : std::false_type {};
-template <class Op>
-struct op_shared_ctx<Op, std::void_t<decltype(Op::kSharedCtx)>> : std::integral_constant<bool, Op::kSharedCtx> {};
-
-// An Op may ask for a number of resident blocks per SM (`static constexpr int
-// kMinBlocks`), which bounds its registers.
-template <class Op, class = void>
-struct op_min_blocks : std::integral_constant<int, 1> {};
-template <class Op>
-struct op_min_blocks<Op, std::void_t<decltype(Op::kMinBlocks)>> : std::integral_constant<int, Op::kMinBlocks> {};
-
-// An Op may fix its blocks per SM (`static constexpr int kGridPerSm`, at most
-// what an SM holds), so that its sums have one order in every form.
-template <class Op, class = void>
-struct op_grid_per_sm : std::integral_constant<int, 0> {};
+struct op_grid_per_sm : std::integral_constant<int, 2> {};
 template <class Op>
 struct op_grid_per_sm<Op, std::void_t<decltype(Op::kGridPerSm)>> : std::integral_constant<int, Op::kGridPerSm> {};
-
-// An Op with a nested `Stage` has one of them in the last block's shared
-// memory: stage_load(stage, tid, nthreads) runs before that block combines
-// the partials, and finalize takes the stage as a fourth argument.
-struct NoStage {};
-template <class Op, class = void>
-struct op_stage { using type = NoStage; static constexpr bool value = false; };
-template <class Op>
-struct op_stage<Op, std::void_t<typename Op::Stage>> { using type = typename Op::Stage; static constexpr bool value = true; };
 
 template <class C, int MF>
 __device__ inline float comb_k(int k, float a, float b) {
   return k >= MF ? fmaxf(a, b) : C::comb(a, b);
+}
+
+// Slot k's total over the FP32 partials of nblk blocks, taken by a warp: lane l
+// sums blocks l, l + 32, ... (eight loads in flight), then a fixed shuffle tree
+// (lane 0 has the result).  Partials lie slot by slot, kMaxPassBlocks apart.
+template <class C, int MF>
+__device__ __forceinline__ float combine_slot_f(const float *part, int k, uint32_t nblk) {
+  const int lane = threadIdx.x & 31;
+  const float *p = part + (size_t)k * kMaxPassBlocks;
+  float v = k >= MF ? -INFINITY : 0.0f;
+  for (uint32_t b = lane; b < nblk; b += 8 * 32) {
+    float r[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (b + 32 * u < nblk) r[u] = __ldcg(p + b + 32 * u);
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (b + 32 * u < nblk) v = comb_k<C, MF>(k, v, r[u]);
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) v = comb_k<C, MF>(k, v, __shfl_down_sync(0xffffffffu, v, off));
+  return v;
 }
 
 // block bid of nblk blocks of the pass over particles 0..n-1
@@ -274,19 +263,11 @@ __device__ __forceinline__ void pass_body_f(const Op &op, uint32_t n, PassScratc
   __shared__ double tot[K];
   __shared__ int is_last;
   __shared__ typename Op::Ctx sctx;
-  typename Op::Ctx rctx;
-  if constexpr (op_thread_setup<Op>::value) {
-    rctx = op.setup();
-  } else {
-    if (threadIdx.x == 0) sctx = op.setup();
-    __syncthreads();
-    if constexpr (!op_shared_ctx<Op>::value) rctx = sctx;
-  }
-  const typename Op::Ctx &ctx = op_shared_ctx<Op>::value ? sctx : rctx;
+  if (threadIdx.x == 0) sctx = op.setup();
+  __syncthreads();
+  const typename Op::Ctx ctx = sctx;
   constexpr int MF = op_max_from<Op>::value;
   static_assert(MF == K || op_fast<Op>::value, "max slots need the FP32 combine");
-  static_assert(!op_stage<Op>::value || op_fast<Op>::value, "a stage needs the FP32 combine");
-  __shared__ typename op_stage<Op>::type stage;
   float acc[K];
 #pragma unroll
   for (int k = 0; k < K; ++k) acc[k] = k >= MF ? -INFINITY : 0.0f;
@@ -307,70 +288,36 @@ __device__ __forceinline__ void pass_body_f(const Op &op, uint32_t n, PassScratc
 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if constexpr (op_fast<Op>::value) {
-    // FP32 partials, no FP64 arithmetic on the reduction's critical path:
-    // warps summed in order per block; then the last block's thread t takes
-    // the K slots of blocks t, t + 256, ... (every load of a row in flight at
-    // once: the 304 rows of a large beam's 14 slots cost one or two memory
-    // round trips, where a warp per slot took several per slot), the lanes by
-    // a fixed shuffle tree and the warps in order.  A pass of one block has
-    // its totals at once.
+    // FP32 partials: warps summed in order per block, blocks by the warps of
+    // the last block (slot k by warp k mod 8).  No FP64 arithmetic on the
+    // reduction's critical path.
     __shared__ float smf[kBlock / 32][K];
     float *partf = (float *)scr.part;
-    auto warps = [&](const float (&a)[K]) {
 #pragma unroll
-      for (int k = 0; k < K; ++k) {
-        float v = a[k];
+    for (int k = 0; k < K; ++k) {
+      float v = acc[k];
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) v = comb_k<C, MF>(k, v, __shfl_down_sync(0xffffffffu, v, off));
-        if (lane == 0) smf[warp][k] = v;
-      }
-    };
-    auto block_sum = [&](int k, int nw) {
-      float v = k >= MF ? -INFINITY : 0.0f;
-      for (int w = 0; w < nw; ++w) v = comb_k<C, MF>(k, v, smf[w][k]);
-      return v;
-    };
-    warps(acc);
-    __syncthreads();
-    if (nblk == 1) {
-      if constexpr (op_stage<Op>::value) op.stage_load(stage, threadIdx.x, blockDim.x);
-      if (threadIdx.x < K) tot[threadIdx.x] = (double)block_sum(threadIdx.x, kBlock / 32);
-      __syncthreads();
-    } else {
-      if (threadIdx.x < K) partf[bid * K + threadIdx.x] = block_sum(threadIdx.x, kBlock / 32);
-      __threadfence();
-      __syncthreads();
-      if (threadIdx.x == 0) is_last = (atomicAdd(scr.counter, 1u) == nblk - 1);
-      __syncthreads();
-      if (!is_last) return;
-      __threadfence();
-      if constexpr (op_stage<Op>::value) op.stage_load(stage, threadIdx.x, blockDim.x);
-      const int nw = min(kBlock / 32, (int)((nblk + 31) / 32));  // warps with rows to take
-      if (warp < nw) {
-#pragma unroll
-        for (int k = 0; k < K; ++k) acc[k] = k >= MF ? -INFINITY : 0.0f;
-        for (uint32_t b = threadIdx.x; b < nblk; b += kBlock) {
-          float row[K];
-          if constexpr (K % 2 == 0) {
-#pragma unroll
-            for (int k = 0; k < K / 2; ++k) {
-              const float2 v = __ldcg((const float2 *)(partf + (size_t)b * K) + k);
-              row[2 * k] = v.x;
-              row[2 * k + 1] = v.y;
-            }
-          } else {
-#pragma unroll
-            for (int k = 0; k < K; ++k) row[k] = __ldcg(partf + (size_t)b * K + k);
-          }
-#pragma unroll
-          for (int k = 0; k < K; ++k) acc[k] = comb_k<C, MF>(k, acc[k], row[k]);
-        }
-        warps(acc);
-      }
-      __syncthreads();
-      if (threadIdx.x < K) tot[threadIdx.x] = (double)block_sum(threadIdx.x, nw);
-      __syncthreads();
+      for (int off = 16; off > 0; off >>= 1) v = comb_k<C, MF>(k, v, __shfl_down_sync(0xffffffffu, v, off));
+      if (lane == 0) smf[warp][k] = v;
     }
+    __syncthreads();
+    if (threadIdx.x < K) {
+      const int k = threadIdx.x;
+      float v = k >= MF ? -INFINITY : 0.0f;
+      for (int w = 0; w < kBlock / 32; ++w) v = comb_k<C, MF>(k, v, smf[w][k]);
+      partf[(size_t)k * kMaxPassBlocks + bid] = v;
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) is_last = (atomicAdd(scr.counter, 1u) == nblk - 1);
+    __syncthreads();
+    if (!is_last) return;
+    __threadfence();
+    for (int k = warp; k < K; k += kBlock / 32) {
+      const float v = combine_slot_f<C, MF>(partf, k, nblk);
+      if (lane == 0) tot[k] = (double)v;
+    }
+    __syncthreads();
   } else {
     __shared__ double sm[combine_rows<K>()][K];
 #pragma unroll
@@ -395,14 +342,13 @@ __device__ __forceinline__ void pass_body_f(const Op &op, uint32_t n, PassScratc
     __threadfence();
     combine_partials<C, K>(scr.part, nblk, sm, tot);
   }
-  if constexpr (op_stage<Op>::value) op.finalize(tot, threadIdx.x, blockDim.x, stage);
-  else op.finalize(tot, threadIdx.x, blockDim.x);
+  op.finalize(tot, threadIdx.x, blockDim.x);
   __syncthreads();
   if (threadIdx.x == 0) *scr.counter = 0u;
 }
 
 template <class Op>
-__global__ void __launch_bounds__(kBlock, op_min_blocks<Op>::value) pass_kernel_f(Op op, uint32_t n, PassScratch scr) {
+__global__ void __launch_bounds__(kBlock) pass_kernel_f(Op op, uint32_t n, PassScratch scr) {
   pdl_enter();
   pass_body_f(op, n, scr, blockIdx.x, gridDim.x);
 }
@@ -415,7 +361,7 @@ struct PassSeg {
   PassScratch scr;
 };
 template <class Op, int B>
-__global__ void __launch_bounds__(kBlock, op_min_blocks<Op>::value) pass_kernel_f_seg(const __grid_constant__ SegArgs<PassSeg<Op>, B> a) {
+__global__ void __launch_bounds__(kBlock) pass_kernel_f_seg(const __grid_constant__ SegArgs<PassSeg<Op>, B> a) {
   uint32_t bid, nblk;
   const PassSeg<Op> &p = a.p[seg_find(a, blockIdx.x, bid, nblk)];
   pass_body_f(p.op, p.n, p.scr, bid, nblk);
@@ -437,21 +383,12 @@ inline void launch_pass_f_grid(const Op &op, uint32_t n, PassScratch scr, cudaSt
   launch_after(n, pass_kernel_f<Op>, dim3(blocks), dim3(kBlock), 0, s, op, n, scr);
 }
 
-// With the FP64 combine, at most two blocks per SM: the last block sums
-// every block's partials in FP64 on one SM (1/64-rate FP64 on GB300), so
-// fewer, fuller blocks keep that tail short; each thread walks more
-// particles in batches instead.  With the FP32 combine, every block the SMs
-// hold at once (up to the scratch's kMaxPassBlocks).
-// A pass that takes a particle at a time (batch 1) spreads a small beam over
-// the SMs, a particle a thread up to one block on each; beyond that its blocks
-// hold four a thread as the others' do (more blocks make a lone beam no
-// faster and cost beams that share the SMs their reductions: a scan of 32
-// beams 24.6 -> 26.3 ms with a particle a thread throughout).  Up to 1,024
-// particles one block without a grid-wide sum is as fast (558 against 552 us
-// for eight kicks).
-inline int pass_blocks_f(uint32_t n, int per_sm = 2, int batch = kPassBatch) {
+// Blocks of a pass: four particles a thread until there are per_sm blocks on
+// every SM, then more a thread.  With the FP64 combine that is two: the last
+// block sums every block's partials in FP64 on one SM (1/64-rate FP64 on
+// GB300), so fewer, fuller blocks keep that tail short.
+inline int pass_blocks_f(uint32_t n, int per_sm = 2) {
   uint32_t b = (uint32_t)(((uint64_t)n + kPassBatch * kBlock - 1) / (kPassBatch * kBlock));
-  if (batch == 1 && n > 4 * kBlock) b = std::max(b, std::min<uint32_t>((uint32_t)(((uint64_t)n + kBlock - 1) / kBlock), 152u));
   if (b < 1) b = 1;
   const uint32_t cap = std::min<uint32_t>((uint32_t)per_sm * 152u, (uint32_t)kMaxPassBlocks);
   if (b > cap) b = cap;
@@ -459,20 +396,8 @@ inline int pass_blocks_f(uint32_t n, int per_sm = 2, int batch = kPassBatch) {
 }
 
 template <class Op>
-inline int pass_resident() {
-  static int r = 0;  // blocks of this kernel an SM holds at once
-  if (!r && (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, pass_kernel_f<Op>, kBlock, 0) != cudaSuccess || r < 1))
-    r = 1;
-  return r;
-}
-
-// cap: at most this many blocks per SM (0: no cap)
-template <class Op>
-inline void launch_pass_f(const Op &op, uint32_t n, PassScratch scr, cudaStream_t s, uint32_t cap = 0,
-                          const char *site = "pass") {
-  int per_sm = op_grid_per_sm<Op>::value ? op_grid_per_sm<Op>::value : op_fast<Op>::value ? pass_resident<Op>() : 2;
-  if (cap && (uint32_t)per_sm > cap) per_sm = (int)cap;
-  launch_pass_f_grid(op, n, scr, s, (uint32_t)pass_blocks_f(n, per_sm, op_fast<Op>::value ? op_batch<Op>::value : kPassBatch), site);
+inline void launch_pass_f(const Op &op, uint32_t n, PassScratch scr, cudaStream_t s) {
+  launch_pass_f_grid(op, n, scr, s, (uint32_t)pass_blocks_f(n, op_grid_per_sm<Op>::value), "pass");
 }
 
 // FP32 version of rel_phase for offsets that are already small

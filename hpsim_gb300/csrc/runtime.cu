@@ -1439,7 +1439,9 @@ struct RunPlan {
   double solves0 = 0.0;
 };
 
-hps_status plan_run(hps_sim_t s, int32_t start, int32_t end, RunPlan *p) {
+// in_batch: the range shares the GPU with other simulators' ranges.  It shapes
+// the launches, not the results, so a graph captured either way serves both.
+hps_status plan_run(hps_sim_t s, int32_t start, int32_t end, RunPlan *p, bool in_batch = false) {
   if (!s) return fail(HPS_ERR_INVALID, "bad sim handle");
   p->c = Ctx{s, s->beam, s->bl, s->sc};
   Ctx &c = p->c;
@@ -1458,6 +1460,7 @@ hps_status plan_run(hps_sim_t s, int32_t start, int32_t end, RunPlan *p) {
   hps_beam_t b = c.b;
   cudaStream_t st = b->stream;
   b->d.sweep_cap = s->sweep_cap;
+  b->d.in_batch = in_batch;
   p->monitor = s->mon_host && s->mon_cap >= (uint32_t)n;
   if (p->monitor && s->mon_dev_cap < (uint32_t)n) {
     if (s->mon_dev) cudaFree(s->mon_dev);
@@ -1934,7 +1937,7 @@ hps_status hps_batch_simulate(hps_batch_t bt, int32_t start, int32_t end) {
   std::vector<RunPlan> plans(m);
   for (size_t k = 0; k < m; ++k) {
     CK(cudaStreamSynchronize(bt->sims[k]->beam->stream));  // the beam's own work first
-    hps_status e = plan_run(bt->sims[k], start, end, &plans[k]);
+    hps_status e = plan_run(bt->sims[k], start, end, &plans[k], m > 1);
     if (e) return e;
     if (!plans[k].empty && !plans[k].graph)
       return fail(HPS_ERR_STATE, "batch_simulate: a simulator cannot run as a graph (graphs off, profiling on, "

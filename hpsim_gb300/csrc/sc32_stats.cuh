@@ -168,17 +168,19 @@ __device__ void sc32_decide_consts(const BeamStats &st, const DevBeam &b, ScStat
 }
 
 // The SCHEFF moments from their totals s[0..7] (FP32 arithmetic, see
-// Sc32Host) into the beam's scalars (num_loss and num_good set), one thread
+// Sc32Host) into the beam's scalars (num_loss and num_good set), one thread.
+// fmaf says what is rounded (one product of each difference; which one is
+// free, but fixed): the mesh's edge follows, and it decides single particles by
+// its last bit.
 __device__ inline void sc_moments(const DevBeam &b, BeamStats &st, const double *s) {
   const float isv = 1.0f / (float)(uint32_t)(b.n - st.num_loss), ing = 1.0f / (float)st.num_good;
   st.st[PHI_AVG_R] = (float)s[0] * isv;
-  const float pa = (float)s[1] * ing, pa2 = (float)s[2] * ing;
-  st.st[PHI_SIG_GOOD] = sqrtf(pa2 - pa * pa);
-  const float xa = (float)s[3] * isv, x2 = (float)s[4] * isv, ya = (float)s[5] * isv, y2 = (float)s[6] * isv;
+  const float pa = (float)s[1] * ing, xa = (float)s[3] * isv, ya = (float)s[5] * isv;
+  st.st[PHI_SIG_GOOD] = sqrtf(fmaf((float)s[2], ing, -(pa * pa)));
   st.st[X_AVG_GOOD] = xa;
-  st.st[X_SIG_GOOD] = sqrtf(x2 - xa * xa);
+  st.st[X_SIG_GOOD] = sqrtf(fmaf((float)s[4], isv, -(xa * xa)));
   st.st[Y_AVG_GOOD] = ya;
-  st.st[Y_SIG_GOOD] = sqrtf(y2 - ya * ya);
+  st.st[Y_SIG_GOOD] = sqrtf(fmaf(-ya, ya, (float)s[6] * isv));
   st.st[W_AVG_GOOD] = st.num_good > 0 ? (double)((float)s[7] * ing) + b.w_ref : -99999;
 }
 
@@ -198,17 +200,6 @@ __device__ void sc_moments_finish(const DevBeam &b, const double *s, Sc32Stage &
   sc_moments(b, st, s);
   g.st = st;
   sc32_decide_consts(st, b, &g.sc, &g.c, h, freq, frac);
-}
-
-// the SCHEFF moments' per-particle terms: 0 mean relative phase of the live
-// set, 1-2 phase, 3-6 x, x^2, y, y^2, 7 W of the good set
-__device__ inline void sc_moments_add(float (&a)[12], float pr, uint32_t lo, uint32_t ll, float x, float y, float w) {
-  const float alive = lo == 0u ? 1.0f : 0.0f;
-  const float gd = (lo == 0u && ll == 0u) ? 1.0f : 0.0f;
-  a[0] += alive * pr;
-  a[1] += gd * pr; a[2] += gd * pr * pr;
-  a[3] += gd * x; a[4] += gd * x * x; a[5] += gd * y; a[6] += gd * y * y;
-  a[7] += gd * w;
 }
 
 }  // namespace

@@ -61,6 +61,7 @@ struct NoCtx {};
 struct Op32GoodPhi {
   static constexpr int K = 2;
   static constexpr bool kFast = true;
+  static constexpr int kGridPerSm = 8;
   using Comb = SumComb;
   using Ctx = NoCtx;
   DevBeam b;
@@ -85,6 +86,7 @@ struct Op32GoodPhi {
 struct Op32LlossGoodPhi {
   static constexpr int K = 3;
   static constexpr bool kFast = true;
+  static constexpr int kGridPerSm = 8;
   using Comb = SumComb;
   struct Ctx { float lim; };
   DevBeam b;
@@ -119,6 +121,7 @@ struct Op32LlossGoodPhi {
 struct Op32ScStats {
   static constexpr int K = 8;
   static constexpr bool kFast = true;
+  static constexpr int kGridPerSm = 2;
   using Comb = SumComb;
   struct Ctx { float pag; };
   DevBeam b;
@@ -162,21 +165,27 @@ struct Op32ScStats {
 //
 // One launch of clusters of kStatCluster CTAs: the whole grid takes the first
 // sweep, and the last cluster to finish takes the totals and, when the good
-// set changed, sweeps the moments again with all its threads (partial sums
-// through distributed shared memory in rank order).  Beams whose bunch
-// stretches over the whole period (a quad channel behind one buncher) lose
-// particles longitudinally at almost every kick, so the second sweep is their
-// common path: one block of 256 threads took 31 us a kick at 20,011 particles
-// (sweep phase of the quad channel, 1.26 ms over 40 kicks) and over a
-// millisecond at 524,288; a second grid-wide launch would cost its launch at
-// every kick of every beam, where this one returns at once when it is not
-// needed.  Beams of one cluster take the sums from its shared memory, and the
-// finaliser works on a staged copy of the state (20,011 particles, a set-point
-// change: 1.665 -> 1.608 ms).
+// set changed, sweeps the moments again with all its threads.  Beams whose
+// bunch stretches over the whole period (a quad channel behind one buncher)
+// lose particles longitudinally at almost every kick, so the second sweep is
+// their common path: one block of 256 threads took 31 us a kick at 20,011
+// particles and over a millisecond at 524,288; a second grid-wide launch would
+// cost its launch at every kick of every beam, where this one returns at once
+// when it is not needed.
+//
+// The sums have one order, whatever the clusters: the first sweep's that of
+// `order blocks` of 256 threads, one an SM at most, the second's that of a
+// single one (the mesh edge follows from them, and single particles at the edge
+// are kicked from either side by its last bit).  Each thread of an order block
+// adds its particles in turn, then shuffle trees, then the warps in order.  In
+// the first sweep a CTA is four groups of 256 threads: up to 155,648 particles
+// (four a thread) each has an order block, beyond that they share one.  In the
+// second a CTA has one warp of the order block's eight: its 32 warps load the
+// rounds, and warps 0-7 add one moment each, round by round.
 constexpr int kStatCluster = 8;
 constexpr int kStatThreads = 1024;
-constexpr int kStatWarps = kStatThreads / 32;
 constexpr int kStatBatch = 4;  // particles a thread has in flight
+constexpr int kStatGroups = kStatThreads / kBlock;
 
 struct StatArgs {
   DevBeam b;
@@ -195,25 +204,19 @@ __device__ __forceinline__ StatIn stat_load(const DevBeam &b, uint32_t i) {
   return {b.loss[i], b.lloss[i], b.fphi[i], b.fx[i], b.fy[i], b.fw[i]};
 }
 
-// block sums of a[0..K) into out[0..K) (shared memory): a fixed shuffle tree,
-// then the warps in order
-template <int K>
-__device__ __forceinline__ void stat_block_sum(const float (&a)[12], float (*red)[12], float *out) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    float v = a[k];
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-    if (lane == 0) red[warp][k] = v;
-  }
-  __syncthreads();
-  if (threadIdx.x < K) {
-    float v = 0.0f;
-    for (int w = 0; w < kStatWarps; ++w) v += red[w][threadIdx.x];
-    out[threadIdx.x] = v;
-  }
-  __syncthreads();
+// order blocks of the first sweep
+__host__ __device__ inline uint32_t stat_order_blocks(uint32_t n) {
+  const uint32_t b = (uint32_t)(((uint64_t)n + 4 * kBlock - 1) / (4 * kBlock));
+  return b < 1u ? 1u : b > 152u ? 152u : b;
+}
+// a term of the good set or the live set as the moments take it: the factor 0
+// or 1 keeps an infinity or NaN of a lost particle visible
+struct StatTerms {
+  float pr_live, pr, x, y, w;
+};
+__device__ __forceinline__ StatTerms stat_terms(float pr, uint32_t lo, uint32_t ll, const StatIn &p) {
+  const float alive = lo == 0u ? 1.0f : 0.0f, gd = (lo == 0u && ll == 0u) ? 1.0f : 0.0f;
+  return {alive * pr, gd * pr, gd * p.x, gd * p.y, gd * p.w};
 }
 
 // blocks [0, nblk) of the launch, whole clusters
@@ -222,57 +225,152 @@ __device__ __forceinline__ void stat_body(const StatArgs &a, uint32_t bid, uint3
   if (b.st->sc_redo != 2u) return;  // uniform over the launch: it is reset behind the last cluster's sum
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
-  __shared__ float red[kStatWarps][12];
-  __shared__ float sums[12];
+  constexpr int kWarps = kBlock / 32;
+  __shared__ float term[10][kStatThreads];        // the second sweep's five terms, in two sets
+  __shared__ float red[kStatGroups][kWarps][12];
+  __shared__ float sums[kStatGroups][12];         // of the CTA's order blocks
   __shared__ double tot[12];
   __shared__ int last, again;
   __shared__ float pag_new;
   __shared__ Sc32Stage stage;  // rank 0 of the last cluster
-  const int tid = threadIdx.x;
-  const uint32_t rank = cl.block_rank();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, grp = tid / kBlock, t = tid % kBlock, wg = t >> 5;
+  const uint32_t rank = cl.block_rank(), nord = stat_order_blocks(b.n);
+  float *partf = (float *)a.scr.part;
+  // a launch of one cluster has its sums in shared memory
+  const bool one = nblk == (uint32_t)kStatCluster;
+  auto tree = [&](float v) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+    return v;
+  };
   {
     const double pag_abs = b.st->st[PHI_AVG_GOOD];
     const float lim = (float)(pag_abs - b.phi_ref + TWOPI + PI), pag = (float)(pag_abs - b.phi_ref);
-    float s[12];
+    const uint32_t stride = nord * kBlock, rounds = (b.n + stride - 1) / stride;
+    uint32_t nll = 0, ngood = 0, nnew = 0;
+    // the loss test and the terms of particle i
+    auto take = [&](uint32_t i, const StatIn &p, float &ph) {
+      uint32_t ll = p.ll;
+      if (p.ph > lim && ll != 1u) {
+        if (p.lo == 0u && ll == 0u) ++nnew;
+        ll = 1u;
+        b.lloss[i] = 1u;
+      }
+      const float pr = rel_phase_f(p.ph - pag);
+      b.fphi_r[i] = pr;
+      const bool g = (uint32_t)(p.lo + ll) == 0u;
+      nll += ll != 0u;
+      ngood += g;
+      ph = g ? p.ph : 0.0f;
+      return stat_terms(pr, p.lo, ll, p);
+    };
+    auto count = [&](float *r) {  // a warp's counts: whole numbers, exact in any order
+      const uint32_t c0 = __reduce_add_sync(0xffffffffu, nll), c1 = __reduce_add_sync(0xffffffffu, ngood),
+                     c2 = __reduce_add_sync(0xffffffffu, nnew);
+      if (lane == 0) { r[8] = (float)c0; r[9] = (float)c1; r[11] = (float)c2; }
+    };
+    if (rounds <= (uint32_t)kStatBatch) {
+      // a group of 256 threads per order block, its rounds one after the other
+      const uint32_t vb = bid + grp * nblk;
+      float s[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f}, sph = 0.0f;
+      if (vb < nord) {
+        StatIn p[kStatBatch];
+        const uint32_t i0 = vb * kBlock + t;
 #pragma unroll
-    for (int k = 0; k < 12; ++k) s[k] = 0.0f;
-    const uint32_t stride = nblk * kStatThreads;
-    for (uint32_t base = bid * kStatThreads + tid; base < b.n; base += kStatBatch * stride) {
-      StatIn p[kStatBatch];
+        for (int u = 0; u < kStatBatch; ++u)
+          if (i0 + u * stride < b.n) p[u] = stat_load(b, i0 + u * stride);
 #pragma unroll
-      for (int u = 0; u < kStatBatch; ++u)
-        if (base + u * stride < b.n) p[u] = stat_load(b, base + u * stride);
-#pragma unroll
-      for (int u = 0; u < kStatBatch; ++u) {
-        const uint32_t i = base + u * stride;
-        if (i >= b.n) continue;
-        uint32_t ll = p[u].ll;
-        float newly = 0.0f;
-        if (p[u].ph > lim && ll != 1u) {
-          if (p[u].lo == 0u && ll == 0u) newly = 1.0f;
-          ll = 1u;
-          b.lloss[i] = 1u;
+        for (int u = 0; u < kStatBatch; ++u) {
+          if (i0 + u * stride >= b.n) continue;
+          float ph;
+          const StatTerms e = take(i0 + u * stride, p[u], ph);
+          s[0] += e.pr_live;
+          s[1] += e.pr; s[2] = fmaf(e.pr, e.pr, s[2]);
+          s[3] += e.x; s[4] = fmaf(e.x, e.x, s[4]);
+          s[5] += e.y; s[6] = fmaf(e.y, e.y, s[6]);
+          s[7] += e.w;
+          sph += ph;
         }
-        const float pr = rel_phase_f(p[u].ph - pag);
-        b.fphi_r[i] = pr;
-        sc_moments_add(s, pr, p[u].lo, ll, p[u].x, p[u].y, p[u].w);
-        const bool g = (uint32_t)(p[u].lo + ll) == 0u;
-        s[8] += ll != 0u ? 1.0f : 0.0f;
-        s[9] += g ? 1.0f : 0.0f;
-        s[10] += g ? p[u].ph : 0.0f;
-        s[11] += newly;
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const float v = tree(s[k]);
+        if (lane == 0) red[grp][wg][k] = v;
+      }
+      sph = tree(sph);
+      if (lane == 0) red[grp][wg][10] = sph;
+      count(red[grp][wg]);
+    } else {
+      // one order block, four of its rounds side by side: the groups hand each
+      // other the particles' terms, and a sum is kept by one group, which adds
+      // the rounds in order
+      float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f;  // x | y | pr | pr live, W, phi
+      auto index = [&](uint32_t r) { return (r + grp) * stride + bid * kBlock + t; };
+      for (uint32_t r0 = 0; r0 < rounds && bid < nord; r0 += kStatBatch * kStatGroups) {
+        StatIn p[kStatBatch];
+#pragma unroll
+        for (int u = 0; u < kStatBatch; ++u) {
+          const uint32_t r = r0 + u * kStatGroups, i = index(r);
+          if (r + grp < rounds && i < b.n) p[u] = stat_load(b, i);
+        }
+#pragma unroll
+        for (int u = 0; u < kStatBatch; ++u) {
+          const uint32_t r = r0 + u * kStatGroups, i = index(r);
+          if (r >= rounds) break;
+          StatTerms e = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+          float ph = 0.0f;
+          if (r + grp < rounds && i < b.n) e = take(i, p[u], ph);
+          term[0][tid] = e.pr_live; term[1][tid] = e.pr; term[2][tid] = e.x;
+          term[3][tid] = e.y; term[4][tid] = e.w; term[5][tid] = ph;
+          __syncthreads();
+          auto sum = [&](int q, float &v) {
+#pragma unroll
+            for (int j = 0; j < kStatGroups; ++j) v += term[q][j * kBlock + t];
+          };
+          auto sum2 = [&](int q) {
+#pragma unroll
+            for (int j = 0; j < kStatGroups; ++j) {
+              const float v = term[q][j * kBlock + t];
+              s0 += v;
+              s1 = fmaf(v, v, s1);
+            }
+          };
+          if (grp == 0) sum2(2);
+          else if (grp == 1) sum2(3);
+          else if (grp == 2) sum2(1);
+          else { sum(0, s0); sum(4, s1); sum(5, s2); }
+          __syncthreads();
+        }
+      }
+      const float v0 = tree(s0), v1 = tree(s1), v2 = tree(s2);
+      if (lane == 0) {
+        float *r = red[0][wg];
+        if (grp == 0) { r[3] = v0; r[4] = v1; }
+        else if (grp == 1) { r[5] = v0; r[6] = v1; }
+        else if (grp == 2) { r[1] = v0; r[2] = v1; }
+        else { r[0] = v0; r[7] = v1; r[10] = v2; }
+      }
+      count(red[grp][wg]);
+    }
+    __syncthreads();
+    // the order blocks' sums: the warps in order
+    if (tid < 12 * kStatGroups) {
+      const int g = tid / 12, k = tid % 12;
+      const bool split = rounds > (uint32_t)kStatBatch;
+      const uint32_t vb = bid + g * nblk;
+      if (vb < nord && !(split && g)) {
+        const bool counts = k == 8 || k == 9 || k == 11;
+        float v = 0.0f;
+        for (int q = 0; q < (split && counts ? kStatGroups : 1); ++q)
+          for (int w = 0; w < kWarps; ++w) v += red[g + q][w][k];
+        if (one) sums[g][k] = v;
+        else partf[(size_t)k * kMaxPassBlocks + vb] = v;
       }
     }
-    stat_block_sum<12>(s, red, sums);
   }
-  // a launch of one cluster has its blocks' sums in shared memory; else the
-  // block's partials, then one count per cluster
-  const bool one = nblk == (uint32_t)kStatCluster;
-  float *partf = (float *)a.scr.part;
   if (one) {
     cl.sync();
   } else {
-    if (tid < 12) partf[(size_t)bid * 12 + tid] = sums[tid];
     __threadfence();
     cl.sync();
     if (rank == 0 && tid == 0) {
@@ -286,20 +384,14 @@ __device__ __forceinline__ void stat_body(const StatArgs &a, uint32_t bid, uint3
     }
     __threadfence();
   }
-  // the last cluster: totals in block order, on its first CTA, with the state
-  // staged in shared memory while they arrive
+  // the last cluster: totals over the order blocks, on its first CTA, with the
+  // state staged in shared memory while they arrive
   if (rank == 0) {
-    const int lane = tid & 31, warp = tid >> 5;
     sc32_stage_load(stage, b, a.sc, tid, kStatThreads);
     if (warp < 12) {
-      float v = 0.0f;
-      if (one) {
-        if (lane < kStatCluster) v += *cl.map_shared_rank(&sums[warp], lane);
-      } else {
-        for (uint32_t k = lane; k < nblk; k += 32) v += __ldcg(partf + (size_t)k * 12 + warp);
-      }
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+      float v;
+      if (one) v = tree((uint32_t)lane < nord ? *cl.map_shared_rank(&sums[lane / kStatCluster][warp], lane % kStatCluster) : 0.0f);
+      else v = combine_slot_f<SumComb, 12>(partf, warp, nord);
       if (lane == 0) tot[warp] = (double)v;
     }
     __syncthreads();
@@ -321,33 +413,53 @@ __device__ __forceinline__ void stat_body(const StatArgs &a, uint32_t bid, uint3
   cl.sync();
   if (*cl.map_shared_rank(&again, 0)) {
     const float pag = *cl.map_shared_rank(&pag_new, 0);
-    float s[12];
-#pragma unroll
-    for (int k = 0; k < 12; ++k) s[k] = 0.0f;
-    constexpr uint32_t stride = kStatCluster * kStatThreads;
-    for (uint32_t base = rank * kStatThreads + tid; base < b.n; base += kStatBatch * stride) {
+    const uint32_t rounds = (b.n + kBlock - 1) / kBlock;
+    auto index = [&](uint32_t r) { return (r + warp) * kBlock + rank * 32 + lane; };
+    float s = 0.0f;  // of warps 0-7: moment `warp`
+    for (uint32_t r0 = 0; r0 < rounds; r0 += kStatBatch * 32) {
       StatIn p[kStatBatch];
 #pragma unroll
-      for (int u = 0; u < kStatBatch; ++u)
-        if (base + u * stride < b.n) {
-          p[u] = stat_load(b, base + u * stride);
+      for (int u = 0; u < kStatBatch; ++u) {
+        const uint32_t i = index(r0 + 32 * u);
+        if (r0 + 32 * u + warp < rounds && i < b.n) {
+          p[u] = stat_load(b, i);
           // the flags as the first sweep left them (other CTAs wrote some)
-          p[u].ll = __ldcg(b.lloss + base + u * stride);
+          p[u].ll = __ldcg(b.lloss + i);
         }
+      }
 #pragma unroll
       for (int u = 0; u < kStatBatch; ++u) {
-        const uint32_t i = base + u * stride;
-        if (i >= b.n) continue;
-        const float pr = rel_phase_f(p[u].ph - pag);
-        b.fphi_r[i] = pr;
-        sc_moments_add(s, pr, p[u].lo, p[u].ll, p[u].x, p[u].y, p[u].w);
+        const uint32_t r = r0 + 32 * u, i = index(r);
+        if (r >= rounds) break;
+        StatTerms e = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+        if (r + warp < rounds && i < b.n) {
+          const float pr = rel_phase_f(p[u].ph - pag);
+          b.fphi_r[i] = pr;
+          e = stat_terms(pr, p[u].lo, p[u].ll, p[u]);
+        }
+        // two sets: one is written again behind the next rounds' barrier
+        float (*tm)[kStatThreads] = term + 5 * (u & 1);
+        tm[0][tid] = e.pr_live; tm[1][tid] = e.pr; tm[2][tid] = e.x; tm[3][tid] = e.y; tm[4][tid] = e.w;
+        __syncthreads();
+        if (warp < 8) {
+          const float *q = tm[(warp + 1) / 2] + lane;  // 0 | 1, 1 | 2, 2 | 3, 3 | 4
+          const bool square = warp == 2 || warp == 4 || warp == 6;
+#pragma unroll
+          for (int w = 0; w < 32; ++w) {
+            const float v = q[32 * w];
+            s = square ? fmaf(v, v, s) : s + v;
+          }
+        }
       }
     }
-    stat_block_sum<8>(s, red, sums);
+    if (warp < 8) {
+      s = tree(s);
+      if (lane == 0) sums[0][warp] = s;
+    }
     cl.sync();
     if (rank == 0 && tid < 8) {
       double v = 0.0;
-      for (int c = 0; c < kStatCluster; ++c) v += (double)*cl.map_shared_rank(sums + tid, c);
+      for (int c = 0; c < kStatCluster; ++c) v += (double)*cl.map_shared_rank(&sums[0][tid], c);
       tot[tid] = v;
     }
   }
@@ -380,16 +492,18 @@ void stat_merge(const std::vector<const Rec *> &recs, SegFork &, cudaStream_t st
     k32_stat_sweeps_seg<std::decay_t<decltype(a)>::kB><<<blocks, kStatThreads, 0, st>>>(a);
   });
 }
-// whole clusters, a batch of particles per thread, at most one CTA per SM
+// whole clusters, at most one CTA per SM: four order blocks a CTA while their
+// threads have a batch of particles at most, else one
 uint32_t stat_blocks(uint32_t n) {
-  constexpr uint32_t per = kStatCluster * kStatThreads * kStatBatch;
-  const uint32_t clusters = std::min<uint32_t>(std::max<uint32_t>((n + per - 1) / per, 1u), 152u / kStatCluster);
-  return clusters * kStatCluster;
+  const uint32_t ord = stat_order_blocks(n), own = n <= ord * kBlock * kStatBatch ? kStatGroups : 1;
+  const uint32_t ctas = (ord + own - 1) / own;
+  return (ctas + kStatCluster - 1) / kStatCluster * kStatCluster;
 }
 
 struct Op32AdjMesh {
   static constexpr int K = 2;
   static constexpr bool kFast = true;
+  static constexpr int kGridPerSm = 4;
   using Comb = MaxComb;
   struct Ctx { float xa, ya, pa, pag; };
   DevBeam b;
