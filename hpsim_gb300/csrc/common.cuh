@@ -158,28 +158,33 @@ __device__ __forceinline__ float rcp_fast(float x) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
-__device__ __forceinline__ float div_fast(float x, float y) { return x * rcp_fast(y); }
+// rounded by itself: a product that the compiler may fuse into a sum behind it
+// would depend on the kernel it stands in
+__device__ __forceinline__ float div_fast(float x, float y) { return __fmul_rn(x, rcp_fast(y)); }
 
 // 1/beta_i - 1/beta_ref for a particle dw above the reference, computed from
 // beta_i^2 - beta_r^2 = (gamma_i^2 - gamma_r^2)/(gamma_i^2 gamma_r^2) so the
 // difference keeps FP32 relative precision:
 //   1/beta_i - 1/beta_r = -(dgamma (gamma_i + gamma_r)) /
 //                          (gamma_i gamma_r^2 (beta_i + beta_r) (beta gamma)_i beta_r)
-// (one division); also returns g_i = W_i/m, beta_i and (beta gamma)_i.
-__device__ inline float dinvb(float dw, const RefK &r, float &g, float &beta, float &bg) {
-  g = fmaf(dw, r.minv, r.g);
+// (one division); also returns beta_i and (beta gamma)_i.  SUM_FUSED: whether
+// beta_i is rounded before beta_r is added.
+template <bool SUM_FUSED = true>
+__device__ inline float dinvb(float dw, const RefK &r, float &beta, float &bg) {
+  const float g = fmaf(dw, r.minv, r.g);
   const float gam = g + 1.0f;
   bg = sqrt_fast(g * (g + 2.0f));
   // the denominators are products of gamma, beta and beta gamma of live
   // particles, far from zero and from overflow
   const float rg = rcp_fast(gam);
-  beta = bg * rg;
+  beta = __fmul_rn(bg, rg);
+  const float sum = SUM_FUSED ? fmaf(bg, rg, r.beta) : __fadd_rn(beta, r.beta);
   const float dg = dw * r.minv;
-  return -div_fast(dg * (gam + r.gam), gam * r.gam * r.gam * fmaf(bg, rg, r.beta) * bg * r.beta);
+  return -div_fast(dg * (gam + r.gam), gam * r.gam * r.gam * sum * bg * r.beta);
 }
 __device__ inline float dinvb(float dw, const RefK &r) {
-  float g, beta, bg;
-  return dinvb(dw, r, g, beta, bg);
+  float beta, bg;
+  return dinvb(dw, r, beta, bg);
 }
 
 // deposit weights are accumulated as integers: deterministic in any order

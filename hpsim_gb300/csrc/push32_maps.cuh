@@ -12,8 +12,11 @@
 // reference's beta.
 //
 // A map gives a particle the same bits in every sweep it runs in (alone, in a
-// run, around a kick): where two products meet in a sum, fmaf says which of
-// them is rounded, so that the choice is not the compiler's in each kernel.
+// run, around a kick, in a batch): wherever a product meets a sum, fmaf,
+// __fmul_rn or __fadd_rn says what is rounded, so that the choice is not the
+// compiler's in each kernel.  The space-charge kick behind a map takes one of
+// two fields by a comparison that particles on the mesh's edge decide either
+// way by their last bit.
 #pragma once
 
 #include "common.cuh"
@@ -52,7 +55,7 @@ struct DriftMap {
   template <class F>
   __device__ uint32_t apply(Part &p, const F &D) const {
     const float x = fmaf(p.xp, hf, p.x), y = fmaf(p.yp, hf, p.y);
-    if (aper2 != 0.0f && x * x + y * y > aper2) { p.lo = eid; return WR_LOSS; }
+    if (aper2 != 0.0f && fmaf(x, x, y * y) > aper2) { p.lo = eid; return WR_LOSS; }
     p.x = x;
     p.y = y;
     p.ph = fmaf(c, D(), p.ph);
@@ -87,10 +90,10 @@ struct QuadMap {
       // the drifted coordinates are stored, but the aperture test below sees
       // the ones before the half (the reference writes memory and tests its
       // unchanged locals)
-      p.x = x + xp * len * 0.5f;
-      p.y = y + yp * len * 0.5f;
+      p.x = fmaf(xp * len, 0.5f, x);
+      p.y = fmaf(yp * len, 0.5f, y);
       m = WR_X | WR_Y;
-      if (aper2 != 0.0f && x * x + y * y > aper2) { p.lo = eid; return m | WR_LOSS; }
+      if (aper2 != 0.0f && fmaf(x, x, y * y) > aper2) { p.lo = eid; return m | WR_LOSS; }
       p.ph = fmaf(c, D(), p.ph);
       return m | WR_PH;
     } else {
@@ -100,7 +103,7 @@ struct QuadMap {
       m = WR_X | WR_Y | WR_XP | WR_YP;
     }
     p.x = x; p.y = y; p.xp = xp; p.yp = yp;
-    if (aper2 != 0.0f && x * x + y * y > aper2) { p.lo = eid; return m | WR_LOSS; }
+    if (aper2 != 0.0f && fmaf(x, x, y * y) > aper2) { p.lo = eid; return m | WR_LOSS; }
     p.ph = fmaf(c, D(), p.ph);
     return m | WR_PH;
   }
@@ -111,14 +114,15 @@ struct QuadMap {
     const float rb = rsqrt_fast(bg);
     const float k = sk0 * rb;              // sqrt(kcoef / bg)
     const float inv_k = bg * rb * isk0;    // sqrt(bg / kcoef)
-    const float e = len * 0.25f * k - kds_r;
+    const float e = fmaf(len * 0.25f, k, -kds_r);
     const float e2 = e * e;
-    const float t1 = e * (1.0f + e2 * (1.0f / 6.0f)), t0 = e2 * (0.5f + e2 * (1.0f / 24.0f));
+    const float t1 = e * fmaf(e2, 1.0f / 6.0f, 1.0f), t01 = fmaf(e2, fmaf(e2, 1.0f / 24.0f, 0.5f), 1.0f);
     // sin(a + e) = s_r (1 - e^2/2 + e^4/24) + c_r (e - e^3/6); sinh, cosh alike
-    const float s = fmaf(c_r, e - e * e2 * (1.0f / 6.0f), s_r * (1.0f - e2 * (0.5f - e2 * (1.0f / 24.0f))));
-    const float cc = fmaf(-s_r, e - e * e2 * (1.0f / 6.0f), c_r * (1.0f - e2 * (0.5f - e2 * (1.0f / 24.0f))));
-    const float sh = fmaf(ch_r, t1, sh_r * (1.0f + t0));
-    const float ch = fmaf(sh_r, t1, ch_r * (1.0f + t0));
+    const float so = fmaf(-(e * e2), 1.0f / 6.0f, e), co = fmaf(-e2, fmaf(-e2, 1.0f / 24.0f, 0.5f), 1.0f);
+    const float s = fmaf(c_r, so, s_r * co);
+    const float cc = fmaf(-s_r, so, c_r * co);
+    const float sh = fmaf(ch_r, t1, sh_r * t01);
+    const float ch = fmaf(sh_r, t1, ch_r * t01);
     const float sovk = s * inv_k, shovk = sh * inv_k, sk = s * k, shk = sh * k;
 #pragma unroll
     for (int rep = 0; rep < 2; ++rep) {
@@ -136,8 +140,8 @@ struct QuadMap {
     if constexpr (SIGN > 0) focus(p.x, p.xp, p.y, p.yp, p.w, sl);
     else if constexpr (SIGN < 0) focus(p.y, p.yp, p.x, p.xp, p.w, sl);
     else {
-      p.x = p.x + p.xp * len * 0.5f;
-      p.y = p.y + p.yp * len * 0.5f;
+      p.x = fmaf(p.xp * len, 0.5f, p.x);
+      p.y = fmaf(p.yp * len, 0.5f, p.y);
     }
     p.ph = fmaf(c, D, p.ph);
   }
@@ -189,16 +193,26 @@ __device__ inline float fbessi0c(float x, float *m1) {
   if (ax < 3.75f) {
     float cy = x * (1.0f / 3.75f);
     cy = cy * cy;
-    const float s = cy * (3.5156229f + cy * (3.0899424f + cy * (1.2067492f + cy * (0.2659732f +
-                    cy * (0.360768e-1f + cy * 0.45813e-2f)))));
+    float s = fmaf(cy, 0.45813e-2f, 0.360768e-1f);
+    s = fmaf(cy, s, 0.2659732f);
+    s = fmaf(cy, s, 1.2067492f);
+    s = fmaf(cy, s, 3.0899424f);
+    s = fmaf(cy, s, 3.5156229f);
+    s = __fmul_rn(cy, s);
     *m1 = s;
-    return 1.0f + s;
+    return __fadd_rn(1.0f, s);
   }
   const float cy = div_fast(3.75f, ax);
-  const float ans = (expf(ax) * rsqrt_fast(ax)) * (0.39894228f + cy * (0.1328592e-1f + cy * (0.225319e-2f +
-                    cy * (-0.157565e-2f + cy * (0.916281e-2f + cy * (-0.2057706e-1f + cy * (0.2635537e-1f +
-                    cy * (-0.1647633e-1f + cy * 0.392377e-2f))))))));
-  *m1 = ans - 1.0f;
+  float ans = fmaf(cy, 0.392377e-2f, -0.1647633e-1f);
+  ans = fmaf(cy, ans, 0.2635537e-1f);
+  ans = fmaf(cy, ans, -0.2057706e-1f);
+  ans = fmaf(cy, ans, 0.916281e-2f);
+  ans = fmaf(cy, ans, -0.157565e-2f);
+  ans = fmaf(cy, ans, 0.225319e-2f);
+  ans = fmaf(cy, ans, 0.1328592e-1f);
+  ans = fmaf(cy, ans, 0.39894228f);
+  ans = __fmul_rn(expf(ax) * rsqrt_fast(ax), ans);
+  *m1 = __fadd_rn(ans, -1.0f);
   return ans;
 }
 __device__ inline float fbessi1c(float x) {
@@ -207,14 +221,24 @@ __device__ inline float fbessi1c(float x) {
   if (ax < 3.75f) {
     float cy = x * (1.0f / 3.75f);
     cy = cy * cy;
-    ans = ax * (0.5f + cy * (0.87890594f + cy * (0.51498869f + cy * (0.15084934f + cy * (0.2658733e-1f +
-          cy * (0.301532e-2f + cy * 0.32411e-3f))))));
+    ans = fmaf(cy, 0.32411e-3f, 0.301532e-2f);
+    ans = fmaf(cy, ans, 0.2658733e-1f);
+    ans = fmaf(cy, ans, 0.15084934f);
+    ans = fmaf(cy, ans, 0.51498869f);
+    ans = fmaf(cy, ans, 0.87890594f);
+    ans = fmaf(cy, ans, 0.5f);
+    ans = __fmul_rn(ax, ans);
   } else {
     const float cy = div_fast(3.75f, ax);
-    ans = 0.2282967e-1f + cy * (-0.2895312e-1f + cy * (0.1787654e-1f - cy * 0.420059e-2f));
-    ans = 0.39894228f + cy * (-0.3988024e-1f + cy * (-0.362018e-2f + cy * (0.163801e-2f + cy *
-          (-0.1031555e-1f + cy * ans))));
-    ans = ans * (expf(ax) * rsqrt_fast(ax));
+    ans = fmaf(-cy, 0.420059e-2f, 0.1787654e-1f);
+    ans = fmaf(cy, ans, -0.2895312e-1f);
+    ans = fmaf(cy, ans, 0.2282967e-1f);
+    ans = fmaf(cy, ans, -0.1031555e-1f);
+    ans = fmaf(cy, ans, 0.163801e-2f);
+    ans = fmaf(cy, ans, -0.362018e-2f);
+    ans = fmaf(cy, ans, -0.3988024e-1f);
+    ans = fmaf(cy, ans, 0.39894228f);
+    ans = __fmul_rn(ans, expf(ax) * rsqrt_fast(ax));
   }
   return x < 0.0f ? -ans : ans;
 }
@@ -239,19 +263,22 @@ struct Gap2Map {
     const Gap2Map &G = *this;
     float x = p.x, y = p.y, xp = p.xp, yp = p.yp;
     const float dphi = p.ph, dw = p.w;
-    float g, beta, bg1;
-    const float D = dinvb(dw, G.rin, g, beta, bg1);
+    float beta, bg1;
+    const float D = dinvb<false>(dw, G.rin, beta, bg1);
     // GetTransitTimeFactors (simulation_kernel.cu:290-308) about the reference's beta
     float bcl = beta;
     if (beta > 1.1f * G.fbc) bcl = G.fbc;
     else if (beta < G.fbm) bcl = G.fbm;
-    const float u = bcl - G.b0;
-    const float dT = u * (tc[1] + u * (tc[2] + u * (tc[3] + u * (tc[4] + u * tc[5]))));
-    const float t = tc[0] + dT;
-    const float dTd = tc[1] + u * (2.0f * tc[2] + u * (3.0f * tc[3] + u * (4.0f * tc[4] + 5.0f * u * tc[5])));
-    const float dSd = sc[1] + u * (2.0f * sc[2] + u * (3.0f * sc[3] + u * (4.0f * sc[4] + 5.0f * u * sc[5])));
+    const float u = __fadd_rn(bcl, -G.b0);
+    const float dT = __fmul_rn(u, fmaf(u, fmaf(u, fmaf(u, fmaf(u, tc[5], tc[4]), tc[3]), tc[2]), tc[1]));
+    const float t = __fadd_rn(tc[0], dT);
+    // the derivatives: c1 + u (2 c2 + u (3 c3 + u (4 c4 + 5 u c5)))
+    auto slope = [u](const float *c) {
+      const float d = fmaf(3.0f, c[3], u * fmaf(4.0f, c[4], 5.0f * u * c[5]));
+      return fmaf(u, fmaf(2.0f, c[2], u * d), c[1]);
+    };
     const float coef = bcl * bcl * G.inv2pifbc;
-    const float tp = coef * dTd, sp = -coef * dSd;
+    const float tp = __fmul_rn(coef, slope(tc)), sp = __fmul_rn(-coef, slope(sc));
     if (G.amp0 || (G.ccl && beta < G.fbm)) {
       p.x = fmaf(G.dd2, xp, x);
       p.y = fmaf(G.dd2, yp, y);
@@ -265,53 +292,55 @@ struct Gap2Map {
     }
     float tw, dtw;
     if (G.ccl) {
-      tw = t - F_TWOPI * tp * (div_fast(G.beta_in, beta) - 1.0f) * G.betag_ccl * G.inv_beta_in;
+      tw = fmaf(-(F_TWOPI * tp * fmaf(G.beta_in, rcp_fast(beta), -1.0f) * G.betag_ccl), G.inv_beta_in, t);
       dtw = tw - G.tw_r;
     } else {
       tw = t;
       dtw = dT;
     }
-    const float con5nex = G.concomm * (t * G.inv_fkis - G.X * tp * G.inv_gmg2);
-    const float con5nex1 = G.concomm1 * t;
+    const float con5nex = __fmul_rn(G.concomm, fmaf(t, G.inv_fkis, -(G.X * tp * G.inv_gmg2)));
+    const float con5nex1 = __fmul_rn(G.concomm1, t);
     const float con5nex2 = -G.con2nex * t * G.inv_fkis;
-    const float delta = G.ccl ? dphi - G.ccl_dg * D : dphi;
+    const float delta = G.ccl ? fmaf(-G.ccl_dg, D, dphi) : dphi;
     float sd, cd;
     fast_sincos(delta, &sd, &cd);
-    const float sinp1 = G.sinF * cd + G.cosF * sd, cosp1 = G.cosF * cd - G.sinF * sd;
-    const float prome1 = -G.con1 * (tp * (sinp1 - G.sinps) + sp * (cosp1 - G.cosps));
-    const float eps = delta + (prome1 - G.prome1_r);
+    const float sinp1 = fmaf(G.sinF, cd, G.cosF * sd), cosp1 = fmaf(G.cosF, cd, -(G.sinF * sd));
+    // the difference of the phase modulation from the reference's
+    const float dprome1 = fmaf(-G.con1, fmaf(tp, sinp1 - G.sinps, sp * (cosp1 - G.cosps)), -G.prome1_r);
+    const float eps = delta + dprome1;
     // sin and cos of eps from those of eps/2 (one evaluation instead of two;
     // 2 sin^2(eps/2) = 1 - cos(eps) is the form dcos needs anyway)
     float sh, ch;
     fast_sincos(0.5f * eps, &sh, &ch);
-    const float se = 2.0f * sh * ch, omc = 2.0f * sh * sh, ce = 1.0f - omc;
-    const float sinp = G.sinP * ce + G.cosP * se, cosp = G.cosP * ce - G.sinP * se;
-    const float dcos = -G.cosP * omc - G.sinP * se;
-    const float rs_p = x * x + y * y, rrp = x * xp + y * yp;
+    const float se = __fmul_rn(2.0f * sh, ch), omc = __fmul_rn(2.0f * sh, sh), ce = __fadd_rn(1.0f, -omc);
+    const float sinp = fmaf(G.sinP, ce, G.cosP * se), cosp = fmaf(G.cosP, ce, -(G.sinP * se));
+    const float dcos = fmaf(-G.cosP, omc, -(G.sinP * se));
+    const float rs_p = fmaf(x, x, y * y), rrp = fmaf(x, xp, y * yp);
     const float ris = sqrt_fast(rs_p), fkrris = G.fkr * ris;
     float b0m1;
     const float b0c = fbessi0c(fkrris, &b0m1);
     const float b1c = fbessi1c(fkrris);
-    const float b1p = fkrris != 0.0f ? b0c - div_fast(b1c, fkrris) : 0.5f;
+    const float b1p = fkrris != 0.0f ? fmaf(-b1c, rcp_fast(fkrris), b0c) : 0.5f;
     const float bes1covr = ris != 0.0f ? div_fast(b1c, ris) : G.fkr * 0.5f;
-    const float rest = ((tw - F_TWOPI * tp) * G.inv_gmg * bes1covr + tw * G.inv_gmg * G.fkr * b1p -
-                        tw * G.gmg * bes1covr) * rrp * sinp;
-    const float ddelte = G.q * G.efl * (tw * b0c * dcos + (dtw * b0c + G.tw_r * b0m1) * G.cosP + rest);
-    const float dwh = dw + ddelte;
-    float gh, betah, bg;
-    const float Dh = dinvb(dwh, G.rh, gh, betah, bg);
+    const float rest = fmaf(-(tw * G.gmg), bes1covr,
+                            fmaf(fmaf(-F_TWOPI, tp, tw) * G.inv_gmg, bes1covr, tw * G.inv_gmg * G.fkr * b1p));
+    const float gain = fmaf(rest * rrp, sinp,
+                            fmaf(tw * b0c, dcos, fmaf(dtw, b0c, G.tw_r * b0m1) * G.cosP));
+    const float dwh = fmaf(G.q * G.efl, gain, dw);
+    float betah, bg;
+    const float Dh = dinvb(dwh, G.rh, betah, bg);
     const float bgr = div_fast(bg1, bg);
-    const float onema = 1.0f - (con5nex * bes1covr + con5nex1 * b1p + con5nex2 * bes1covr) * cosp;
+    const float onema = fmaf(-fmaf(con5nex2, bes1covr, fmaf(con5nex1, b1p, con5nex * bes1covr)), cosp, 1.0f);
     const float dovbl = G.con2nex * bes1covr * tw * sinp;
     const float bgrovonema = div_fast(bgr, onema);
-    xp = -dovbl * x + bgrovonema * xp;
-    x = x * onema + G.dd2 * xp;
-    yp = -dovbl * y + bgrovonema * yp;
-    y = y * onema + G.dd2 * yp;
+    xp = fmaf(bgrovonema, xp, -dovbl * x);
+    x = fmaf(x, onema, G.dd2 * xp);
+    yp = fmaf(bgrovonema, yp, -dovbl * y);
+    y = fmaf(y, onema, G.dd2 * yp);
     const float rpris = rs_p > 0.0f ? div_fast(rrp, ris) : 0.0f;
-    const float prome = 2.0f * G.con1 * (-tp * b0c + ris * tw * b1c * G.inv_gmgcl) * (sinp - G.sinps) -
-                        G.efl_m * tw * b1c * rpris * (cosp - G.cosps);
-    const float dphih = dphi + G.K2 * Dh + (prome - G.prome_r);
+    const float mod = fmaf(ris * tw * b1c, G.inv_gmgcl, -tp * b0c);
+    const float prome = fmaf(2.0f * G.con1 * mod, sinp - G.sinps, -(G.efl_m * tw * b1c * rpris * (cosp - G.cosps)));
+    const float dphih = fmaf(G.K2, Dh, dphi) + (prome - G.prome_r);
     const float wabs = G.rh.w + dwh;
     if (wabs <= 0.0f || x != x || y != y || xp != xp || yp != yp || dwh != dwh || dphih != dphih) {
       p.lo = 33333333u;
@@ -340,9 +369,9 @@ struct BunchMap {
     const float sh = sinf(0.5f * delta);
     const float dcos = fmaf(-cosB * 2.0f * sh, sh, -(sinB * sd));
     const float arg = k2q * r2;
-    const float poly = arg * (1.0f + arg * (0.25f + arg / 36.0f));
-    const float dwi = qV * cosph * (1.0f + poly);
-        const float w = r.w + dw;
+    const float poly = __fmul_rn(arg, fmaf(arg, 0.25f + arg / 36.0f, 1.0f));
+    const float dwi = qV * cosph * __fadd_rn(1.0f, poly);
+    const float w = r.w + dw;
     const float wb_par = fmaf(0.5f, dwi, w), wf = __fadd_rn(w, dwi);
     if (wb_par <= 0.0f || wf <= 0.0f) { p.lo = eid; return WR_LOSS; }
     float gt = wb_par * r.minv;
@@ -351,7 +380,7 @@ struct BunchMap {
     const float bg = sqrtf(gt * (gt + 2.0f));
     gt = wf * r.minv;
     const float rbgf = rsqrtf(gt * (gt + 2.0f));
-    const float del = -con1 * sinph * (1.0f - bav * beta_w) * (0.5f + arg * (0.25f + arg / 24.0f)) / bav;
+    const float del = -con1 * sinph * fmaf(-bav, beta_w, 1.0f) * fmaf(arg, 0.25f + arg / 24.0f, 0.5f) / bav;
     p.xp = fmaf(p.xp, bg, del * x) * rbgf;
     p.yp = fmaf(p.yp, bg, del * y) * rbgf;
     p.w = fmaf(qV, fmaf(cosph, poly, dcos), dw);
@@ -364,10 +393,10 @@ struct RotMap {
   float cosa, sina;
   __device__ uint32_t apply(Part &p) const {
     const float x = p.x, y = p.y, xp = p.xp, yp = p.yp;
-    p.x = x * cosa + y * sina;
-    p.y = y * cosa - x * sina;
-    p.xp = xp * cosa + yp * sina;
-    p.yp = yp * cosa - xp * sina;
+    p.x = fmaf(x, cosa, y * sina);
+    p.y = fmaf(y, cosa, -(x * sina));
+    p.xp = fmaf(xp, cosa, yp * sina);
+    p.yp = fmaf(yp, cosa, -(xp * sina));
     return WR_X | WR_Y | WR_XP | WR_YP;
   }
 };
@@ -379,26 +408,25 @@ struct DipMap {
   int second;
   __device__ uint32_t apply(Part &p) const {
     float x = p.x, xp = p.xp, y = p.y, yp = p.yp;
-    const float ddp = cdp * p.w;
-    const float dpop = dpop_ref + ddp;
+    const float ddp = __fmul_rn(cdp, p.w);
+    const float dpop = __fadd_rn(dpop_ref, ddp);
+    // a u + b v, and a u + b v + c w
+    auto two = [](float a, float u, float b, float v) { return fmaf(a, u, b * v); };
+    auto three = [](float a, float u, float b, float v, float c, float w) { return fmaf(c, w, fmaf(a, u, b * v)); };
     if (!second) {
-      xp += e21 * x;
-      yp -= e43 * y;
-      p.x = r11 * x + r12 * xp + r16 * dpop;
-      p.xp = r21 * x + r22 * xp + r26 * dpop;
-      p.y = r33 * y + r34 * yp;
-      p.yp = r43 * y + r44 * yp;
-      p.ph -= cph * (r51 * x + r52 * xp + r56 * ddp);
+      xp = fmaf(e21, x, xp);
+      yp = fmaf(-e43, y, yp);
+      p.x = three(r11, x, r12, xp, r16, dpop);
+      p.xp = three(r21, x, r22, xp, r26, dpop);
+      p.y = two(r33, y, r34, yp);
+      p.yp = two(r43, y, r44, yp);
+      p.ph = fmaf(-cph, three(r51, x, r52, xp, r56, ddp), p.ph);
     } else {
-      p.ph -= cph * (r51 * x + r52 * xp + r56 * ddp);
-      const float xn = r11 * x + r12 * xp + r16 * dpop;
-      xp = r21 * x + r22 * xp + r26 * dpop;
-      const float yn = r33 * y + r34 * yp;
-      yp = r43 * y + r44 * yp;
-      p.x = xn;
-      p.y = yn;
-      p.xp = xp + e21 * xn;
-      p.yp = yp - e43 * yn;
+      p.ph = fmaf(-cph, three(r51, x, r52, xp, r56, ddp), p.ph);
+      p.x = three(r11, x, r12, xp, r16, dpop);
+      p.y = two(r33, y, r34, yp);
+      p.xp = fmaf(e21, p.x, three(r21, x, r22, xp, r26, dpop));
+      p.yp = fmaf(-e43, p.y, two(r43, y, r44, yp));
     }
     return WR_X | WR_Y | WR_XP | WR_YP | WR_PH;
   }

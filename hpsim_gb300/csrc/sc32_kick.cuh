@@ -56,13 +56,14 @@ __device__ inline float wrap_turns(float d) {
 // phi; returns the fields changed.  Quotients whose denominators are
 // bounded away from zero and overflow use the two-ulp reciprocal-multiply
 // (div_fast), the square roots of the common path the hardware
-// approximation (sqrt_fast).
+// approximation (sqrt_fast).  The same bits in every kernel, as the element
+// maps (push32_maps.cuh).
 __device__ inline uint32_t kick_particle(Part &p, float phi, const KickEnv &e) {
   const float dw = p.w;
   const float g = fmaf(dw, e.r.minv, e.r.g);
   const float gm = g + 1.0f;
   const float bgz = sqrt_fast(g * (g + 2.0f));
-    const float dgc = (dw + e.dwc) * e.r.minv;  // gm - gamma_c
+  const float dgc = (dw + e.dwc) * e.r.minv;  // gm - gamma_c
   const float s0 = div_fast(dgc * (gm + e.gmg), e.gmg * fmaf(e.beta, gm, bgz));
   const float xxbar = p.x - e.xbar, yybar = p.y - e.ybar;
   float rr = sqrt_fast(fmaf(xxbar * xxbar, e.inv_epsq, yybar * yybar * e.epsq));
@@ -72,18 +73,18 @@ __device__ inline uint32_t kick_particle(Part &p, float phi, const KickEnv &e) {
   float z = __fmul_rn(-e.c2, wrap_turns(phi - e.phimc));
   float cbgr, cbgzs;
   if (rr > e.rmesh || fabsf(z) > e.hl) {
-    z = -e.c2 * (phi - e.phimc);
+    z = __fmul_rn(-e.c2, phi - e.phimc);
     float d = sqrtf(fmaf(z, z, rr * rr));
     float invd3 = 1.0f / (d * d * d);
     float rod3 = rr * invd3, zod3 = z * invd3;
     for (uint32_t nb = 1; nb <= e.adj; ++nb) {
       float xi = (float)nb;
       for (int lr = 0; lr < 2; ++lr) {
-        const float sft = z + xi * e.pl;
+        const float sft = fmaf(xi, e.pl, z);
         d = sqrtf(fmaf(sft, sft, rr * rr));
         invd3 = 1.0f / (d * d * d);
-        rod3 += rr * invd3;
-        zod3 += sft * invd3;
+        rod3 = fmaf(rr, invd3, rod3);
+        zod3 = fmaf(sft, invd3, zod3);
         xi = -xi;
       }
     }
@@ -107,7 +108,6 @@ __device__ inline uint32_t kick_particle(Part &p, float phi, const KickEnv &e) {
     cbgr = e.er_c3 * fmaf(d, fmaf(a, fl.x, bb * fl1.x), c * fmaf(a, fm.x, bb * fm1.x));
     cbgzs = e.ez_c3 * fmaf(d, fmaf(a, fl.y, bb * fl1.y), c * fmaf(a, fm.y, bb * fm1.y));
   }
-  // the same bits in every kernel, as the element maps (push32_maps.cuh)
   const float bgx = fmaf(bgz, p.xp, cbgr * xovr), bgy = fmaf(bgz, p.yp, cbgr * yovr);
   // bgzf = gamma_c (p* + dp + beta_c (1 + (p* + dp)^2 / 2)) taken as
   // bgz + (bgzf - bgz): the change is formed without cancellation and bgz
