@@ -139,11 +139,19 @@ __host__ __device__ inline RefK make_refk(double w, double mass) {
 
 // Square roots, reciprocal square roots and reciprocals by the hardware
 // approximations (within two ulp), and the quotient they give, for the
-// per-particle sweeps.  The .ftz forms take subnormal operands and results as
-// zero: quantities below 1e-38 of the coordinates' own units.  The other forms
-// scale their operands around every approximation, three to four more
-// instructions each in sweeps that are bound by their instructions.
+// per-particle sweeps.  sqrt_fast takes every operand: a sum of squared
+// coordinates is subnormal where the coordinates are not (a particle 1e-20 m
+// off the axis), and a root of zero there would make the quotient behind it
+// infinite.  The .ftz forms take subnormal operands and results as zero and
+// spare the scaling around the approximation, three to four instructions each
+// in sweeps that are bound by their instructions; they are for operands that
+// are never subnormal: energies, momenta and what is divided by them.
 __device__ __forceinline__ float sqrt_fast(float x) {
+  float r;
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float sqrt_norm(float x) {
   float r;
   asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
@@ -173,7 +181,7 @@ template <bool SUM_FUSED = true>
 __device__ inline float dinvb(float dw, const RefK &r, float &beta, float &bg) {
   const float g = fmaf(dw, r.minv, r.g);
   const float gam = g + 1.0f;
-  bg = sqrt_fast(g * (g + 2.0f));
+  bg = sqrt_norm(g * (g + 2.0f));
   // the denominators are products of gamma, beta and beta gamma of live
   // particles, far from zero and from overflow
   const float rg = rcp_fast(gam);

@@ -110,7 +110,7 @@ struct QuadMap {
   // the half's two steps: u is the focusing plane, v the other; sl = 1 + x'^2 + y'^2
   __device__ void focus(float &u, float &up, float &v, float &vp, float w, float sl) const {
     const float g = fmaf(w, r.minv, r.g);
-    const float bg = sqrt_fast(g * (g + 2.0f) * sl);
+    const float bg = sqrt_norm(g * (g + 2.0f) * sl);
     const float rb = rsqrt_fast(bg);
     const float k = sk0 * rb;              // sqrt(kcoef / bg)
     const float inv_k = bg * rb * isk0;    // sqrt(bg / kcoef)

@@ -56,13 +56,13 @@ __device__ inline float wrap_turns(float d) {
 // phi; returns the fields changed.  Quotients whose denominators are
 // bounded away from zero and overflow use the two-ulp reciprocal-multiply
 // (div_fast), the square roots of the common path the hardware
-// approximation (sqrt_fast).  The same bits in every kernel, as the element
-// maps (push32_maps.cuh).
+// approximation (sqrt_norm for energies, sqrt_fast for the radius).  The same
+// bits in every kernel, as the element maps (push32_maps.cuh).
 __device__ inline uint32_t kick_particle(Part &p, float phi, const KickEnv &e) {
   const float dw = p.w;
   const float g = fmaf(dw, e.r.minv, e.r.g);
   const float gm = g + 1.0f;
-  const float bgz = sqrt_fast(g * (g + 2.0f));
+  const float bgz = sqrt_norm(g * (g + 2.0f));
   const float dgc = (dw + e.dwc) * e.r.minv;  // gm - gamma_c
   const float s0 = div_fast(dgc * (gm + e.gmg), e.gmg * fmaf(e.beta, gm, bgz));
   const float xxbar = p.x - e.xbar, yybar = p.y - e.ybar;
@@ -116,7 +116,7 @@ __device__ inline uint32_t kick_particle(Part &p, float phi, const KickEnv &e) {
   const float dbgz =
       e.gmg * fmaf(e.beta,
                    fmaf(0.5f * cbgzs, fmaf(2.0f, s0, cbgzs),
-                        div_fast(s2 * s2, 4.0f * (fmaf(0.5f, s2, 1.0f) + sqrt_fast(1.0f + s2)))),
+                        div_fast(s2 * s2, 4.0f * (fmaf(0.5f, s2, 1.0f) + sqrt_norm(1.0f + s2)))),
                    cbgzs);
   const float bgzf = __fadd_rn(bgz, dbgz);
   if (bgzf <= 0.0f) {
