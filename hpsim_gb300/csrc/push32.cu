@@ -118,7 +118,7 @@ template <> constexpr MapKind map_kind<DipMap>() { return MAP_DIP; }
 // a map of a run; drift, quad and gap1 begin with the synchronous particle r
 struct RunRec {
   MapKind kind;
-  uint16_t same;   // the energies and the synchronous particle are the previous map's
+  uint16_t same;   // the energies and the synchronous particle are those of the last drift, quad or gap1
   uint16_t loses;  // it may lose a particle
   Shift sh;
   union {
@@ -753,7 +753,13 @@ void launch_run_chunk(const PushQueue &q, size_t k0, size_t n) {
     a.m[j] = q.run[k0 + j];
     a.fields |= map_fields(q.run[k0 + j].kind);
   }
-  a.m[0].same = 0;  // the launch's first map takes the energies afresh
+  // the launch's first map that needs the energies takes them afresh, whatever
+  // stands before it (a steerer, a rotation, a dipole's half)
+  for (size_t j = 0; j < n; ++j) {
+    if (a.m[j].kind > MAP_GAP1) continue;
+    a.m[j].same = 0;
+    break;
+  }
   k32_run<R, B><<<sweep_grid((const void *)k32_run<R, B>, a.b.n, a.b.sweep_cap, kRunBatch), kBlock, 0, q.run_st>>>(a);
   note_launch();
 }
