@@ -115,14 +115,12 @@ __global__ void __launch_bounds__(kSurBlock) k_sur_input(ScState *sc, ScTables t
   }
   __syncthreads();
   if (threadIdx.x == 0) red[0] = a;
-  // the network's inputs are BF16 and FP32 numbers: FP32 arithmetic (in FP64 a
-  // dependent quotient costs a third of a microsecond, a logarithm one); the
-  // field's scale stays FP64
-  if (!fp32 && threadIdx.x == 0) {
-    const float b2 = (float)sc->beta * (float)sc->beta;
-    qs = a ? (float)nb / (float)(long long)a : 0.0f;
-    la = __float2bfloat16_rn(logf((float)sc->dz * rsqrtf(1.0f - b2) / (float)sc->dr));
-  }
+  // an FP64 beam's inputs are formed in FP64 (1 - beta^2 in FP32 is off by
+  // 1e-7 gamma^2) and rounded once; the charge's scale, the field's and the
+  // logarithm on a warp each, as each is a microsecond's chain of FP64
+  if (!fp32 && threadIdx.x == 0) qs = a ? (float)((double)nb / (double)(long long)a) : 0.0f;
+  if (!fp32 && threadIdx.x == 64)
+    la = __float2bfloat16_rn((float)log(sc->dz * rsqrt(1.0 - sc->beta * sc->beta) / sc->dr));
   if (!fp32 && threadIdx.x == 32 && blockIdx.x == 0) {
     const double dzg = sc->dz * rsqrt(1.0 - sc->beta * sc->beta), total = (double)(long long)a * kBinInvScale;
     sd->active = total > 0.0;
