@@ -111,7 +111,7 @@ __global__ void k_half_quad(DevBeam b, double len, double aper, double qg, doubl
       const double bg = sqrt(g2 * (1.0 + xp * xp + yp * yp)), rb = rsqrt(bg);
       const double k = sk0 * rb, inv_k = isk0 * (bg * rb), kds = len * 0.25 * k;
       double s, c, sh, ch;
-      if (kds < 0.75) trig_small(kds, &s, &c, &sh, &ch);
+      if (fabs(kds) < 0.75) trig_small(kds, &s, &c, &sh, &ch);
       else {
         sincos(kds, &s, &c);
         sh = sinh(kds);
