@@ -256,10 +256,9 @@ ALG_BYTES = {
 # coordinates plus both loss flags read (2 * 6 * s + 8 bytes).
 STEP_BYTES = {"fp32": 56, "fp64": 104}
 PHASE_KERNELS = {
-    "fp32": {"quad": "pass_kernel_f<OpPushScStats<QuadMap>>", "gap1": "pass_kernel_f<OpPushScStats<Gap1Map>>",
-             "drift": "pass_kernel_f<OpPushScStats<DriftMap>>",
-             "sc_stats": "pass_kernel_f<Op32LlossScStats> (returns at once when the sweep before the kick "
-                         "certified its statistics)",
+    "fp32": {"quad": "k32_sweep<OpPushScStats<QuadMap>>", "gap1": "k32_sweep<OpPushScStats<Gap1Map>>",
+             "drift": "k32_sweep<OpPushScStats<DriftMap>>",
+             "sc_stats": "k32_stat_sweeps (returns at once when the sweep before the kick certified its statistics)",
              "sc_mesh": "k32_green + k32_green_deposit + k_contract_m | k_contract_tc + k_tc_reduce", "sc_kick": "k32_kick_push<QuadMap|Gap2Map|DriftMap>"},
     "fp64": {},
 }

@@ -31,8 +31,7 @@ struct BeamStats {
   double st[NSTAT];
   uint32_t num_loss, num_lloss, num_good;
   // FP32 beams, SCHEFF statistics fused into the element map before a kick:
-  // 0 done; 2 the loss test and the moments sweep still have to run; 1 the
-  // loss test changed the good set and the moments sweep runs again
+  // 0 done; 2 the loss test and the moments still have to be swept
   uint32_t sc_redo;
 };
 
@@ -49,8 +48,8 @@ struct DevBeam {
   // particle the offsets fphi, fw are taken from.  Tracked on the host in
   // FP64 through the same element formulas (on axis) and passed by value.
   double phi_ref, w_ref;
-  // launch shape of the FP32 particle sweeps and statistics passes: at most
-  // this many blocks per SM (0: as many as the SM holds at once)
+  // launch shape of the FP32 particle sweeps: at most this many blocks per SM
+  // (0: as many as the SM holds at once)
   uint32_t sweep_cap;
   uint32_t in_batch;  // the range shares the GPU with other beams' ranges
 };

@@ -166,9 +166,9 @@ int sur_conv_state(const SurNet &n, int *tc_layers, unsigned int *err);
 
 // ---- FP32 beams (push32.cu, beam32.cu, scheff32.cu) ----------------------
 // the statistics after a PUSH_SCSTATS map that could not certify its own:
-// the longitudinal-loss test and the SCHEFF moments in one sweep, repeated
-// only when the test flagged a particle (the good set, hence <phi>_good,
-// changed).  Both sweeps return at once when they are not needed.
+// the longitudinal-loss test and the SCHEFF moments, the moments again when
+// the test flagged a particle (the good set, hence <phi>_good, changed), in one
+// launch that returns at once when it is not needed
 void sc32_stats_after_push(const DevBeam &b, ScState *sc, const ScTables &t, const ScKickArgs &a,
                            PassScratch s, cudaStream_t st);
 // What an element map runs with:

@@ -196,11 +196,6 @@ inline void launch_pass(const Op &op, uint32_t n, PassScratch scr, cudaStream_t 
 // batch is in flight before the first store.
 constexpr int kPassBatch = 4;
 template <int K> constexpr int pass_batch() { return K > 10 ? 2 : kPassBatch; }
-// an Op may set its own batch (`static constexpr int kBatch`)
-template <class Op, class = void>
-struct op_batch : std::integral_constant<int, pass_batch<Op::K>()> {};
-template <class Op>
-struct op_batch<Op, std::void_t<decltype(Op::kBatch)>> : std::integral_constant<int, Op::kBatch> {};
 
 // An Op with `static constexpr bool kFast = true` has its block and grid
 // partials combined in FP32 (counts stay exact below 2^24 particles); the
@@ -211,13 +206,6 @@ struct op_fast : std::false_type {};
 template <class Op>
 struct op_fast<Op, std::void_t<decltype(Op::kFast)>> : std::integral_constant<bool, Op::kFast> {};
 
-// An Op with `static constexpr int kMaxFrom = m` (fast combine only) takes
-// the maximum, not the sum, of accumulators m .. K-1; they start at -inf.
-template <class Op, class = void>
-struct op_max_from : std::integral_constant<int, Op::K> {};
-template <class Op>
-struct op_max_from<Op, std::void_t<decltype(Op::kMaxFrom)>> : std::integral_constant<int, Op::kMaxFrom> {};
-
 // An Op with kFast fixes its blocks per SM (`static constexpr int kGridPerSm`):
 // the order of its sums follows from the number of blocks, and must not change
 // with the registers that a compiler gives the kernel.
@@ -226,19 +214,16 @@ struct op_grid_per_sm : std::integral_constant<int, 2> {};
 template <class Op>
 struct op_grid_per_sm<Op, std::void_t<decltype(Op::kGridPerSm)>> : std::integral_constant<int, Op::kGridPerSm> {};
 
-template <class C, int MF>
-__device__ inline float comb_k(int k, float a, float b) {
-  return k >= MF ? fmaxf(a, b) : C::comb(a, b);
-}
-
 // Slot k's total over the FP32 partials of nblk blocks, taken by a warp: lane l
 // sums blocks l, l + 32, ... (eight loads in flight), then a fixed shuffle tree
-// (lane 0 has the result).  Partials lie slot by slot, kMaxPassBlocks apart.
+// (lane 0 has the result).  Slots from MF on hold maxima of any sign.  Partials
+// lie slot by slot, kMaxPassBlocks apart.
 template <class C, int MF>
 __device__ __forceinline__ float combine_slot_f(const float *part, int k, uint32_t nblk) {
   const int lane = threadIdx.x & 31;
   const float *p = part + (size_t)k * kMaxPassBlocks;
   float v = k >= MF ? -INFINITY : 0.0f;
+  auto comb = [k](float a, float b) { return k >= MF ? fmaxf(a, b) : (float)C::comb(a, b); };
   for (uint32_t b = lane; b < nblk; b += 8 * 32) {
     float r[8];
 #pragma unroll
@@ -246,10 +231,10 @@ __device__ __forceinline__ float combine_slot_f(const float *part, int k, uint32
       if (b + 32 * u < nblk) r[u] = __ldcg(p + b + 32 * u);
 #pragma unroll
     for (int u = 0; u < 8; ++u)
-      if (b + 32 * u < nblk) v = comb_k<C, MF>(k, v, r[u]);
+      if (b + 32 * u < nblk) v = comb(v, r[u]);
   }
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) v = comb_k<C, MF>(k, v, __shfl_down_sync(0xffffffffu, v, off));
+  for (int off = 16; off > 0; off >>= 1) v = comb(v, __shfl_down_sync(0xffffffffu, v, off));
   return v;
 }
 
@@ -257,7 +242,7 @@ __device__ __forceinline__ float combine_slot_f(const float *part, int k, uint32
 template <class Op>
 __device__ __forceinline__ void pass_body_f(const Op &op, uint32_t n, PassScratch scr, uint32_t bid, uint32_t nblk) {
   constexpr int K = Op::K;
-  constexpr int B = op_batch<Op>::value;
+  constexpr int B = pass_batch<K>();
   using C = typename Op::Comb;
   if (!op.enabled()) return;
   __shared__ double tot[K];
@@ -266,11 +251,9 @@ __device__ __forceinline__ void pass_body_f(const Op &op, uint32_t n, PassScratc
   if (threadIdx.x == 0) sctx = op.setup();
   __syncthreads();
   const typename Op::Ctx ctx = sctx;
-  constexpr int MF = op_max_from<Op>::value;
-  static_assert(MF == K || op_fast<Op>::value, "max slots need the FP32 combine");
   float acc[K];
 #pragma unroll
-  for (int k = 0; k < K; ++k) acc[k] = k >= MF ? -INFINITY : 0.0f;
+  for (int k = 0; k < K; ++k) acc[k] = 0.0f;
   const uint32_t stride = nblk * blockDim.x;
   for (uint32_t base = bid * blockDim.x + threadIdx.x; base < n; base += B * stride) {
     typename Op::P p[B];
@@ -297,14 +280,14 @@ __device__ __forceinline__ void pass_body_f(const Op &op, uint32_t n, PassScratc
     for (int k = 0; k < K; ++k) {
       float v = acc[k];
 #pragma unroll
-      for (int off = 16; off > 0; off >>= 1) v = comb_k<C, MF>(k, v, __shfl_down_sync(0xffffffffu, v, off));
+      for (int off = 16; off > 0; off >>= 1) v = C::comb(v, __shfl_down_sync(0xffffffffu, v, off));
       if (lane == 0) smf[warp][k] = v;
     }
     __syncthreads();
     if (threadIdx.x < K) {
       const int k = threadIdx.x;
-      float v = k >= MF ? -INFINITY : 0.0f;
-      for (int w = 0; w < kBlock / 32; ++w) v = comb_k<C, MF>(k, v, smf[w][k]);
+      float v = 0.0f;
+      for (int w = 0; w < kBlock / 32; ++w) v = C::comb(v, smf[w][k]);
       partf[(size_t)k * kMaxPassBlocks + bid] = v;
     }
     __threadfence();
@@ -314,7 +297,7 @@ __device__ __forceinline__ void pass_body_f(const Op &op, uint32_t n, PassScratc
     if (!is_last) return;
     __threadfence();
     for (int k = warp; k < K; k += kBlock / 32) {
-      const float v = combine_slot_f<C, MF>(partf, k, nblk);
+      const float v = combine_slot_f<C, K>(partf, k, nblk);
       if (lane == 0) tot[k] = (double)v;
     }
     __syncthreads();

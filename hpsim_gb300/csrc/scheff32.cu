@@ -114,10 +114,8 @@ struct Op32LlossGoodPhi {
   }
 };
 
-// accumulate particle p into the SCHEFF moments (pr: its relative phase)
 // relative phase about <phi>_good, the SCHEFF moments, the decision and the
-// kick's constants (as OpScStats in scheff.cu).  With redo_only it runs only
-// when the loss-test sweep below changed the good set (sc_redo == 1).
+// kick's constants (as OpScStats in scheff.cu)
 struct Op32ScStats {
   static constexpr int K = 8;
   static constexpr bool kFast = true;
@@ -129,8 +127,7 @@ struct Op32ScStats {
   ScTables t;
   double freq, frac;
   Sc32Host h;
-  int redo_only;
-  __device__ bool enabled() const { return !redo_only || b.st->sc_redo == 1u; }
+  __device__ bool enabled() const { return true; }
   __device__ Ctx setup() const { return {(float)(b.st->st[PHI_AVG_GOOD] - b.phi_ref)}; }
   struct P { uint32_t lo, ll; float ph, x, y, w; };
   __device__ P load(uint32_t i) const { return {b.loss[i], b.lloss[i], b.fphi[i], b.fx[i], b.fy[i], b.fw[i]}; }
@@ -894,7 +891,7 @@ void beam32_update_stat_for_sc(const DevBeam &b, PassScratch s, cudaStream_t st)
   if (b.n <= 2) return;
   launch_pass_f(Op32GoodPhi{b}, b.n, s, st);
   launch_pass_f(Op32LlossGoodPhi{b}, b.n, s, st);
-  launch_pass_f(Op32ScStats{b, nullptr, ScTables{}, 0.0, 0.0, Sc32Host{}, 0}, b.n, s, st);
+  launch_pass_f(Op32ScStats{b, nullptr, ScTables{}, 0.0, 0.0, Sc32Host{}}, b.n, s, st);
   note_launch(3);
 }
 
@@ -920,7 +917,7 @@ void sc32_stats(const DevBeam &b, ScState *sc, const ScTables &t, const ScKickAr
   if (a.stats_ok) {
     launch_pass_f(Op32GoodPhi{b}, b.n, s, st);
     launch_pass_f(Op32LlossGoodPhi{b}, b.n, s, st);
-    launch_pass_f(Op32ScStats{b, sc, u, a.freq, a.frac, h, 0}, b.n, s, st);
+    launch_pass_f(Op32ScStats{b, sc, u, a.freq, a.frac, h}, b.n, s, st);
     note_launch(3);
   } else {
     launch_k(k32_decide_only, dim3(1), dim3(kBlock), 0, st, b, sc, u, a.freq, a.frac, h);
@@ -994,7 +991,9 @@ void sc32_mesh(const DevBeam &b, ScState *sc, const ScTables &t, const ScKickArg
     // the Green's table on the side stream, beside the deposit: it needs no
     // shared memory, so its blocks take the warp slots the deposit's
     // shared-memory histograms leave free (in one launch they would queue
-    // behind the deposit blocks, which size every block's shared memory)
+    // behind the deposit blocks, which size every block's shared memory).  At
+    // 64 x 256 its 608 blocks fill the register files first, and the deposit's
+    // clusters start when it is nearly through (13.7 us).
     const uint32_t ng = 4u * ngreen;
     cudaEventRecord(fork->ev_fork, st);
     cudaStreamWaitEvent(fork->side, fork->ev_fork, 0);

@@ -276,7 +276,10 @@ hps_status hps_sim_set_space_charge(hps_sim_t sim, int on);
 /* per-element monitor records: host array of capacity * HPS_NMON doubles,
  * filled for every simulated element (NULL disables). */
 hps_status hps_sim_set_monitor(hps_sim_t sim, double *host_out, uint32_t capacity);
-/* capture each simulate() range into a CUDA graph and replay it (default on) */
+/* CUDA graphs (default on): a simulate() range is launched kernel by kernel the
+ * first time its inputs are seen, captured into a graph the second time and
+ * replayed from then on while they stay the same; off: launched kernel by
+ * kernel every time.  The results are the same bits. */
 hps_status hps_sim_use_graph(hps_sim_t sim, int on);
 /* wait for the simulator's stream */
 hps_status hps_sim_synchronize(hps_sim_t sim);
@@ -286,7 +289,11 @@ hps_status hps_sim_last_time_ms(hps_sim_t sim, double *ms);
  * Simulate, src/util/src/timer.cpp:4-18, broken down by phase).  While on,
  * simulate() issues launches directly (no graph) with an event pair around
  * every phase; hps_sim_profile_read returns the accumulated milliseconds and
- * phase counts per HPS_PROF_* class. */
+ * phase counts per HPS_PROF_* class.  FP32 beams: every element map is then a
+ * launch of its own, where a pass without the timers runs maps with nothing
+ * between them as one sweep, and a kick, the half behind it and the next
+ * element's half as another.  So the phases show where the time goes, and
+ * their sum is above such a pass's; the results are the same bits. */
 #define HPS_PROF_DRIFT 0     /* partial drifts */
 #define HPS_PROF_QUAD 1      /* half quads */
 #define HPS_PROF_GAP1 2      /* RF gap first halves */
@@ -345,8 +352,8 @@ hps_status hps_batch_last_mode(hps_batch_t batch, int *lockstep, char *why, size
  * 1024; 0 reads as 256)}.  hps_sim_autotune times candidate shapes on the
  * simulator's own simulate(start, end) with CUDA events (coordinate descent
  * over the knobs, the deposit's block size and blocks per SM together; each
- * candidate the median of `reps` runs
- * after an untimed one that captures its graph; every run starts from a
+ * candidate the median of `reps` runs after two untimed ones, the second of
+ * which captures its graph; every run starts from a
  * snapshot of the beam, solver and engine state, which is restored at the
  * end), keeps the fastest and caches it per (device, mesh, power-of-two
  * particle-count bucket, precision): a later call with the same key applies
