@@ -103,7 +103,7 @@ struct QuadMap {
       m = WR_X | WR_Y | WR_XP | WR_YP;
     }
     p.x = x; p.y = y; p.xp = xp; p.yp = yp;
-    if (aper2 != 0.0f && fmaf(x, x, y * y) > aper2) { p.lo = eid; return m | WR_LOSS; }
+    if (aper2 != 0.0f && fmaf(y, y, x * x) > aper2) { p.lo = eid; return m | WR_LOSS; }
     p.ph = fmaf(c, D(), p.ph);
     return m | WR_PH;
   }
@@ -273,12 +273,15 @@ struct Gap2Map {
     const float dT = __fmul_rn(u, fmaf(u, fmaf(u, fmaf(u, fmaf(u, tc[5], tc[4]), tc[3]), tc[2]), tc[1]));
     const float t = __fadd_rn(tc[0], dT);
     // the derivatives: c1 + u (2 c2 + u (3 c3 + u (4 c4 + 5 u c5)))
-    auto slope = [u](const float *c) {
-      const float d = fmaf(3.0f, c[3], u * fmaf(4.0f, c[4], 5.0f * u * c[5]));
-      return fmaf(u, fmaf(2.0f, c[2], u * d), c[1]);
-    };
+    const float u5 = 5.0f * u;
+    float dTd = fmaf(4.0f, tc[4], __fmul_rn(u5, tc[5]));
+    dTd = fmaf(3.0f, tc[3], __fmul_rn(u, dTd));
+    dTd = fmaf(u, fmaf(2.0f, tc[2], __fmul_rn(u, dTd)), tc[1]);
+    float dSd = fmaf(u5, sc[5], __fmul_rn(4.0f, sc[4]));
+    dSd = fmaf(u, dSd, __fmul_rn(3.0f, sc[3]));
+    dSd = fmaf(u, fmaf(u, dSd, __fmul_rn(2.0f, sc[2])), sc[1]);
     const float coef = bcl * bcl * G.inv2pifbc;
-    const float tp = __fmul_rn(coef, slope(tc)), sp = __fmul_rn(-coef, slope(sc));
+    const float tp = __fmul_rn(coef, dTd), sp = __fmul_rn(-coef, dSd);
     if (G.amp0 || (G.ccl && beta < G.fbm)) {
       p.x = fmaf(G.dd2, xp, x);
       p.y = fmaf(G.dd2, yp, y);
