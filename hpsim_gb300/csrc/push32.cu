@@ -487,7 +487,10 @@ __device__ __forceinline__ void sweep_body(const Op &op, PassScratch scr, uint32
       if (r + grp < rounds && i < n) e = take(i, p, ll);
       // a set is written again behind the next rounds' barrier
       float(&tm)[6][kBlock] = term[(r / 2) & 1];
-      auto sync = [&] { asm volatile("bar.sync %0, 64;" ::"r"(1 + wg) : "memory"); };
+      auto sync = [&] {  // the two warps that take the same 32 threads' rounds
+        __syncwarp();    // lanes that had no particle have come together again
+        asm volatile("bar.sync %0, 64;" ::"r"(1 + wg) : "memory");
+      };
       if (grp == 0) {
         tm[3][t] = e.d; tm[4][t] = e.f; tm[5][t] = e.fl;
         sync();

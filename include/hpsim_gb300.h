@@ -330,10 +330,9 @@ hps_status hps_batch_last_time_ms(hps_batch_t batch, double *ms);
  * kernels' parameter space (up to 64 beams a launch).  Each beam keeps its
  * own block count, so its reductions run in the order they have alone; the
  * merged kernels are separate compilations, so results agree with the
- * child-graph form to FP32 rounding.  It is off by default because the
- * child-graph form is faster on the batch workloads measured (beams at
- * different phases overlap: a mesh kernel of one beam beside a particle
- * sweep of another).  A range with a launch that has no lockstep form
+ * child-graph form to FP32 rounding.  It is off by default: child graphs
+ * give each beam the bits it has alone (lockstep was 6% faster on the batch
+ * workloads measured).  A range with a launch that has no lockstep form
  * (FP64 beams, monitors, the field surrogate, adjacent bunches) runs as
  * child graphs.  hps_batch_last_mode reports which form the last simulate
  * ran in (1: lockstep) and, if not lockstep, why. */
